@@ -420,20 +420,20 @@ struct Builder {
     ps_handle* H = h;
     if (fused) {
       ops.push_back([=](cudaStream_t st) {
-        return launch_plane<double>(A->d_pw + pw0, n, nx_, ny_, nz_, H->bd.tw_y, H->bd.tw_zh, H->bd.tw_z, 0, st);
+        return launch_plane<double>(A->d_pw + pw0, n, nx_, ny_, nz_, H->bd.tw_y, H->bd.tw_zh, H->bd.tw_z, st);
       });
       return;
     }
     if (mode != MODE_FIRST && ny > 1)
       ops.push_back([=](cudaStream_t st) {
-        return launch_pencil<double>(A->d_xw + yx0, n, PENCIL_INV, ny_, nx_, nzh_, H->bd.tw_y, nx_, ny_, nz_, 0, st);
+        return launch_pencil<double>(A->d_xw + yx0, n, PENCIL_INV, ny_, nx_, nzh_, H->bd.tw_y, nx_, ny_, nz_, st);
       });
     ops.push_back([=](cudaStream_t st) {
       return launch_rows<double>(A->d_pw + pw0, n, nx_ * ny_, nz_, H->bd.tw_zh, H->bd.tw_z, st);
     });
     if (mode != MODE_LAST && ny > 1)
       ops.push_back([=](cudaStream_t st) {
-        return launch_pencil<double>(A->d_xw + yx0, n, PENCIL_FWD, ny_, nx_, nzh_, H->bd.tw_y, nx_, ny_, nz_, 0, st);
+        return launch_pencil<double>(A->d_xw + yx0, n, PENCIL_FWD, ny_, nx_, nzh_, H->bd.tw_y, nx_, ny_, nz_, st);
       });
   }
   void x_pass(std::vector<Op>& ops, size_t x0, int n, int mode) {
@@ -441,7 +441,7 @@ struct Builder {
     const int nx_ = nx, ny_ = ny, nz_ = nz, inner = ny * nzh;
     ps_handle* H = h;
     ops.push_back([=](cudaStream_t st) {
-      return launch_pencil<double>(A->d_xw + x0, n, mode, nx_, 1, inner, H->bd.tw_x, nx_, ny_, nz_, 0, st);
+      return launch_pencil<double>(A->d_xw + x0, n, mode, nx_, 1, inner, H->bd.tw_x, nx_, ny_, nz_, st);
     });
   }
   // Lockstep sweeps over `len` steps.  Sweep i runs steps s0[i] .. s0[i]+len-1

@@ -148,7 +148,7 @@ static int build_class_tables(ps_batch* b, BatchClass& c) {
 }
 
 static int class_variant(ps_batch* b, const BatchClass& c) {
-  int v = (b->forced_variant >= 0) ? b->forced_variant : (c.variant < 0 ? 0 : c.variant);
+  int v = (b->forced_variant >= 0) ? b->forced_variant : (c.variant < 0 ? (VARIANT_FUSE_Z | VARIANT_FUSE_K) : c.variant);
   if ((v & VARIANT_XY) && !b->inst[c.members[0]]->xy_ok) v &= ~VARIANT_XY;
   return v & ~VARIANT_SPLIT;  // the kernels; bit 3 is the class's chains mode
 }

@@ -304,14 +304,25 @@ static int build_device_tables(ps_handle* h) {
             (T)(exp(-1.0 * ds * (ky * ky) * b * b) * exp(-1.0 * ds * (kzv * kzv) * b * b));
       }
     }
+    // compact order: [y][kz < nz/2], then the nz/2 column; halved, since the step
+    // plane pass leaves twice the transform
+    std::vector<T> kyzc((size_t)h->n[1] * h->nzh);
+    const int hz = h->nzh - 1;
+    for (int j = 0; j < h->n[1]; ++j)
+      for (int kz = 0; kz < h->nzh; ++kz)
+        kyzc[kz < hz ? (size_t)j * hz + kz : (size_t)h->n[1] * hz + j] = T(0.5) * kyz[(size_t)j * h->nzh + kz];
     T* dkx = nullptr;
     T* dkyz = nullptr;
+    T* dkyzc = nullptr;
     int rc = alloc_copy(h, &dkx, kx);
     if (rc) return rc;
+    B.kx.push_back(dkx);
     rc = alloc_copy(h, &dkyz, kyz);
     if (rc) return rc;
-    B.kx.push_back(dkx);
     B.kyz.push_back(dkyz);
+    rc = alloc_copy(h, &dkyzc, kyzc);
+    if (rc) return rc;
+    B.kyzc.push_back(dkyzc);
   }
   int rc = make_twiddles<T>(h, &B.tw_x, h->n[0]);
   if (!rc) rc = make_twiddles<T>(h, &B.tw_y, h->n[1]);
@@ -374,6 +385,7 @@ static int build_device_tables(ps_handle* h) {
         x.spec = B.spec[e];
         x.kx = B.kx[seg_of(sw, kl).ktab_id];
         x.kyz = B.kyz[seg_of(sw, kl).ktab_id];
+        x.kyzc = B.kyzc[seg_of(sw, kl).ktab_id];
         if (dc) {
           x.dc_parts = dc;
           x.dc_count = dc + B.dc_cap + 1;
@@ -491,7 +503,9 @@ static int launch_iteration(ps_handle* h, long long* nlaunch) {
   // node of the graph (a plain record would only order the capture).
   if (h->timing_cap > 0)
     PS_CUDA(h, cudaEventRecordWithFlags(h->ev_cap_start, h->st, cudaEventRecordExternal));
-  rc = launch_sweeps<T>(h, nlaunch, h->variant < 0 ? (h->branched ? VARIANT_SPLIT : 0) : h->variant);
+  // before tuning: the fused passes, branched polymers as dependent chains
+  const int first = VARIANT_FUSE_Z | VARIANT_FUSE_K | (h->branched ? VARIANT_SPLIT : 0);
+  rc = launch_sweeps<T>(h, nlaunch, h->variant < 0 ? first : h->variant);
   if (rc) return rc;
   if (h->timing_cap > 0)
     PS_CUDA(h, cudaEventRecordWithFlags(h->ev_cap_end, h->st, cudaEventRecordExternal));
@@ -680,6 +694,7 @@ template <typename T> static void free_buffers(Buffers<T>& B) {
   for (auto p : B.dcbuf) f(p);
   for (auto p : B.kx) f(p);
   for (auto p : B.kyz) f(p);
+  for (auto p : B.kyzc) f(p);
   f(B.tw_x); f(B.tw_y); f(B.tw_z); f(B.tw_zh); f(B.d_plane); f(B.d_pencil);
   B = Buffers<T>();
 }

@@ -69,6 +69,7 @@ template <typename T> struct Buffers {
                                  // fed-back rounding at dc_cap + 2)
   int dc_cap = 0;
   std::vector<T*> kx, kyz;       // per (ds, bseg) key
+  std::vector<T*> kyzc;          // kyz in the column order of the compact layout (step_plane.cuh)
   c2_t<T>* tw_x = nullptr;
   c2_t<T>* tw_y = nullptr;
   c2_t<T>* tw_z = nullptr;

@@ -189,16 +189,16 @@ int ps_fft_scaled_pair_noalloc(const int n[3], const double* d_data, const doubl
   noalloc_order_kernel<<<1, 1, 0, st>>>();
   NA_CUDA(cudaGetLastError());
   if (plane_fused_supported(8, ny, nz)) {
-    NA_CUDA(launch_plane<double>(pw, 1, nx, ny, nz, twy, twzh, twz, 0, st));
-    NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_KFULL, nx, 1, ny * nzh, twx, nx, ny, nz, 0, st));
-    NA_CUDA(launch_plane<double>(pw + 1, 1, nx, ny, nz, twy, twzh, twz, 0, st));
+    NA_CUDA(launch_plane<double>(pw, 1, nx, ny, nz, twy, twzh, twz, st));
+    NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_KFULL, nx, 1, ny * nzh, twx, nx, ny, nz, st));
+    NA_CUDA(launch_plane<double>(pw + 1, 1, nx, ny, nz, twy, twzh, twz, st));
   } else {
     NA_CUDA(launch_rows<double>(pw, 1, nx * ny, nz, twzh, twz, st));
     if (ny > 1)
-      NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_FWD, ny, nx, nzh, twy, nx, ny, nz, 0, st));
-    NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_KFULL, nx, 1, ny * nzh, twx, nx, ny, nz, 0, st));
+      NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_FWD, ny, nx, nzh, twy, nx, ny, nz, st));
+    NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_KFULL, nx, 1, ny * nzh, twx, nx, ny, nz, st));
     if (ny > 1)
-      NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_INV, ny, nx, nzh, twy, nx, ny, nz, 0, st));
+      NA_CUDA(launch_pencil<double>(xw, 1, PENCIL_INV, ny, nx, nzh, twy, nx, ny, nz, st));
     NA_CUDA(launch_rows<double>(pw + 1, 1, nx * ny, nz, twzh, twz, st));
   }
   return PS_OK;

@@ -163,14 +163,14 @@ static cudaError_t fft_r2c(ps_fft* f, const PlaneWork<double>* pw, const PencilW
   const int nx = f->n[0], ny = f->n[1], nz = f->n[2];
   cudaError_t e;
   if (f->fused) {
-    e = launch_plane<double>(pw, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, 0, f->st);
+    e = launch_plane<double>(pw, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, f->st);
   } else {
     e = launch_rows<double>(pw, 1, nx * ny, nz, f->tw_zh, f->tw_z, f->st);
     if (e == cudaSuccess && ny > 1)
-      e = launch_pencil<double>(xw, 1, PENCIL_FWD, ny, nx, f->nzh, f->tw_y, nx, ny, nz, 0, f->st);
+      e = launch_pencil<double>(xw, 1, PENCIL_FWD, ny, nx, f->nzh, f->tw_y, nx, ny, nz, f->st);
   }
   if (e == cudaSuccess)
-    e = launch_pencil<double>(xw, 1, PENCIL_FWD, nx, 1, ny * f->nzh, f->tw_x, nx, ny, nz, 0, f->st);
+    e = launch_pencil<double>(xw, 1, PENCIL_FWD, nx, 1, ny * f->nzh, f->tw_x, nx, ny, nz, f->st);
   return e;
 }
 
@@ -202,16 +202,16 @@ static int fft_pair_call(ps_fft* f, const double* data, const double* other, dou
     xk = f->d_xw + 2;
   }
   if (f->fused) {
-    FFT_CUDA(launch_plane<double>(f->d_pw, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, 0, f->st));
-    FFT_CUDA(launch_pencil<double>(xk, 1, kmode, nx, 1, ny * f->nzh, f->tw_x, nx, ny, nz, 0, f->st));
-    FFT_CUDA(launch_plane<double>(f->d_pw + 1, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, 0, f->st));
+    FFT_CUDA(launch_plane<double>(f->d_pw, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, f->st));
+    FFT_CUDA(launch_pencil<double>(xk, 1, kmode, nx, 1, ny * f->nzh, f->tw_x, nx, ny, nz, f->st));
+    FFT_CUDA(launch_plane<double>(f->d_pw + 1, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, f->st));
   } else {
     FFT_CUDA(launch_rows<double>(f->d_pw, 1, nx * ny, nz, f->tw_zh, f->tw_z, f->st));
     if (ny > 1)
-      FFT_CUDA(launch_pencil<double>(f->d_xw, 1, PENCIL_FWD, ny, nx, f->nzh, f->tw_y, nx, ny, nz, 0, f->st));
-    FFT_CUDA(launch_pencil<double>(xk, 1, kmode, nx, 1, ny * f->nzh, f->tw_x, nx, ny, nz, 0, f->st));
+      FFT_CUDA(launch_pencil<double>(f->d_xw, 1, PENCIL_FWD, ny, nx, f->nzh, f->tw_y, nx, ny, nz, f->st));
+    FFT_CUDA(launch_pencil<double>(xk, 1, kmode, nx, 1, ny * f->nzh, f->tw_x, nx, ny, nz, f->st));
     if (ny > 1)
-      FFT_CUDA(launch_pencil<double>(f->d_xw, 1, PENCIL_INV, ny, nx, f->nzh, f->tw_y, nx, ny, nz, 0, f->st));
+      FFT_CUDA(launch_pencil<double>(f->d_xw, 1, PENCIL_INV, ny, nx, f->nzh, f->tw_y, nx, ny, nz, f->st));
     FFT_CUDA(launch_rows<double>(f->d_pw + 1, 1, nx * ny, nz, f->tw_zh, f->tw_z, f->st));
   }
   FFT_CUDA(cudaMemcpyAsync(res, f->d_res, sizeof(double) * N, cudaMemcpyDeviceToHost, f->st));

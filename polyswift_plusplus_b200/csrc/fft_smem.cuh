@@ -88,6 +88,46 @@ template <bool INV, typename C> struct Dft<8, INV, C> {
   }
 };
 
+// 6- and 12-point DFTs without twiddles (Good-Thomas: 2 x 3 and 4 x 3): input
+// index R n1 + 3 n2, output index by the Chinese remainder theorem.
+template <bool INV, typename C> struct Dft<6, INV, C> {
+  static __device__ __forceinline__ void run(C* v) {
+    C a[2][3];  // a[n2][n1] = v[(2 n1 + 3 n2) % 6]
+#pragma unroll
+    for (int n2 = 0; n2 < 2; ++n2) {
+#pragma unroll
+      for (int n1 = 0; n1 < 3; ++n1) a[n2][n1] = v[(2 * n1 + 3 * n2) % 6];
+      Dft<3, INV, C>::run(a[n2]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      C b[2] = {a[0][k1], a[1][k1]};
+      Dft<2, INV, C>::run(b);
+#pragma unroll
+      for (int k2 = 0; k2 < 2; ++k2) v[(4 * k1 + 3 * k2) % 6] = b[k2];
+    }
+  }
+};
+
+template <bool INV, typename C> struct Dft<12, INV, C> {
+  static __device__ __forceinline__ void run(C* v) {
+    C a[4][3];  // a[n2][n1] = v[(4 n1 + 3 n2) % 12]
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+#pragma unroll
+      for (int n1 = 0; n1 < 3; ++n1) a[n2][n1] = v[(4 * n1 + 3 * n2) % 12];
+      Dft<3, INV, C>::run(a[n2]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      C b[4] = {a[0][k1], a[1][k1], a[2][k1], a[3][k1]};
+      Dft<4, INV, C>::run(b);
+#pragma unroll
+      for (int k2 = 0; k2 < 4; ++k2) v[(4 * k1 + 9 * k2) % 12] = b[k2];
+    }
+  }
+};
+
 // 16-point DFT as 4 x 4: radix-4 over n1 for each n2, twiddle w16^(n2 k1),
 // radix-4 over n2; output index k1 + 4 k2.
 template <bool INV, typename C> struct Dft<16, INV, C> {

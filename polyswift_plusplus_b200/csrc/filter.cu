@@ -256,12 +256,12 @@ static int filter_apply(ps_handle* h) {
     PS_CUDA(h, cudaGetLastError());
     // forward r2c
     if (f->fused) {
-      PS_CUDA(h, launch_plane<double>(f->d_pw + 2 * i, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, 0, st));
+      PS_CUDA(h, launch_plane<double>(f->d_pw + 2 * i, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, st));
     } else {
       PS_CUDA(h, launch_rows<double>(f->d_pw + 2 * i, 1, nx * ny, nz, f->tw_zh, f->tw_z, st));
-      if (ny > 1) PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_FWD, ny, nx, h->nzh, f->tw_y, nx, ny, nz, 0, st));
+      if (ny > 1) PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_FWD, ny, nx, h->nzh, f->tw_y, nx, ny, nz, st));
     }
-    PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_FWD, nx, 1, ny * h->nzh, f->tw_x, nx, ny, nz, 0, st));
+    PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_FWD, nx, 1, ny * h->nzh, f->tw_x, nx, ny, nz, st));
     if (f->multi) {
       const Regions g = regions_of(h, c);
       PS_CUDA(h, cudaMemsetAsync(f->cut, 0, sizeof(double) * (size_t)f->ncells, st));
@@ -280,11 +280,11 @@ static int filter_apply(ps_handle* h) {
     }
     PS_CUDA(h, cudaGetLastError());
     // inverse c2r, stored back into w
-    PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_INV, nx, 1, ny * h->nzh, f->tw_x, nx, ny, nz, 0, st));
+    PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_INV, nx, 1, ny * h->nzh, f->tw_x, nx, ny, nz, st));
     if (f->fused) {
-      PS_CUDA(h, launch_plane<double>(f->d_pw + 2 * i + 1, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, 0, st));
+      PS_CUDA(h, launch_plane<double>(f->d_pw + 2 * i + 1, 1, nx, ny, nz, f->tw_y, f->tw_zh, f->tw_z, st));
     } else {
-      if (ny > 1) PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_INV, ny, nx, h->nzh, f->tw_y, nx, ny, nz, 0, st));
+      if (ny > 1) PS_CUDA(h, launch_pencil<double>(f->d_xw, 1, PENCIL_INV, ny, nx, h->nzh, f->tw_y, nx, ny, nz, st));
       PS_CUDA(h, launch_rows<double>(f->d_pw + 2 * i + 1, 1, nx * ny, nz, f->tw_zh, f->tw_z, st));
     }
   }

@@ -49,13 +49,15 @@ enum {
   PENCIL_KINV = 2,
   PENCIL_KFULL = 3,
   PENCIL_KFULL_IM = 4,
-  PENCIL_KSPEC = 5
+  PENCIL_KSPEC = 5,
+  PENCIL_KINVC = 6  // PENCIL_KINV with the columns of the compact layout
 };
 
 template <typename T> struct PencilWork {
   c2_t<T>* spec;
   const T* kx;        // PENCIL_KINV: factor along the pencil axis (1/N folded in)
   const T* kyz;       // PENCIL_KINV: factor per (y, kz) column
+  const T* kyzc;      // ... in the column order of the compact layout (step_plane.cuh)
   const double* kfull;// PENCIL_KFULL(_IM): full real k array [nx][ny][nz] (plugin path)
   const c2_t<T>* kspec;// PENCIL_KSPEC: a second, fully transformed half spectrum (same layout)
   const double* dc_parts;  // PENCIL_KINV / x-y pass: the plane pass's dc_out (mean-mode carry)
@@ -72,10 +74,9 @@ bool plane_fused_supported(int prec_bytes, int ny, int nz);
 
 // Twiddle tables: tw_L[m] = exp(-2 pi i m / L); tw_zh has length nz/2, tw_z length nz.
 // Kernel variants (chosen by the engine's autotuner, all verified by tests):
-// bit 0: the plane pass runs the inverse-z last pass, the real-space step and
-// the forward-z first pass as one shared-memory round trip; bit 1: the pencil
-// pass does the same with its forward last pass, the k2 multiply and the
-// inverse first pass.
+// bit 0: the plane pass with group-local FFTs (step_plane.cuh), for every y-z
+// plane of extents 16 to 128, square or not; bit 1: the x pass in registers
+// (step_pencil.cu) instead of the shared-memory pencil pass.
 // bit 2: the sweeps use the row + x-y plane design (transposed half spectrum
 // S[kz][x][y]) instead of the y-z plane + x pencil design.
 // bit 3: each sweep of an instance runs as its own chain of launches on its
@@ -116,19 +117,27 @@ cudaError_t launch_xy(const PencilWork<T>* d_works, int nworks, int nx, int nzh,
 
 template <typename T>
 cudaError_t launch_plane(const PlaneWork<T>* d_works, int nworks, int nx, int ny, int nz,
-                         const c2_t<T>* tw_y, const c2_t<T>* tw_zh, const c2_t<T>* tw_z,
-                         int variant, cudaStream_t st);
+                         const c2_t<T>* tw_y, const c2_t<T>* tw_zh, const c2_t<T>* tw_z, cudaStream_t st);
 
 // Row (z only) pass over nrows = nx*ny flattened rows.
 template <typename T>
 cudaError_t launch_rows(const PlaneWork<T>* d_works, int nworks, int nrows, int nz,
                         const c2_t<T>* tw_zh, const c2_t<T>* tw_z, cudaStream_t st);
 
+// Plane pass with group-local FFTs on the compact spectrum layout
+// (step_plane.cuh), and the x pass in registers (step_pencil.cu).
+bool step_plane_supported(int ny, int nz);
+template <typename T>
+cudaError_t launch_step_plane(const PlaneWork<T>* d_works, int nworks, int nx, int ny, int nz,
+                              const c2_t<T>* tw_y, const c2_t<T>* tw_z, cudaStream_t st);
+template <typename T>
+cudaError_t launch_step_pencil(const PencilWork<T>* d_works, int nworks, int L, int inner, bool compact,
+                               const c2_t<T>* tw, cudaStream_t st);
+
 // Pencils of length L along an axis of stride `inner` (elements), `outer`
 // independent groups of L*inner elements; dims used only by PENCIL_KFULL.
 template <typename T>
 cudaError_t launch_pencil(const PencilWork<T>* d_works, int nworks, int mode, int L, int outer,
-                          int inner, const c2_t<T>* tw, int nx, int ny, int nz, int variant,
-                          cudaStream_t st);
+                          int inner, const c2_t<T>* tw, int nx, int ny, int nz, cudaStream_t st);
 
 }  // namespace psb

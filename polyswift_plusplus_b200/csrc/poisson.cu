@@ -142,19 +142,19 @@ static int poisson_apply(ps_handle* h) {
     filter_shift<<<blocks, 256, 0, st>>>(rho, N, p->scal);
     PS_CUDA(h, cudaGetLastError());
     if (p->fused) {
-      PS_CUDA(h, launch_plane<double>(p->d_pw + 2 * i, 1, nx, ny, nz, p->tw_y, p->tw_zh, p->tw_z, 0, st));
+      PS_CUDA(h, launch_plane<double>(p->d_pw + 2 * i, 1, nx, ny, nz, p->tw_y, p->tw_zh, p->tw_z, st));
     } else {
       PS_CUDA(h, launch_rows<double>(p->d_pw + 2 * i, 1, nx * ny, nz, p->tw_zh, p->tw_z, st));
-      if (ny > 1) PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_FWD, ny, nx, h->nzh, p->tw_y, nx, ny, nz, 0, st));
+      if (ny > 1) PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_FWD, ny, nx, h->nzh, p->tw_y, nx, ny, nz, st));
     }
-    PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_FWD, nx, 1, ny * h->nzh, p->tw_x, nx, ny, nz, 0, st));
+    PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_FWD, nx, 1, ny * h->nzh, p->tw_x, nx, ny, nz, st));
     coulomb_multiply<<<blocks, 256, 0, st>>>(p->spec, p->kc, nspec);
     PS_CUDA(h, cudaGetLastError());
-    PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_INV, nx, 1, ny * h->nzh, p->tw_x, nx, ny, nz, 0, st));
+    PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_INV, nx, 1, ny * h->nzh, p->tw_x, nx, ny, nz, st));
     if (p->fused) {
-      PS_CUDA(h, launch_plane<double>(p->d_pw + 2 * i + 1, 1, nx, ny, nz, p->tw_y, p->tw_zh, p->tw_z, 0, st));
+      PS_CUDA(h, launch_plane<double>(p->d_pw + 2 * i + 1, 1, nx, ny, nz, p->tw_y, p->tw_zh, p->tw_z, st));
     } else {
-      if (ny > 1) PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_INV, ny, nx, h->nzh, p->tw_y, nx, ny, nz, 0, st));
+      if (ny > 1) PS_CUDA(h, launch_pencil<double>(p->d_xw, 1, PENCIL_INV, ny, nx, h->nzh, p->tw_y, nx, ny, nz, st));
       PS_CUDA(h, launch_rows<double>(p->d_pw + 2 * i + 1, 1, nx * ny, nz, p->tw_zh, p->tw_z, st));
     }
     potential_update<<<blocks, 256, 0, st>>>(psi, p->res, N, 1.0 / ((double)N));

@@ -21,6 +21,7 @@
 #include "../../include/pswift.h"
 #include "fft_smem.cuh"
 #include "kernels.h"
+#include "step_common.cuh"
 #include "tma.cuh"
 
 namespace psb {
@@ -34,91 +35,6 @@ template <typename T>
 __device__ __forceinline__ T ld_or_one(const T* p, size_t i) {
   return p ? __ldg(p + i) : T(1);
 }
-
-// ---------------------------------------------------------------------------
-// Mean-mode carry (see PlaneWork in kernels.h).
-// ---------------------------------------------------------------------------
-// Per-warp FP64 sums of the forward input, summed into one CTA partial.
-__shared__ double s_dc_warp[32];
-// The mean-mode value of the inverse transform rounded to T; written by
-// thread 0 after pdl_wait(), read after the barriers that precede the inverse
-// step (kept in shared memory, not in registers, through the FFT passes).  What
-// the rounding drops comes back through the next step's mean (dc_err).
-__shared__ __align__(16) double s_dc_hilo[2];
-
-template <typename T>
-__device__ __forceinline__ void dc_hilo_store(const double* dc_in) {
-  if (threadIdx.x == 0 && dc_in) reinterpret_cast<T*>(s_dc_hilo)[0] = T(*dc_in);
-}
-
-// x + mean-mode value
-template <typename T>
-__device__ __forceinline__ c2_t<T> dc_add2(c2_t<T> x) {
-  const T m = reinterpret_cast<const T*>(s_dc_hilo)[0];
-  return cadd(x, c2_t<T>{m, m});
-}
-template <typename T>
-__device__ __forceinline__ T dc_add(T x) {
-  return x + reinterpret_cast<const T*>(s_dc_hilo)[0];
-}
-
-// Every thread of the CTA calls this (CTA-uniform): lane 0 keeps its warp's sum.
-__device__ __forceinline__ void dc_warp_sum(double v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  if ((threadIdx.x & 31) == 0) s_dc_warp[threadIdx.x >> 5] = v;
-}
-
-// After a __syncthreads() that follows dc_warp_sum: thread 0 stores the CTA's
-// partial (warps in order) and CTA 0 the number of partials.  The pointers are
-// read from the descriptor here, not kept in registers through the kernel.
-template <typename T>
-__device__ __forceinline__ void dc_cta_store(const PlaneWork<T>* wp) {
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += s_dc_warp[i];
-    double* out = reinterpret_cast<double*>(
-        __ldg(reinterpret_cast<const unsigned long long*>(&wp->dc_out)));
-    out[blockIdx.x] = s;
-    if (blockIdx.x == 0) {
-      double* cnt = reinterpret_cast<double*>(
-          __ldg(reinterpret_cast<const unsigned long long*>(&wp->dc_count)));
-      *cnt = (double)gridDim.x;
-    }
-  }
-}
-
-// Spectral pass side: one warp sums the plane pass's partials in a fixed order
-// (lane l takes slots l, l + 32, ...; then a butterfly) and stores the mean.
-// load() issues the count and the first kDcMinSlots slots (before the count is
-// known) so that they travel with the tile loads; finish() sums them.
-template <typename T> struct DcFinish {
-  double cnt;
-  double v[kDcMinSlots / 32];
-  __device__ __forceinline__ void load(const PencilWork<T>& w) {
-    const int lane = threadIdx.x & 31;
-    cnt = *w.dc_count;
-#pragma unroll
-    for (int k = 0; k < kDcMinSlots / 32; ++k) v[k] = w.dc_parts[lane + 32 * k];
-  }
-  __device__ __forceinline__ void finish(const PencilWork<T>& w) const {
-    const int lane = threadIdx.x & 31;
-    const int n = (int)cnt;
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < kDcMinSlots / 32; ++k)
-      if (lane + 32 * k < n) s += v[k];
-    for (int i = kDcMinSlots + lane; i < n; i += 32) s += w.dc_parts[i];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) {
-      // error feedback: add what the previous step's rounding to T dropped
-      const double m = s * w.dc_scale + (w.dc_first ? 0.0 : *w.dc_err);
-      *w.dc_total = m;
-      *w.dc_err = m - (double)T(m);
-    }
-  }
-};
 
 // 16-byte vector of T: 4 floats or 2 doubles.
 template <typename T> struct Vec16;
@@ -205,24 +121,6 @@ __device__ __forceinline__ void c2r_pre(C* buf, const C* twn, int rows) {
 // (p = 1..3), or 0 and 4 (p = 0).  The elements {j + 8r} of the two butterflies
 // hold every partner pair (k, 64 - k) that the pre- and post-processing combine.
 // ---------------------------------------------------------------------------
-template <typename C>
-__device__ __forceinline__ C c2r_pre_one(C a, C b, C w) {
-  // C'[k] = (A[k] + conj(A[h-k])) + i conj(W^k) (A[k] - conj(A[h-k]))
-  const C ep = {a.x + b.x, a.y - b.y};
-  const C dm = {a.x - b.x, a.y + b.y};
-  const C op = cmulc(dm, w);
-  return {ep.x - op.y, ep.y + op.x};
-}
-
-template <typename C>
-__device__ __forceinline__ C r2c_post_one(C c, C d, C w) {
-  // E = (C[k] + conj(C[km]))/2, O = -i (C[k] - conj(C[km]))/2, A[k] = E + W^k O
-  using S = decltype(c.x);
-  const C E = {S(0.5) * (c.x + d.x), S(0.5) * (c.y - d.y)};
-  const C O = {S(0.5) * (c.y + d.y), S(0.5) * (d.x - c.x)};
-  return cadd(E, cmul(w, O));
-}
-
 template <int ROWS, int TH, typename C>
 __device__ __forceinline__ void z64_inverse_first(C* buf, const C* tw_z) {
   static_assert(ROWS * 4 == TH, "one butterfly pair per thread");
@@ -499,45 +397,6 @@ __device__ __forceinline__ void real_space(const PlaneWork<T>& w, T* rbuf, size_
   }
 }
 
-// Real-space step of a MID pass inside one block (wfac_in == wfac_out),
-// applied inside the fused z pass: slot p of row b holds (a[2p], a[2p+1]);
-// q = a*wfac is stored and a = q*wfac goes on to the forward transform.
-template <typename T, int NZ, int R>
-struct RealStepOp {
-  using T2 = c2_t<T>;
-  static constexpr int M = (NZ / 2) / R;
-  const T* wfac;
-  T* store;
-  size_t roff;
-  int rows;
-  bool dc_on = false;  // add the mean-mode value (s_dc_hilo) after the inverse transform
-  T acc = T(0);        // sum of the forward input (mean-mode carry)
-  T2 wf[R];
-  __device__ __forceinline__ void prefetch(int b, int j) {
-    if (b >= rows) return;
-    const T* wi = wfac + roff + (size_t)b * NZ;
-#pragma unroll
-    for (int r = 0; r < R; ++r) wf[r] = __ldg(reinterpret_cast<const T2*>(wi + 2 * (j + r * M)));
-  }
-  __device__ __forceinline__ void apply(int b, int j, T2 (&v)[R]) {
-    if (b >= rows) return;
-    T* st = store + roff + (size_t)b * NZ;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const T2 x = dc_on ? dc_add2<T>(v[r]) : v[r];
-      const T q0 = x.x * wf[r].x;
-      const T q1 = x.y * wf[r].y;
-      *reinterpret_cast<T2*>(st + 2 * (j + r * M)) = T2{q0, q1};
-      v[r] = T2{q0 * wf[r].x, q1 * wf[r].y};
-    }
-  }
-  // s = the sum of this butterfly's forward inputs (a local FP32 sum: its
-  // rounding differs from butterfly to butterfly)
-  __device__ __forceinline__ void after(int b, T2 s) {
-    if (b < rows) acc += s.x + s.y;
-  }
-};
-
 // ---------------------------------------------------------------------------
 // Plane / row pass.  DO_Y: tile = one whole x-plane (ROWS = ny), moved in and
 // out with bulk TMA copies, and the y FFT is done here; otherwise tile = ROWS
@@ -550,7 +409,7 @@ template <typename T, int TH> struct PlaneMinBlocks {
 
 // LT (row mode only): the half spectrum is stored transposed, S[kz][x][y], for
 // the x-y plane pass; a tile is ROWS consecutive y of one x (ROWS divides ny).
-template <typename T, int ROWS, int NZ, int TH, bool DO_Y, bool FZ, bool LT>
+template <typename T, int ROWS, int NZ, int TH, bool DO_Y, bool LT>
 __global__ void __launch_bounds__(TH, (PlaneMinBlocks<T, TH>::v))
     plane_kernel(const PlaneWork<T>* __restrict__ works, int nrows_total,
                  const c2_t<T>* __restrict__ tw_y, const c2_t<T>* __restrict__ tw_zh,
@@ -632,45 +491,6 @@ __global__ void __launch_bounds__(TH, (PlaneMinBlocks<T, TH>::v))
     __syncthreads();
     if constexpr (DO_Y) plane_y_inverse<ROWS, NZH, TH>(buf, s_tw_y);
     if constexpr (NZ > 1) {
-      if (FZ && w.mode == MODE_MID && w.wfac_in && w.wfac_in == w.wfac_out && w.store) {
-        if constexpr (NZ == 128 && DO_Y && ROWS * 4 == TH) {
-          // pre-processing + first inverse pass; last inverse pass + real-space
-          // step + first forward pass (index-fastest: each warp covers 4 rows x
-          // 8 butterflies, so the wfac loads and q stores are 64-byte segments);
-          // last forward pass + post-processing
-          z64_inverse_first<ROWS, TH>(buf, s_tw_z);
-          RealStepOp<T, NZ, 8> op;
-          op.wfac = w.wfac_in;
-          op.store = w.store;
-          op.roff = roff;
-          op.rows = rows;
-          op.dc_on = (w.dc_in != nullptr);
-          fused_pass_pair<H, 8, ROWS, TH, true, false, false>(buf, NZH, 1, s_tw_zh, op);
-          if (dc_sum) dc_warp_sum((double)op.acc);
-          z64_forward_last<ROWS, TH>(buf, s_tw_zh, s_tw_z);
-          goto forward_y;
-        }
-        c2r_pre<NZ, ROWS, TH>(buf, s_tw_z, rows);
-        __syncthreads();
-        // inverse z FFT, real-space step and forward z FFT with the last inverse
-        // pass, the step and the first forward pass in one round trip
-        using PI = typename Plan<H>::type;
-        using PF = typename RLReverse<PI>::type;
-        constexpr int RF = RLLast<PI>::value;
-        smem_fft_head<H, PI, ROWS, TH, true, true>(buf, NZH, 1, s_tw_zh);
-        RealStepOp<T, NZ, RF> op;
-        op.wfac = w.wfac_in;
-        op.store = w.store;
-        op.roff = roff;
-        op.rows = rows;
-        op.dc_on = (w.dc_in != nullptr);
-        fused_pass_pair<H, RF, ROWS, TH, true, false, true>(buf, NZH, 1, s_tw_zh, op);
-        if (dc_sum) dc_warp_sum((double)op.acc);
-        smem_fft_tail<H, PF, ROWS, TH, false, true>(buf, NZH, 1, s_tw_zh);
-        r2c_post<NZ, ROWS, TH>(buf, s_tw_z, rows);
-        __syncthreads();
-        goto forward_y;
-      }
       if constexpr (NZ == 128 && DO_Y && ROWS * 4 == TH) {
         z64_inverse_first<ROWS, TH>(buf, s_tw_z);
         stockham_pass<H, 8, 8, ROWS, TH, true, true>(buf, NZH, 1, s_tw_zh);
@@ -698,7 +518,6 @@ __global__ void __launch_bounds__(TH, (PlaneMinBlocks<T, TH>::v))
       __syncthreads();
     }
   }
-forward_y:
   if constexpr (DO_Y) plane_y_forward<ROWS, NZH, TH>(buf, s_tw_y);
   if constexpr (BULK) {
     fence_proxy_async_smem();
@@ -727,38 +546,11 @@ forward_y:
   if (dc_sum) dc_cta_store(works + blockIdx.y);
 }
 
-// k2 multiply applied inside the fused x pass: exp(-ds b^2 k^2)/N as the
-// product of the x table and the (y, kz) table.
-template <typename T, int L, int R>
-struct KStepOp {
-  using T2 = c2_t<T>;
-  static constexpr int M = L / R;
-  const T* kx;
-  const T* kyz;
-  int c0;
-  int inner;
-  bool dc0;  // this tile holds the k = 0 coefficient and the mean mode is carried in FP64
-  T fyz;
-  __device__ __forceinline__ void prefetch(int b, int j) {
-    const int c = c0 + b;
-    fyz = (c < inner) ? __ldg(kyz + c) : T(0);
-  }
-  __device__ __forceinline__ void apply(int b, int j, T2 (&v)[R]) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const T f = __ldg(kx + j + r * M) * fyz;
-      v[r] = T2{v[r].x * f, v[r].y * f};
-    }
-    if (dc0 && b == 0 && j == 0) v[0] = T2{T(0), T(0)};
-  }
-  __device__ __forceinline__ void after(int, T2) {}
-};
-
 // ---------------------------------------------------------------------------
 // Pencil pass along a strided axis.  Tile = TK adjacent columns of `inner`,
 // loaded with 16-byte vector loads all issued before use.
 // ---------------------------------------------------------------------------
-template <typename T, int L, int TK, int TH, int MODE, bool FK>
+template <typename T, int L, int TK, int TH, int MODE>
 __global__ void __launch_bounds__(TH)
     pencil_kernel(const PencilWork<T>* __restrict__ works, int inner, int tiles,
                   const c2_t<T>* __restrict__ tw, int nx, int ny, int nz) {
@@ -780,7 +572,7 @@ __global__ void __launch_bounds__(TH)
   const bool full = (c0 + TK <= inner) && (inner % CPV == 0);
   // mean-mode carry: the tile of column 0 drops the FP32 k = 0 coefficient and
   // its first warp turns the plane pass's FP64 partials into the mean
-  const bool dc0 = (MODE == PENCIL_KINV) && w.dc_total && o == 0 && c0 == 0;
+  const bool dc0 = (MODE == PENCIL_KINV || MODE == PENCIL_KINVC) && w.dc_total && o == 0 && c0 == 0;
   for (int i = tid; i < L; i += TH) s_tw[i] = tw[i];
   pdl_wait();  // before any read or write of the spectrum
   DcFinish<T> dcf;
@@ -811,30 +603,15 @@ __global__ void __launch_bounds__(TH)
   }
   if (dc0 && tid < 32) dcf.finish(w);
   __syncthreads();
-  if constexpr (MODE == PENCIL_KINV && L > 1 && FK) {
-    // forward FFT, k2 multiply and inverse FFT with the last forward pass, the
-    // multiply and the first inverse pass in one round trip
-    using RI = typename RLReverse<RL>::type;
-    constexpr int RF = RLLast<RL>::value;
-    smem_fft_head<L, RL, TK, TH, false, true>(buf, 1, TK, s_tw);
-    KStepOp<T, L, RF> op;
-    op.kx = w.kx;
-    op.kyz = w.kyz;
-    op.c0 = c0;
-    op.inner = inner;
-    op.dc0 = dc0;
-    fused_pass_pair<L, RF, TK, TH, false, true, true>(buf, 1, TK, s_tw, op);
-    smem_fft_tail<L, RI, TK, TH, true, true>(buf, 1, TK, s_tw);
-    goto store_tile;
-  }
   if (MODE != PENCIL_INV) smem_fft<L, TK, TH, false, true, C, RL>(buf, 1, TK, s_tw);
-  if (MODE == PENCIL_KINV) {
+  if (MODE == PENCIL_KINV || MODE == PENCIL_KINVC) {
+    const T* kyz = (MODE == PENCIL_KINVC) ? w.kyzc : w.kyz;
     for (int e = tid; e < L * TK; e += TH) {
       const int i = e / TK;
       const int cc = e - i * TK;
       const int c = c0 + cc;
       if (c < inner) {
-        const T f = __ldg(w.kx + i) * __ldg(w.kyz + c);
+        const T f = __ldg(w.kx + i) * __ldg(kyz + c);
         const C v = buf[e];
         buf[e] = (dc0 && e == 0) ? C{T(0), T(0)} : C{v.x * f, v.y * f};
       }
@@ -898,7 +675,6 @@ __global__ void __launch_bounds__(TH)
     __syncthreads();
   }
   if (MODE != PENCIL_FWD) smem_fft<L, TK, TH, true, true, C, RL>(buf, 1, TK, s_tw);
-store_tile:
   if (full) {
 #pragma unroll
     for (int u = 0; u < UV; ++u) {
@@ -922,46 +698,6 @@ store_tile:
 // ---------------------------------------------------------------------------
 // Dispatch.
 // ---------------------------------------------------------------------------
-// Opt in to large dynamic shared memory once per (kernel, device).
-template <typename K>
-static cudaError_t ensure_smem_attr(K kern, size_t smem, unsigned* done_mask) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned bit = 1u << (dev & 31);
-  if (*done_mask & bit) return cudaSuccess;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) *done_mask |= bit;
-  return e;
-}
-
-// Sweep kernels are launched with programmatic stream serialisation (they call
-// pdl_wait() before touching data another kernel wrote), unless PSB_PDL=0.
-static bool pdl_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("PSB_PDL");
-    on = (e && e[0] == '0') ? 0 : 1;
-  }
-  return on != 0;
-}
-
-template <typename... K, typename... Args>
-static cudaError_t launch_sweep_kernel(void (*kern)(K...), dim3 grid, dim3 block, size_t smem,
-                                       cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 static const int kExtents[] = {1, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128, 256};
 
 bool extent_supported(int n) {
@@ -970,7 +706,7 @@ bool extent_supported(int n) {
   return false;
 }
 
-template <typename T, int ROWS, int NZ, int TH, bool DO_Y, bool FZ, bool LT = false>
+template <typename T, int ROWS, int NZ, int TH, bool DO_Y, bool LT = false>
 static cudaError_t launch_plane_t(const PlaneWork<T>* d_works, int nworks, int ntiles,
                                   int nrows_total, const c2_t<T>* tw_y, const c2_t<T>* tw_zh,
                                   const c2_t<T>* tw_z, cudaStream_t st, int lt_nx = 0,
@@ -980,7 +716,7 @@ static cudaError_t launch_plane_t(const PlaneWork<T>* d_works, int nworks, int n
   constexpr int H = (NZ > 1) ? NZ / 2 : 1;
   const size_t smem =
       sizeof(C) * ((size_t)ROWS * NZH + H + NZ + (DO_Y ? ROWS : 0)) + sizeof(uint64_t);
-  auto kern = plane_kernel<T, ROWS, NZ, TH, DO_Y, FZ, LT>;
+  auto kern = plane_kernel<T, ROWS, NZ, TH, DO_Y, LT>;
   static unsigned attr_mask = 0;
   cudaError_t ea = ensure_smem_attr(kern, smem, &attr_mask);
   if (ea != cudaSuccess) return ea;
@@ -1264,15 +1000,12 @@ bool cluster_plane_supported(int prec_bytes, int ny, int nz) {
 
 #define PSB_PLANE_CASE(T, NY, NZ, TH)                                                      \
   if (ny == NY && nz == NZ)                                                                \
-    return (variant & 1) ? launch_plane_t<T, NY, NZ, TH, true, true>(                      \
-                               d_works, nworks, nx, nx * ny, tw_y, tw_zh, tw_z, st)        \
-                         : launch_plane_t<T, NY, NZ, TH, true, false>(                     \
-                               d_works, nworks, nx, nx * ny, tw_y, tw_zh, tw_z, st);
+    return launch_plane_t<T, NY, NZ, TH, true>(d_works, nworks, nx, nx * ny, tw_y, tw_zh, tw_z, st);
 
 template <typename T>
 cudaError_t launch_plane_impl(const PlaneWork<T>* d_works, int nworks, int nx, int ny, int nz,
                               const c2_t<T>* tw_y, const c2_t<T>* tw_zh, const c2_t<T>* tw_z,
-                              int variant, cudaStream_t st) {
+                              cudaStream_t st) {
   PSB_PLANE_CASE(T, 8, 8, 64)
   PSB_PLANE_CASE(T, 12, 12, 64)
   PSB_PLANE_CASE(T, 16, 16, 128)
@@ -1291,7 +1024,7 @@ cudaError_t launch_plane_impl(const PlaneWork<T>* d_works, int nworks, int nx, i
 
 #define PSB_ROW_CASE(T, NZ, ROWS, TH)                                                      \
   if (nz == NZ)                                                                            \
-    return launch_plane_t<T, ROWS, NZ, TH, false, false>(                                  \
+    return launch_plane_t<T, ROWS, NZ, TH, false>(                                  \
         d_works, nworks, (nrows + ROWS - 1) / ROWS, nrows, nullptr, tw_zh, tw_z, st);
 
 template <typename T>
@@ -1315,7 +1048,7 @@ cudaError_t launch_rows_impl(const PlaneWork<T>* d_works, int nworks, int nrows,
 // Row pass writing the transposed spectrum S[kz][x][y] (tiles of ROWS y of one x).
 #define PSB_ROWT_CASE(T, NZ, ROWS, TH)                                                      \
   if (nz == NZ && ny % ROWS == 0)                                                           \
-    return launch_plane_t<T, ROWS, NZ, TH, false, false, true>(                             \
+    return launch_plane_t<T, ROWS, NZ, TH, false, true>(                             \
         d_works, nworks, nx * ny / ROWS, nx * ny, nullptr, tw_zh, tw_z, st, nx, ny);
 
 template <typename T>
@@ -1490,12 +1223,12 @@ cudaError_t launch_xy_impl(const PencilWork<T>* d_works, int nworks, int nx, int
   return cudaErrorInvalidValue;
 }
 
-template <typename T, int L, int TK, int TH, int MODE, bool FK>
+template <typename T, int L, int TK, int TH, int MODE>
 static cudaError_t launch_pencil_t(const PencilWork<T>* d_works, int nworks, int outer, int inner,
                                    const c2_t<T>* tw, int nx, int ny, int nz, cudaStream_t st) {
   using C = c2_t<T>;
   const size_t smem = sizeof(C) * ((size_t)L * TK + (size_t)L);
-  auto kern = pencil_kernel<T, L, TK, TH, MODE, FK>;
+  auto kern = pencil_kernel<T, L, TK, TH, MODE>;
   static unsigned attr_mask = 0;
   cudaError_t ea = ensure_smem_attr(kern, smem, &attr_mask);
   if (ea != cudaSuccess) return ea;
@@ -1507,28 +1240,26 @@ static cudaError_t launch_pencil_t(const PencilWork<T>* d_works, int nworks, int
 template <typename T, int L, int TK, int TH>
 static cudaError_t launch_pencil_modes(const PencilWork<T>* d_works, int nworks, int mode, int outer,
                                        int inner, const c2_t<T>* tw, int nx, int ny, int nz,
-                                       int variant, cudaStream_t st) {
+                                       cudaStream_t st) {
   switch (mode) {
     case PENCIL_FWD:
-      return launch_pencil_t<T, L, TK, TH, PENCIL_FWD, false>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
+      return launch_pencil_t<T, L, TK, TH, PENCIL_FWD>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
     case PENCIL_INV:
-      return launch_pencil_t<T, L, TK, TH, PENCIL_INV, false>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
+      return launch_pencil_t<T, L, TK, TH, PENCIL_INV>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
     case PENCIL_KINV:
-      return (variant & 2)
-                 ? launch_pencil_t<T, L, TK, TH, PENCIL_KINV, true>(d_works, nworks, outer, inner, tw,
-                                                                    nx, ny, nz, st)
-                 : launch_pencil_t<T, L, TK, TH, PENCIL_KINV, false>(d_works, nworks, outer, inner, tw,
-                                                                     nx, ny, nz, st);
+      return launch_pencil_t<T, L, TK, TH, PENCIL_KINV>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
+    case PENCIL_KINVC:
+      return launch_pencil_t<T, L, TK, TH, PENCIL_KINVC>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
     case PENCIL_KFULL:
-      return launch_pencil_t<T, L, TK, TH, PENCIL_KFULL, false>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
+      return launch_pencil_t<T, L, TK, TH, PENCIL_KFULL>(d_works, nworks, outer, inner, tw, nx, ny, nz, st);
     case PENCIL_KFULL_IM:
       if constexpr (sizeof(T) == 8)
-        return launch_pencil_t<T, L, TK, TH, PENCIL_KFULL_IM, false>(d_works, nworks, outer, inner, tw, nx, ny,
+        return launch_pencil_t<T, L, TK, TH, PENCIL_KFULL_IM>(d_works, nworks, outer, inner, tw, nx, ny,
                                                                      nz, st);
       break;
     case PENCIL_KSPEC:
       if constexpr (sizeof(T) == 8)
-        return launch_pencil_t<T, L, TK, TH, PENCIL_KSPEC, false>(d_works, nworks, outer, inner, tw, nx, ny,
+        return launch_pencil_t<T, L, TK, TH, PENCIL_KSPEC>(d_works, nworks, outer, inner, tw, nx, ny,
                                                                   nz, st);
       break;
   }
@@ -1542,12 +1273,12 @@ template <> struct PencilTK<double> { static constexpr int v = 16; };
 #define PSB_PENCIL_CASE(T, L, TH)                                                          \
   if (len == L)                                                                             \
     return launch_pencil_modes<T, L, PencilTK<T>::v, TH>(d_works, nworks, mode, outer, inner, tw, \
-                                                         nx, ny, nz, variant, st);
+                                                         nx, ny, nz, st);
 
 template <typename T>
 cudaError_t launch_pencil_impl(const PencilWork<T>* d_works, int nworks, int mode, int len,
                                int outer, int inner, const c2_t<T>* tw, int nx, int ny, int nz,
-                               int variant, cudaStream_t st) {
+                               cudaStream_t st) {
   PSB_PENCIL_CASE(T, 1, 64)
   PSB_PENCIL_CASE(T, 4, 64)
   PSB_PENCIL_CASE(T, 8, 64)
@@ -1560,7 +1291,7 @@ cudaError_t launch_pencil_impl(const PencilWork<T>* d_works, int nworks, int mod
   PSB_PENCIL_CASE(T, 96, 256)
   if (len == 128 && sizeof(T) == 4)
     return launch_pencil_modes<T, 128, 16, 128>(d_works, nworks, mode, outer, inner, tw, nx, ny, nz,
-                                                variant, st);
+                                                st);
   PSB_PENCIL_CASE(T, 128, 256)
   PSB_PENCIL_CASE(T, 256, 256)
   return cudaErrorInvalidValue;
@@ -1570,14 +1301,14 @@ cudaError_t launch_pencil_impl(const PencilWork<T>* d_works, int nworks, int mod
 template <>
 cudaError_t launch_plane<float>(const PlaneWork<float>* w, int nw, int nx, int ny, int nz,
                                 const float2* ty, const float2* tzh, const float2* tz,
-                                int variant, cudaStream_t st) {
-  return launch_plane_impl<float>(w, nw, nx, ny, nz, ty, tzh, tz, variant, st);
+                                cudaStream_t st) {
+  return launch_plane_impl<float>(w, nw, nx, ny, nz, ty, tzh, tz, st);
 }
 template <>
 cudaError_t launch_plane<double>(const PlaneWork<double>* w, int nw, int nx, int ny, int nz,
                                  const double2* ty, const double2* tzh, const double2* tz,
-                                 int variant, cudaStream_t st) {
-  return launch_plane_impl<double>(w, nw, nx, ny, nz, ty, tzh, tz, variant, st);
+                                 cudaStream_t st) {
+  return launch_plane_impl<double>(w, nw, nx, ny, nz, ty, tzh, tz, st);
 }
 template <>
 cudaError_t launch_rows<float>(const PlaneWork<float>* w, int nw, int nrows, int nz,
@@ -1611,15 +1342,15 @@ cudaError_t launch_xy<double>(const PencilWork<double>* w, int nw, int nx, int n
 }
 template <>
 cudaError_t launch_pencil<float>(const PencilWork<float>* w, int nw, int mode, int L, int outer,
-                                 int inner, const float2* tw, int nx, int ny, int nz, int variant,
+                                 int inner, const float2* tw, int nx, int ny, int nz,
                                  cudaStream_t st) {
-  return launch_pencil_impl<float>(w, nw, mode, L, outer, inner, tw, nx, ny, nz, variant, st);
+  return launch_pencil_impl<float>(w, nw, mode, L, outer, inner, tw, nx, ny, nz, st);
 }
 template <>
 cudaError_t launch_pencil<double>(const PencilWork<double>* w, int nw, int mode, int L, int outer,
-                                  int inner, const double2* tw, int nx, int ny, int nz, int variant,
+                                  int inner, const double2* tw, int nx, int ny, int nz,
                                   cudaStream_t st) {
-  return launch_pencil_impl<double>(w, nw, mode, L, outer, inner, tw, nx, ny, nz, variant, st);
+  return launch_pencil_impl<double>(w, nw, mode, L, outer, inner, tw, nx, ny, nz, st);
 }
 
 }  // namespace psb

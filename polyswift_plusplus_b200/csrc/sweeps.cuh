@@ -58,6 +58,20 @@ inline cudaError_t launch_plane_cluster_t(const PlaneWork<T>* w, int nw, int nx,
   return launch_plane_cluster<T>(w, nw, nx, ty, tzh, tz, st);
 }
 
+// The sweeps' spectra are in the compact layout of step_plane.cuh.
+template <typename T>
+inline bool compact_path(const SweepSet<T>& s, int variant) {
+  return (variant & VARIANT_FUSE_Z) && step_plane_supported(s.n[1], s.n[2]);
+}
+template <typename T>
+inline cudaError_t launch_x_pass(const SweepSet<T>& s, const PencilWork<T>* w, int nw, bool compact, int variant,
+                                 cudaStream_t st) {
+  if (variant & VARIANT_FUSE_K)
+    return launch_step_pencil<T>(w, nw, s.n[0], s.n[1] * s.nzh, compact, s.tw_x, st);
+  return launch_pencil<T>(w, nw, compact ? PENCIL_KINVC : PENCIL_KINV, s.n[0], 1, s.n[1] * s.nzh, s.tw_x, s.n[0],
+                          s.n[1], s.n[2], st);
+}
+
 template <typename T>
 cudaError_t launch_sweep_set(const SweepSet<T>& s, int variant, cudaStream_t st, long long* nlaunch) {
   const int nx = s.n[0], ny = s.n[1], nz = s.n[2];
@@ -80,20 +94,21 @@ cudaError_t launch_sweep_set(const SweepSet<T>& s, int variant, cudaStream_t st,
     if ((variant & VARIANT_XY) && s.xy_ok) {
       PSB_L(launch_rows_t<T>(pw, np, nx, ny, nz, s.tw_zh, s.tw_z, st));
       if (nxw > 0) PSB_L(launch_xy<T>(xw, nxw, nx, s.nzh, s.tw_x, variant, st));
+    } else if (compact_path(s, variant)) {
+      PSB_L(launch_step_plane<T>(pw, np, nx, ny, nz, s.tw_y, s.tw_z, st));
+      if (nxw > 0) PSB_L(launch_x_pass<T>(s, xw, nxw, true, variant, st));
     } else if (s.fused_plane) {
-      PSB_L(launch_plane<T>(pw, np, nx, ny, nz, s.tw_y, s.tw_zh, s.tw_z, variant, st));
-      if (nxw > 0)
-        PSB_L(launch_pencil<T>(xw, nxw, PENCIL_KINV, nx, 1, ny * s.nzh, s.tw_x, nx, ny, nz, variant, st));
+      PSB_L(launch_plane<T>(pw, np, nx, ny, nz, s.tw_y, s.tw_zh, s.tw_z, st));
+      if (nxw > 0) PSB_L(launch_x_pass<T>(s, xw, nxw, false, variant, st));
     } else if (cluster_path(s, variant)) {
       PSB_L(launch_plane_cluster_t<T>(pw, np, nx, s.tw_y, s.tw_zh, s.tw_z, st));
-      if (nxw > 0)
-        PSB_L(launch_pencil<T>(xw, nxw, PENCIL_KINV, nx, 1, ny * s.nzh, s.tw_x, nx, ny, nz, variant, st));
+      if (nxw > 0) PSB_L(launch_x_pass<T>(s, xw, nxw, false, variant, st));
     } else {
       PSB_L(launch_rows<T>(pw, np, nx * ny, nz, s.tw_zh, s.tw_z, st));
       if (nxw > 0) {
-        if (ny > 1) PSB_L(launch_pencil<T>(xw, nxw, PENCIL_FWD, ny, nx, s.nzh, s.tw_y, nx, ny, nz, variant, st));
-        PSB_L(launch_pencil<T>(xw, nxw, PENCIL_KINV, nx, 1, ny * s.nzh, s.tw_x, nx, ny, nz, variant, st));
-        if (ny > 1) PSB_L(launch_pencil<T>(xw, nxw, PENCIL_INV, ny, nx, s.nzh, s.tw_y, nx, ny, nz, variant, st));
+        if (ny > 1) PSB_L(launch_pencil<T>(xw, nxw, PENCIL_FWD, ny, nx, s.nzh, s.tw_y, nx, ny, nz, st));
+        PSB_L(launch_x_pass<T>(s, xw, nxw, false, variant, st));
+        if (ny > 1) PSB_L(launch_pencil<T>(xw, nxw, PENCIL_INV, ny, nx, s.nzh, s.tw_y, nx, ny, nz, st));
       }
     }
   }

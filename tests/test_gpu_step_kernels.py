@@ -1,0 +1,84 @@
+"""The step plane pass (variant bit 0) and the x pass in registers (bit 1) over every plane
+shape and x extent they exist for, against the passes they replace (variant 0: the
+shared-memory plane pass, or row and y-pencil passes where no such pass exists) and, on an
+uneven grid, against the FP64 oracle.
+
+Tolerances: both paths compute the same transforms with another order of operations.  FP64:
+about 2 Ns log2(N) roundings of 1e-16, below 1e-12 of the field's maximum.  FP32 sweeps: a
+transform pair's error is about 1e-7 of the maximum and adds up over the 40 steps of two
+sweeps as a random walk, below 5e-6.
+"""
+import math
+
+import numpy as np
+import pytest
+
+import oracle as O
+from polyswift_plusplus_b200 import workloads as W
+from polyswift_plusplus_b200.scft import ScftSolver
+
+pytestmark = pytest.mark.gpu
+EXTENTS = (16, 24, 32, 48, 64, 96, 128)
+
+
+def _case(n, precision, ns=20):
+    """A diblock with joints inside the sweep (wfac_in != wfac_out), odd and even step counts."""
+    cfg = W.diblock_config(16, 2.0, 0.35, 20.0, ns, W.Updater(kind="steepestDescent", relaxlambdas=(0.1, 0.05)),
+                           precision)
+    cfg.n = tuple(n)
+    cfg.cell = (0.11, 0.07, 0.05)
+    x, y, z = W.coords(cfg)
+    c = (np.cos(2 * math.pi * x / cfg.box[0]) + np.cos(4 * math.pi * y / cfg.box[1])
+         + np.cos(6 * math.pi * z / cfg.box[2])).reshape(-1)
+    w = W.random_fields(cfg, 0.3)
+    return cfg, [w[0] + c, w[1] - c]
+
+
+def _fields(cfg, w, variant):
+    s = ScftSolver(cfg)
+    s.set_variant(variant)
+    s.restore(w)
+    s.update(2)  # one eager iteration and one from the graph
+    out = [s.w(0), s.w(1), s.phi(0), s.phi(1), s.pressure()]
+    q = s.scalars()["q"][0]
+    s.close()
+    return out, q
+
+
+def _compare(n, precision, variants, against):
+    tol = 1e-12 if precision == "fp64" else 5e-6
+    cfg, w = _case(n, precision)
+    ref, qr = _fields(cfg, w, against)
+    for v in variants:
+        got, q = _fields(cfg, w, v)
+        assert abs(q - qr) <= tol * qr, (n, v)
+        for a, b in zip(got, ref):
+            assert np.abs(a - b).max() <= tol * max(1.0, np.abs(b).max()), (n, precision, v)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("ny", EXTENTS)
+def test_every_plane_shape(gpu, ny, precision):
+    for nz in EXTENTS:
+        _compare((4, ny, nz), precision, [3, 11], 0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_every_x_extent(gpu, precision):
+    """x extents with their own butterfly split, whole and partial column tiles (12 x 7 columns
+    of the row-pass grid), on the compact layout (variant 3) and the plain one (2)."""
+    for nx in (1, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128, 256):
+        _compare((nx, 16, 24), precision, [2, 3], 0)
+        _compare((nx, 12, 12), precision, [2], 0)
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 1e-5)])
+def test_uneven_grid_matches_oracle(gpu, oracle_lib, precision, tol):
+    cfg, w = _case((12, 48, 32), precision)
+    got, q = _fields(cfg, w, 3)
+    o = O.Oracle(cfg)
+    o.restore(w)
+    h = o.update(2)
+    assert abs(q - h[-1]["q"][0]) <= tol * q
+    for a, b in zip(got, [o.w(0), o.w(1), o.phi(0), o.phi(1), o.pressure()]):
+        assert np.abs(a - b).max() <= tol * max(1.0, np.abs(b).max())
