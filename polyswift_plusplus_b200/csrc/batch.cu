@@ -38,6 +38,8 @@ struct BatchClass {
   std::vector<JunctionLaunch<float>> junc_f;
   std::vector<JunctionLaunch<double>> junc_d;
   std::vector<int> junc_off, junc_cnt;
+  std::vector<SweepLevel> levels;  // one-launch sweeps of all members
+  void* d_sweep = nullptr;   // SweepWork<T>[]
   void* d_plane = nullptr;   // PlaneWork<T>[]
   void* d_pencil = nullptr;  // PencilWork<T>[]
   cudaStream_t st = nullptr;
@@ -93,6 +95,9 @@ static SweepSet<T> class_sweep_set(ps_batch* b, BatchClass& c) {
   s.kmax = c.kmax;
   s.d_plane = static_cast<const PlaneWork<T>*>(c.d_plane);
   s.d_pencil = static_cast<const PencilWork<T>*>(c.d_pencil);
+  s.d_sweep = static_cast<const SweepWork<T>*>(c.d_sweep);
+  s.levels = c.levels.data();
+  s.nlevels = (int)c.levels.size();
   s.plane_off = c.plane_off.data();
   s.plane_cnt = c.plane_cnt.data();
   s.pencil_off = c.pencil_off.data();
@@ -139,6 +144,28 @@ static int build_class_tables(ps_batch* b, BatchClass& c) {
     }
     c.plane_cnt[k] = (int)pw.size() - c.plane_off[k];
     c.pencil_cnt[k] = (int)xw.size() - c.pencil_off[k];
+  }
+  // one-launch sweeps: every member's, by start step
+  std::vector<std::pair<int, SweepWork<T>>> sw;
+  bool all = true;
+  for (int i : c.members) {
+    ps_handle* h = b->inst[i];
+    const Buffers<T>& B = bufs<T>(h);
+    all = all && B.d_sweep;
+    for (const SweepLevel& l : h->levels)
+      for (int j = 0; all && j < l.cnt; ++j) sw.push_back({l.k, B.h_sweep[l.off + j]});
+  }
+  std::stable_sort(sw.begin(), sw.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+  std::vector<SweepWork<T>> swv;
+  c.levels.clear();
+  for (size_t i = 0; all && i < sw.size(); ++i) {
+    if (c.levels.empty() || c.levels.back().k != sw[i].first) c.levels.push_back(SweepLevel{sw[i].first, (int)i, 0});
+    c.levels.back().cnt++;
+    swv.push_back(sw[i].second);
+  }
+  if (all) {
+    PB_CUDA(b, cudaMalloc(&c.d_sweep, sizeof(SweepWork<T>) * swv.size()));
+    PB_CUDA(b, cudaMemcpy(c.d_sweep, swv.data(), sizeof(SweepWork<T>) * swv.size(), cudaMemcpyHostToDevice));
   }
   PB_CUDA(b, cudaMalloc(&c.d_plane, sizeof(PlaneWork<T>) * std::max<size_t>(pw.size(), 1)));
   PB_CUDA(b, cudaMemcpy(c.d_plane, pw.data(), sizeof(PlaneWork<T>) * pw.size(), cudaMemcpyHostToDevice));
@@ -254,6 +281,10 @@ static int batch_autotune(ps_batch* b) {
                         : autotune_sweep_set<double>(class_sweep_set<double>(b, c), c.st, c.tune_ms, &best);
     PB_CUDA(b, e);
     c.variant = best;
+    // one-launch sweeps are single launches either way: the members share them
+    const bool one_launch = (c.prec == PS_PREC_MIXED) ? resident_path(class_sweep_set<float>(b, c), best)
+                                                      : resident_path(class_sweep_set<double>(b, c), best);
+    if (one_launch) continue;
     // the same kernels as the members' own concurrent chains: one warm-up and
     // one timed pass, forked from and joined back into c.st
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -348,6 +379,7 @@ static void batch_free(ps_batch* b) {
   if (b->st) cudaStreamSynchronize(b->st);
   drop_graph(b);
   for (BatchClass& c : b->classes) {
+    if (c.d_sweep) cudaFree(c.d_sweep);
     if (c.d_plane) cudaFree(c.d_plane);
     if (c.d_pencil) cudaFree(c.d_pencil);
     if (c.ev) cudaEventDestroy(c.ev);

@@ -308,6 +308,11 @@ static int build_device_tables(ps_handle* h) {
     // plane pass leaves twice the transform
     std::vector<T> kyzc((size_t)h->n[1] * h->nzh);
     const int hz = h->nzh - 1;
+    if (h->n[2] == 1) {
+      // a film's one-launch sweep transforms real rows of ny: ky <= ny/2
+      kyzc.assign((size_t)h->n[1] / 2 + 1, T(0));
+      for (size_t j = 0; j < kyzc.size(); ++j) kyzc[j] = T(0.5) * kyz[j];
+    } else
     for (int j = 0; j < h->n[1]; ++j)
       for (int kz = 0; kz < h->nzh; ++kz)
         kyzc[kz < hz ? (size_t)j * hz + kz : (size_t)h->n[1] * hz + j] = T(0.5) * kyz[(size_t)j * h->nzh + kz];
@@ -404,6 +409,39 @@ static int build_device_tables(ps_handle* h) {
   if (!rc) rc = alloc_copy(h, &B.d_pencil, xw);
   B.h_plane = pw;
   B.h_pencil = xw;
+  // one-launch sweeps in start order (blocks beyond kSweepSegs: none)
+  std::vector<int> order(ne);
+  for (size_t e = 0; e < ne; ++e) order[e] = (int)e;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->sw_start[a] < h->sw_start[b]; });
+  h->levels.clear();
+  h->sw_level.assign(ne, SweepLevel{0, 0, 1});
+  B.h_sweep.clear();
+  bool fits = !h->no_slices;
+  for (int e : order) fits = fits && (int)h->sweeps[h->exec[e]].segs.size() <= kSweepSegs;
+  for (size_t i = 0; i < ne && fits; ++i) {
+    const int e = order[i];
+    const Sweep& sw = h->sweeps[h->exec[e]];
+    SweepWork<T> w;
+    memset(&w, 0, sizeof(w));
+    w.src = sw.jbuf >= 0 ? B.jbuf[sw.jbuf] : nullptr;
+    w.slices = B.slices[e];
+    w.status = &h->d_sc->error_flags;
+    w.total = sw.total;
+    w.dc = B.dcbuf.empty() ? 0 : 1;
+    w.dc_scale = 1.0 / (double)N;
+    for (size_t g = 0; g < sw.segs.size(); ++g) {
+      w.seg[g].wfac = B.wfac[sw.segs[g].wfac_id];
+      w.seg[g].kx = B.kx[sw.segs[g].ktab_id];
+      w.seg[g].kyzc = B.kyzc[sw.segs[g].ktab_id];
+      w.seg[g].end = sw.segs[g].off + sw.segs[g].steps;
+    }
+    if (h->levels.empty() || h->levels.back().k != h->sw_start[e])
+      h->levels.push_back(SweepLevel{h->sw_start[e], (int)i, 0});
+    h->levels.back().cnt++;
+    h->sw_level[e] = SweepLevel{h->sw_start[e], (int)i, 1};
+    B.h_sweep.push_back(w);
+  }
+  if (!rc && fits) rc = alloc_copy(h, &B.d_sweep, B.h_sweep);
   // junction starts for lockstep launches, before the leaving sweep's first step
   B.junc.clear();
   h->junc_off.assign(h->kmax + 1, 0);
@@ -444,6 +482,8 @@ static int launch_sweeps(ps_handle* h, long long* nlaunch, int variant) {
     s.pencil_off = h->sw_pencil_off[e].data();
     s.pencil_cnt = h->sw_pencil_cnt[e].data();
     s.junc = nullptr;  // this chain launches its own junction start below
+    s.levels = &h->sw_level[e];
+    s.nlevels = 1;
     PS_CUDA(h, cudaStreamWaitEvent(h->sw_st[e], h->ev_split, 0));
     const Sweep& sw = h->sweeps[h->exec[e]];
     if (sw.jbuf >= 0) {
@@ -695,7 +735,7 @@ template <typename T> static void free_buffers(Buffers<T>& B) {
   for (auto p : B.kx) f(p);
   for (auto p : B.kyz) f(p);
   for (auto p : B.kyzc) f(p);
-  f(B.tw_x); f(B.tw_y); f(B.tw_z); f(B.tw_zh); f(B.d_plane); f(B.d_pencil);
+  f(B.tw_x); f(B.tw_y); f(B.tw_z); f(B.tw_zh); f(B.d_plane); f(B.d_pencil); f(B.d_sweep);
   B = Buffers<T>();
 }
 

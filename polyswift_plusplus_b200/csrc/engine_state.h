@@ -78,6 +78,8 @@ template <typename T> struct Buffers {
   PencilWork<T>* d_pencil = nullptr;
   std::vector<PlaneWork<T>> h_plane;    // host copies of the work tables
   std::vector<PencilWork<T>> h_pencil;
+  SweepWork<T>* d_sweep = nullptr;      // one-launch sweeps, by start step (ps_handle::levels)
+  std::vector<SweepWork<T>> h_sweep;
   std::vector<JunctionLaunch<T>> junc;  // junction starts, by global step (junc_off/junc_cnt)
 };
 
@@ -124,6 +126,9 @@ struct ps_handle {
   // arriving sweep's final step, and its junction kernel runs in between.
   std::vector<int> sw_start;
   std::vector<int> junc_off, junc_cnt;  // per global step, into Buffers<T>::junc
+  // one-launch sweeps: executed sweeps ordered by start step, and each one alone
+  std::vector<psb::SweepLevel> levels;
+  std::vector<psb::SweepLevel> sw_level;  // by executed sweep
   // the same tables restricted to one executed sweep (VARIANT_SPLIT), and the
   // streams and events of its launch chain
   std::vector<std::vector<int>> sw_plane_off, sw_plane_cnt, sw_pencil_off, sw_pencil_cnt;
@@ -273,6 +278,9 @@ template <typename T> SweepSet<T> handle_sweep_set(ps_handle* h) {
   s.plane_cnt = h->plane_cnt.data();
   s.pencil_off = h->pencil_off.data();
   s.pencil_cnt = h->pencil_cnt.data();
+  s.d_sweep = B.d_sweep;
+  s.levels = h->levels.data();
+  s.nlevels = (int)h->levels.size();
   if (!B.junc.empty()) {
     s.junc = B.junc.data();
     s.junc_off = h->junc_off.data();

@@ -68,6 +68,33 @@ template <typename T> struct PencilWork {
   int dc_first;            // the sweep's first step: no error to feed back
 };
 
+// One whole sweep (sweep_cluster.cuh): its blocks in order, with the global step
+// at which each ends, and its slices (total + 1 of them, N values each).
+constexpr int kSweepSegs = 16;
+template <typename T> struct SweepWork {
+  const T* src;  // initial q (nullptr = ones)
+  T* slices;
+  int* status;      // error word: bit 2 set when a cluster exchange did not arrive in time
+  int total;
+  int dc;           // mean-mode carry (see PlaneWork)
+  double dc_scale;  // 1 / N
+  struct Seg {
+    const T* wfac;
+    const T* kx;
+    const T* kyzc;
+    int end;
+    int pad;
+  } seg[kSweepSegs];
+};
+
+// The grid has a one-launch sweep (a film nx x ny x 1 runs as nx rows of ny).
+bool sweep_cluster_supported(int nx, int ny, int nz);
+template <typename T>
+cudaError_t launch_sweep_cluster(const SweepWork<T>* d_works, int nworks, int nx, int ny, int nz, const c2_t<T>* tw_x,
+                                 const c2_t<T>* tw_y, const c2_t<T>* tw_z, cudaStream_t st);
+// Poll limit of its waits (ps_gpu_set_bulk_wait_limit).
+cudaError_t sweep_cluster_set_polls(uint32_t polls);
+
 bool extent_supported(int n);
 // The fused y-z plane kernel exists for this plane and fits in shared memory.
 bool plane_fused_supported(int prec_bytes, int ny, int nz);
@@ -76,7 +103,8 @@ bool plane_fused_supported(int prec_bytes, int ny, int nz);
 // Kernel variants (chosen by the engine's autotuner, all verified by tests):
 // bit 0: the plane pass with group-local FFTs (step_plane.cuh), for every y-z
 // plane of extents 16 to 128, square or not; bit 1: the x pass in registers
-// (step_pencil.cu) instead of the shared-memory pencil pass.
+// (step_pencil.cu) instead of the shared-memory pencil pass; both, on a grid
+// that has one: every sweep in one launch (sweep_cluster.cuh).
 // bit 2: the sweeps use the row + x-y plane design (transposed half spectrum
 // S[kz][x][y]) instead of the y-z plane + x pencil design.
 // bit 3: each sweep of an instance runs as its own chain of launches on its

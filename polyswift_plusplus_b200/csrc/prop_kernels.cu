@@ -1357,5 +1357,7 @@ cudaError_t launch_pencil<double>(const PencilWork<double>* w, int nw, int mode,
 
 extern "C" int ps_gpu_set_bulk_wait_limit(unsigned int polls) {
   const uint32_t v = (polls == 0xFFFFFFFFu) ? psb::kMaxPolls : (uint32_t)polls;
-  return cudaMemcpyToSymbol(psb::c_bulk_wait_polls, &v, sizeof(v)) == cudaSuccess ? PS_OK : PS_GPU_ERR;
+  cudaError_t e = cudaMemcpyToSymbol(psb::c_bulk_wait_polls, &v, sizeof(v));
+  if (e == cudaSuccess) e = psb::sweep_cluster_set_polls(v);
+  return e == cudaSuccess ? PS_OK : PS_GPU_ERR;
 }

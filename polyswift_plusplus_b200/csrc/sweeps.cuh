@@ -24,6 +24,12 @@ template <typename T> struct JunctionLaunch {
   long long n;
 };
 
+// Sweeps that start at the same global step (one-launch sweeps).
+struct SweepLevel {
+  int k;         // the step before which their junction starts are launched
+  int off, cnt;  // into the sweep works
+};
+
 template <typename T> struct SweepSet {
   int n[3] = {0, 0, 0};
   int nzh = 0;
@@ -40,6 +46,10 @@ template <typename T> struct SweepSet {
   const int* plane_cnt = nullptr;
   const int* pencil_off = nullptr;
   const int* pencil_cnt = nullptr;
+  // one-launch sweeps, by the global step at which they start
+  const SweepWork<T>* d_sweep = nullptr;
+  const SweepLevel* levels = nullptr;
+  int nlevels = 0;
   // junction starts launched before global step k (branched polymers in lockstep)
   const JunctionLaunch<T>* junc = nullptr;
   const int* junc_off = nullptr;
@@ -58,6 +68,13 @@ inline cudaError_t launch_plane_cluster_t(const PlaneWork<T>* w, int nw, int nx,
   return launch_plane_cluster<T>(w, nw, nx, ty, tzh, tz, st);
 }
 
+// Every sweep in one launch.
+template <typename T>
+inline bool resident_path(const SweepSet<T>& s, int variant) {
+  constexpr int both = VARIANT_FUSE_Z | VARIANT_FUSE_K;
+  return (variant & both) == both && !(variant & (VARIANT_XY | VARIANT_CLUSTER)) && s.d_sweep &&
+         sweep_cluster_supported(s.n[0], s.n[1], s.n[2]);
+}
 // The sweeps' spectra are in the compact layout of step_plane.cuh.
 template <typename T>
 inline bool compact_path(const SweepSet<T>& s, int variant) {
@@ -82,6 +99,16 @@ cudaError_t launch_sweep_set(const SweepSet<T>& s, int variant, cudaStream_t st,
     if (e != cudaSuccess) return e; \
     ++*nlaunch;                \
   } while (0)
+  if (resident_path(s, variant)) {
+    for (int l = 0; l < s.nlevels; ++l) {
+      const SweepLevel& v = s.levels[l];
+      if (s.junc)
+        for (int j = s.junc_off[v.k]; j < s.junc_off[v.k] + s.junc_cnt[v.k]; ++j)
+          PSB_L(launch_junction<T>(s.junc[j].in, s.junc[j].n, s.junc[j].out, st));
+      PSB_L(launch_sweep_cluster<T>(s.d_sweep + v.off, v.cnt, nx, ny, nz, s.tw_x, s.tw_y, s.tw_z, st));
+    }
+    return cudaSuccess;
+  }
   for (int k = 0; k <= s.kmax; ++k) {
     if (s.junc)
       for (int j = s.junc_off[k]; j < s.junc_off[k] + s.junc_cnt[k]; ++j)

@@ -1,7 +1,7 @@
 """The step plane pass (variant bit 0) and the x pass in registers (bit 1) over every plane
-shape and x extent they exist for, against the passes they replace (variant 0: the
-shared-memory plane pass, or row and y-pencil passes where no such pass exists) and, on an
-uneven grid, against the FP64 oracle.
+shape and x extent they exist for, and the one-launch sweeps (both bits) over every grid that
+has them, against the passes they replace (variant 0: the shared-memory plane pass, or row
+and y-pencil passes where no such pass exists) and, on an uneven grid, against the FP64 oracle.
 
 Tolerances: both paths compute the same transforms with another order of operations.  FP64:
 about 2 Ns log2(N) roundings of 1e-16, below 1e-12 of the field's maximum.  FP32 sweeps: a
@@ -82,3 +82,84 @@ def test_uneven_grid_matches_oracle(gpu, oracle_lib, precision, tol):
     assert abs(q - h[-1]["q"][0]) <= tol * q
     for a, b in zip(got, [o.w(0), o.w(1), o.phi(0), o.phi(1), o.pressure()]):
         assert np.abs(a - b).max() <= tol * max(1.0, np.abs(b).max())
+
+
+ONE_LAUNCH = [(16, 16, 16), (24, 24, 24), (32, 32, 32), (16, 16, 1), (32, 32, 1), (64, 64, 1), (128, 128, 1)]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", ONE_LAUNCH)
+def test_one_launch_sweeps(gpu, n, precision):
+    """A diblock (a change of block inside each sweep), its shortest blocks, and one launch per
+    sweep set or per sweep."""
+    for ns in (12, 20, 33):
+        tol = 1e-12 if precision == "fp64" else 5e-6
+        cfg, w = _case(n, precision, ns)
+        cfg.polymers[0].blocks[0].force_block_steps = cfg.polymers[0].blocks[1].force_block_steps = True
+        ref, qr = _fields(cfg, w, 0)
+        for v in (3, 11):
+            got, q = _fields(cfg, w, v)
+            assert abs(q - qr) <= tol * qr
+            for a, b in zip(got, ref):
+                assert np.abs(a - b).max() <= tol * max(1.0, np.abs(b).max()), (n, precision, ns, v)
+    s = ScftSolver(cfg)
+    s.set_variant(3)
+    s.restore(w)
+    s.update(2)
+    assert s.launches_per_iteration < 20
+    s.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_one_launch_sweeps_with_junctions_and_in_a_batch(gpu, precision):
+    """Sweeps that start from a junction product, and a batch whose members' sweeps share the
+    launches: bit for bit the single runs."""
+    from polyswift_plusplus_b200.scft import ScftBatch
+    items = [W.star_abc(16, precision=precision), W.star_abc(16, precision=precision, fracs=(0.2, 0.4, 0.4), seed=9)]
+    cfg = W.blend(16, 18.0, 0.35, 0.15, precision=precision, seed=12, anderson=False, ns=20)
+    items.append((cfg, W.random_fields(cfg, 0.3)))
+    tol = 1e-12 if precision == "fp64" else 5e-6
+    single = []
+    for cfg, w in items:
+        out = {}
+        for v in (0, 3, 11):
+            s = ScftSolver(cfg)
+            s.set_variant(v)
+            s.restore(w)
+            s.update(3)
+            out[v] = [s.w(i) for i in range(len(cfg.fields))] + [s.phi(i) for i in range(len(cfg.fields))]
+            s.close()
+        for v in (3, 11):
+            for a, b in zip(out[v], out[0]):
+                assert np.abs(a - b).max() <= tol * max(1.0, np.abs(b).max())
+        single.append(out)
+    for v in (3, 11):
+        with ScftBatch([c for c, _ in items]) as b:
+            b.set_variant(v)
+            for i, (_, w) in enumerate(items):
+                b.instance(i).restore(w)
+            b.update(3)
+            for i, (cfg, _) in enumerate(items):
+                nf = len(cfg.fields)
+                got = [b.instance(i).w(k) for k in range(nf)] + [b.instance(i).phi(k) for k in range(nf)]
+                for a, r in zip(got, single[i][v]):
+                    assert np.array_equal(a, r)
+
+
+def test_one_launch_sweep_wait_timeout_is_reported(gpu, oracle_lib):
+    """With a poll limit of 0 every wait of the cluster exchange gives up: the error flag is
+    reported, the launch ends and the context stays usable."""
+    from polyswift_plusplus_b200 import _abi as A
+    cfg, w = _case((16, 16, 16), "fp64")
+    s = ScftSolver(cfg)
+    s.set_variant(3)
+    s.restore(w)
+    assert gpu.ps_gpu_set_bulk_wait_limit(0) == A.PS_OK
+    try:
+        with pytest.raises(A.PsError) as ei:
+            s.update(1)
+    finally:
+        assert gpu.ps_gpu_set_bulk_wait_limit(0xFFFFFFFF) == A.PS_OK
+    assert ei.value.code == A.PS_GPU_ERR and "wait limit" in str(ei.value)
+    s.close()
+    test_one_launch_sweeps(gpu, (16, 16, 16), "fp64")
