@@ -33,6 +33,11 @@
 // lam^(j)_end += lam_0 prod_{j' != j} q^(j')_end, before that sweep's adjoint
 // starts.
 //
+// On square planes of extents 16 to 128 an adjoint step is two launches
+// (adjoint.cuh, adj_step.cu): the plane pass finishes mu, does the pointwise update
+// and starts the transforms of the next wf lambda and wf q; the x pass forms the
+// stress sums and U's way back.  Elsewhere the passes are separate.
+//
 // Every launch and descriptor is fixed at creation; reductions use a fixed
 // grid and are summed on the host in a fixed order, so results are
 // deterministic.
@@ -44,6 +49,7 @@
 #include <string>
 #include <vector>
 
+#include "adjoint.cuh"
 #include "engine_state.h"
 
 namespace psb {
@@ -56,30 +62,6 @@ struct AccumEntry {
   const double* x;
   const double* y;
   double coef;
-};
-
-struct SrcEntry {
-  const double* gphi;
-  const double* partner;
-  double coef;  // without the 1/Q factor
-};
-
-struct AdjPoint {
-  const double* mu;
-  const double* lam_next;
-  const double* q_s;
-  const double* q_next;
-  const double* w;
-  double* gwb;
-  double* lam_out;   // nullptr: lambda_s is not needed (s = 0)
-  double* dsw_part;  // kAdjRB partials
-  double half_ds;
-  int n_src;
-  SrcEntry src[2];
-  const double* q_partner;  // Q source partner (nullptr: none at this slice)
-  const double* extra;      // adj_init only: junction contributions to lambda (nullptr: none)
-  const double* psi;        // charged block: the exponent is w + facz psi (nullptr: w alone)
-  double facz;
 };
 
 // lam_out[j] += lam0 * prod_{i != j} q_in[i] for the sweeps arriving at a
@@ -143,6 +125,16 @@ __global__ void adj_dot_kernel(const double* __restrict__ a, const double* __res
   if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
 
+// sum (w + facz psi) g
+__global__ void adj_dotw_kernel(const double* __restrict__ w, const double* __restrict__ psi, double facz,
+                                const double* __restrict__ g, long long n, double* __restrict__ part) {
+  __shared__ double sh[kAdjRT];
+  double acc = 0.0;
+  ADJ_LOOP(r, n) acc += (psi ? w[r] + facz * psi[r] : w[r]) * g[r];
+  acc = adj_block_sum(acc, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
+}
+
 // dL/dQ = g_lnQ / Q - (1/Q) sum_f <g_phi_f, phi_f>  (phi carries 1/Q).
 __global__ void adj_gq_kernel(const double* __restrict__ part, double g_lnq, const DevScalars* __restrict__ sc,
                               double* __restrict__ gq) {
@@ -154,6 +146,15 @@ __global__ void adj_gq_kernel(const double* __restrict__ part, double g_lnq, con
     const double q = sc->q[0];
     *gq = g_lnq / q - acc / q;
   }
+}
+
+// out[row] = the sum of row's `stride` partials, in a fixed order.
+__global__ void adj_rows_kernel(const double* __restrict__ part, int stride, double* __restrict__ out) {
+  __shared__ double sh[kAdjRT];
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < stride; i += blockDim.x) acc += part[(size_t)blockIdx.x * stride + i];
+  acc = adj_block_sum(acc, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = acc;
 }
 
 __global__ void adj_kmul_kernel(double2* __restrict__ spec, const double* __restrict__ kx,
@@ -178,7 +179,8 @@ __device__ __forceinline__ double adj_kcomp(int i, int n, double dx) {
 // Re(conj(U) V) * kx*kyz * k_d^2; kx carries 1/N.
 __global__ void adj_stress_kernel(const double2* __restrict__ U, const double2* __restrict__ V,
                                   const double* __restrict__ kx, const double* __restrict__ kyz, int nx,
-                                  int ny, int nz, double dx, double dy, double dz, double* __restrict__ part) {
+                                  int ny, int nz, double dx, double dy, double dz, int stride,
+                                  double* __restrict__ part) {
   __shared__ double sh[kAdjRT];
   const int nzh = nz / 2 + 1;
   const long long n = (long long)nx * ny * nzh;
@@ -201,8 +203,8 @@ __global__ void adj_stress_kernel(const double2* __restrict__ U, const double2* 
   a2 = adj_block_sum(a2, sh);
   if (threadIdx.x == 0) {
     part[blockIdx.x] = a0;
-    part[kAdjRB + blockIdx.x] = a1;
-    part[2 * kAdjRB + blockIdx.x] = a2;
+    part[stride + blockIdx.x] = a1;
+    part[2 * stride + blockIdx.x] = a2;
   }
 }
 
@@ -311,15 +313,22 @@ struct ps_adj {
   double* seg[2] = {nullptr, nullptr};
   double* lam[2] = {nullptr, nullptr};
   double* mu = nullptr;
-  double2* spec[2] = {nullptr, nullptr};
+  double2* spec[2] = {nullptr, nullptr};   // U and V of the adjoint steps
+  double2* rspec[2] = {nullptr, nullptr};  // the recomputed sweeps' (U stays across segments)
   double* P = nullptr;
   double* gwb = nullptr;
   double* gphi = nullptr;
   double* gq = nullptr;
+  // rows of `stride` partials: four per adjoint step (stress x, y, z, explicit ds),
+  // two per block (E, and w . dL/dw of the fused steps), one for <g_phi, phi>; summed by rows into d_sum, read to h_sum
   double* part = nullptr;
-  double* h_part = nullptr;
-  size_t part_len = 0;
+  double* d_sum = nullptr;
+  double* h_sum = nullptr;
+  int stride = 0;
+  size_t rows = 0;
   std::vector<int> slot_block;
+  psb::AdjXWork* d_ax = nullptr;
+  std::vector<psb::AdjXWork> h_ax;
   psb::PlaneWork<double>* d_pw = nullptr;
   psb::PencilWork<double>* d_xw = nullptr;
   psb::AccumEntry* d_acc = nullptr;
@@ -338,7 +347,8 @@ struct ps_adj {
   std::vector<psb::JunctionAdj> h_jn;
   psb::JunctionAdj* d_jn = nullptr;
   size_t storage_bytes = 0;
-  size_t E_off = 0, gq_off = 0;  // offsets (in doubles) into part
+  size_t E_row = 0, W_row = 0, gq_row = 0;  // rows of part
+  double* row(size_t r) const { return part + r * (size_t)stride; }
   bool have_forward = false;
   bool have_backward = false;
 };
@@ -363,6 +373,13 @@ struct Builder {
   ps_handle* h;
   int nx, ny, nz, nzh;
   bool fused;
+  bool step;  // the sweeps run the step plane pass and the register x pass (compact layout)
+  bool adj;   // ... and the adjoint steps their fused forms
+  Builder(ps_adj* a_, ps_handle* h_) : a(a_), h(h_), nx(h_->n[0]), ny(h_->n[1]), nz(h_->n[2]), nzh(h_->nzh) {
+    fused = plane_fused_supported(8, ny, nz);
+    step = step_plane_supported(ny, nz);
+    adj = adj_step_supported(ny, nz);
+  }
 
   const double* wf(int b) const {
     const BlockMap& bm = h->blocks[a->ip][b];
@@ -408,6 +425,7 @@ struct Builder {
     if (b >= 0) {
       x.kx = h->bd.kx[ktab(b)];
       x.kyz = h->bd.kyz[ktab(b)];
+      x.kyzc = h->bd.kyzc[ktab(b)];
     }
     return x;
   }
@@ -444,6 +462,55 @@ struct Builder {
       return launch_pencil<double>(A->d_xw + x0, n, mode, nx_, 1, inner, H->bd.tw_x, nx_, ny_, nz_, st);
     });
   }
+  void step_pass(std::vector<Op>& ops, size_t p0, int n) {
+    ps_adj* A = a;
+    ps_handle* H = h;
+    const int nx_ = nx, ny_ = ny, nz_ = nz;
+    ops.push_back([=](cudaStream_t st) {
+      return launch_step_plane<double>(A->d_pw + p0, n, nx_, ny_, nz_, H->bd.tw_y, H->bd.tw_z, st);
+    });
+  }
+  // Fused adjoint steps.  lam: the lambda work in an adjoint mode with its point;
+  // q: the start of FFT(wf q) for the next step beside it (block -1: none).
+  void lambda_pass(std::vector<Op>& ops, int mode, const AdjPoint& p, const double* win, const double* wout,
+                   const double* q, const double* wq) {
+    const size_t p0 = plane(pw(mode, nullptr, a->spec[0], win, wout, nullptr));
+    int n = 1;
+    if (q) {
+      plane(pw(MODE_FIRST, q, a->spec[1], nullptr, wq, nullptr));
+      n = 2;
+    }
+    a->h_pt.push_back(p);
+    const size_t pi = a->h_pt.size() - 1;
+    ps_adj* A = a;
+    ps_handle* H = h;
+    const int nx_ = nx, ny_ = ny;
+    ops.push_back([=](cudaStream_t st) {
+      const AdjArgs args{A->d_pt + pi, &H->d_sc->q[0], A->gq, (double)A->N};
+      return launch_step_plane_adj(A->d_pw + p0, n, nx_, ny_, H->bd.tw_y, H->bd.tw_z, args, st);
+    });
+  }
+  void q_pass(std::vector<Op>& ops, const double* q, const double* wq) {
+    step_pass(ops, plane(pw(MODE_FIRST, q, a->spec[1], nullptr, wq, nullptr)), 1);
+  }
+  // x pass of an adjoint step of block b: stress sums of slot, U <- IFFT(K U).
+  void stress_x(std::vector<Op>& ops, int b, int slot) {
+    AdjXWork x;
+    x.u = a->spec[0];
+    x.v = a->spec[1];
+    x.kx = h->bd.kx[ktab(b)];
+    x.kyzc = h->bd.kyzc[ktab(b)];
+    x.part = a->row((size_t)slot * 4);
+    a->h_ax.push_back(x);
+    const size_t xi = a->h_ax.size() - 1;
+    ps_adj* A = a;
+    ps_handle* H = h;
+    const int nx_ = nx, ny_ = ny, nz_ = nz;
+    ops.push_back([=](cudaStream_t st) {
+      return launch_adj_x(A->d_ax + xi, nx_, ny_, nz_, H->cfg.cell[0], H->cfg.cell[1], H->cfg.cell[2], A->stride,
+                          H->bd.tw_x, st);
+    });
+  }
   // Lockstep sweeps over `len` steps.  Sweep i runs steps s0[i] .. s0[i]+len-1
   // of sweep sig[i] from slice src[i] (nullptr: ones); store(i, k) gives the
   // destination of its slice k (nullptr: not stored).
@@ -456,21 +523,31 @@ struct Builder {
         const std::vector<int>& bl = a->blk[sig[i]];
         const double* win = (k > 0) ? wf(bl[s0[i] + k - 1]) : nullptr;
         const double* wout = (k < len) ? wf(bl[s0[i] + k]) : nullptr;
-        const size_t p = plane(pw(mode, k == 0 ? src[i] : nullptr, a->spec[i], win, wout, store(i, k)));
-        const size_t y = pencil(xw(a->spec[i], -1));
+        const size_t p = plane(pw(mode, k == 0 ? src[i] : nullptr, a->rspec[i], win, wout, store(i, k)));
+        const size_t y = pencil(xw(a->rspec[i], -1));
         if (i == 0) {
           p0 = p;
           y0 = y;
         }
       }
-      real_pass(ops, p0, nsw, y0, mode);
+      if (step) step_pass(ops, p0, nsw);
+      else real_pass(ops, p0, nsw, y0, mode);
       if (k < len) {
         size_t x0 = 0;
         for (int i = 0; i < nsw; ++i) {
-          const size_t x = pencil(xw(a->spec[i], a->blk[sig[i]][s0[i] + k]));
+          const size_t x = pencil(xw(a->rspec[i], a->blk[sig[i]][s0[i] + k]));
           if (i == 0) x0 = x;
         }
-        x_pass(ops, x0, nsw, PENCIL_KINV);
+        if (step) {
+          ps_adj* A = a;
+          ps_handle* H = h;
+          const int nx_ = nx, inner = ny * nzh;
+          ops.push_back([=](cudaStream_t st) {
+            return launch_step_pencil<double>(A->d_xw + x0, nsw, nx_, inner, true, H->bd.tw_x, st);
+          });
+        } else {
+          x_pass(ops, x0, nsw, PENCIL_KINV);
+        }
       }
     }
   }
@@ -516,12 +593,36 @@ static void fill_sources(ps_adj* a, AdjPoint& p, int sig, int idx, int j) {
 // One adjoint step through block b: mu = wf G(wf lam_next), the stress
 // partials of (U, V) = (FFT(wf lam_next), FFT(wf q_s)), dL/dw of the step and,
 // when lam_out is set, lam_s = mu + the explicit sources of slice s (in `src`).
+static AdjPoint step_point(Builder& B, int b, int slot, const double* q_s, const double* q_next,
+                           const double* lam_next, double* lam_out, const AdjPoint& src, int b2 = -1) {
+  ps_adj* a = B.a;
+  ps_handle* h = B.h;
+  const BlockMap& bm = h->blocks[a->ip][b];
+  AdjPoint p = src;
+  if (b2 >= 0) {
+    p.gwb2 = a->gwb + (size_t)b2 * a->N;
+    p.half_ds2 = 0.5 * h->blocks[a->ip][b2].ds;
+  }
+  p.mu = a->mu;
+  p.lam_next = lam_next;
+  p.q_s = q_s;
+  p.q_next = q_next;
+  p.w = h->d_w + (size_t)bm.field * a->N;
+  p.gwb = a->gwb + (size_t)b * a->N;
+  p.lam_out = lam_out;
+  p.dsw_part = a->row((size_t)slot * 4 + 3);
+  p.half_ds = 0.5 * bm.ds;
+  p.extra = nullptr;
+  p.psi = (bm.charge_field >= 0) ? h->d_psi + (size_t)bm.charge_field * a->N : nullptr;
+  p.facz = bm.facz;
+  return p;
+}
+
 static void adjoint_step_p(Builder& B, std::vector<Op>& ops, int b, const double* q_s, const double* q_next,
                            const double* lam_next, double* lam_out, const AdjPoint& src) {
   ps_adj* a = B.a;
   ps_handle* h = B.h;
   const double* wfb = B.wf(b);
-  const BlockMap& bm = h->blocks[a->ip][b];
   const int slot = (int)a->slot_block.size();
   a->slot_block.push_back(b);
   // U = FFT(wf lam_{s+1}) in spec[0], V = FFT(wf q_s) in spec[1]
@@ -536,10 +637,11 @@ static void adjoint_step_p(Builder& B, std::vector<Op>& ops, int b, const double
   const int kt = B.ktab(b);
   const int nx = B.nx, ny = B.ny, nz = B.nz;
   const double dx = h->cfg.cell[0], dy = h->cfg.cell[1], dz = h->cfg.cell[2];
-  const size_t poff = (size_t)slot * 4 * kAdjRB;
+  double* const part = a->row((size_t)slot * 4);
+  const int stride = a->stride;
   ops.push_back([=](cudaStream_t st) {
     adj_stress_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->spec[0], a->spec[1], h->bd.kx[kt], h->bd.kyz[kt], nx, ny,
-                                                   nz, dx, dy, dz, a->part + poff);
+                                                   nz, dx, dy, dz, stride, part);
     return cudaGetLastError();
   });
   const int inner = ny * B.nzh;
@@ -552,19 +654,7 @@ static void adjoint_step_p(Builder& B, std::vector<Op>& ops, int b, const double
   const size_t p1 = B.plane(B.pw(MODE_LAST, nullptr, a->spec[0], wfb, nullptr, a->mu));
   const size_t y1 = B.pencil(B.xw(a->spec[0], -1));
   B.real_pass(ops, p1, 1, y1, MODE_LAST);
-  AdjPoint p = src;
-  p.mu = a->mu;
-  p.lam_next = lam_next;
-  p.q_s = q_s;
-  p.q_next = q_next;
-  p.w = h->d_w + (size_t)bm.field * a->N;
-  p.gwb = a->gwb + (size_t)b * a->N;
-  p.lam_out = lam_out;
-  p.dsw_part = a->part + poff + 3 * kAdjRB;
-  p.half_ds = 0.5 * bm.ds;
-  p.extra = nullptr;
-  p.psi = (bm.charge_field >= 0) ? h->d_psi + (size_t)bm.charge_field * a->N : nullptr;
-  p.facz = bm.facz;
+  const AdjPoint p = step_point(B, b, slot, q_s, q_next, lam_next, lam_out, src);
   a->h_pt.push_back(p);
   const size_t pi = a->h_pt.size() - 1;
   const long long N = a->N;
@@ -581,6 +671,41 @@ static void adjoint_step(Builder& B, std::vector<Op>& ops, int sig, int s, int j
   if (s >= 1) fill_sources(a, src, sig, s, j);
   adjoint_step_p(B, ops, a->blk[sig][s], slice_ptr(a, sig, s, j), slice_ptr(a, sig, s + 1, j), a->lam[cur],
                  (s >= 1) ? a->lam[1 - cur] : nullptr, src);
+}
+
+// The adjoint steps seg_hi - 1 .. seg_lo of sweep sig while segment j is resident,
+// fused: one plane pass and one x pass a step.  At the sweep's end (first) lambda
+// starts there; at later segments only q's transform is missing.
+static void adjoint_segment(Builder& B, std::vector<Op>& ops, int sig, int j, int lo, int hi, bool first, int& cur) {
+  ps_adj* a = B.a;
+  const std::vector<int>& bl = a->blk[sig];
+  const double* wtop = B.wf(bl[hi - 1]);
+  if (first) {
+    AdjPoint p;
+    memset(&p, 0, sizeof(p));
+    p.lam_out = a->lam[cur];
+    p.q_s = slice_ptr(a, sig, hi, j);
+    p.gwb2 = a->gwb + (size_t)bl[hi - 1] * a->N;
+    p.half_ds2 = 0.5 * B.h->blocks[a->ip][bl[hi - 1]].ds;
+    fill_sources(a, p, sig, hi, j);
+    B.lambda_pass(ops, MODE_ADJ_INIT, p, nullptr, wtop, slice_ptr(a, sig, hi - 1, j), wtop);
+  } else {
+    B.q_pass(ops, slice_ptr(a, sig, hi - 1, j), wtop);
+  }
+  for (int s = hi - 1; s >= lo; --s) {
+    const int slot = (int)a->slot_block.size();
+    a->slot_block.push_back(bl[s]);
+    B.stress_x(ops, bl[s], slot);
+    AdjPoint src;
+    memset(&src, 0, sizeof(src));
+    if (s >= 1) fill_sources(a, src, sig, s, j);
+    const AdjPoint p = step_point(B, bl[s], slot, slice_ptr(a, sig, s, j), slice_ptr(a, sig, s + 1, j), a->lam[cur],
+                                  (s >= 1) ? a->lam[1 - cur] : nullptr, src, s >= 1 ? bl[s - 1] : -1);
+    const double* wn = (s >= 1) ? B.wf(bl[s - 1]) : nullptr;
+    B.lambda_pass(ops, s >= 1 ? MODE_ADJ_MID : MODE_ADJ_LAST, p, B.wf(bl[s]), wn,
+                  s > lo ? slice_ptr(a, sig, s - 1, j) : nullptr, wn);
+    cur = 1 - cur;
+  }
 }
 
 static void adjoint_init(ps_adj* a, std::vector<Op>& ops, int sig, int j, int cur) {
@@ -614,6 +739,39 @@ static BlockFieldMap field_map(ps_adj* a) {
   return fm;
 }
 
+
+static void push_dotw(Builder& B, std::vector<Op>& ops) {
+  if (!B.adj) return;
+  ps_adj* a = B.a;
+  ps_handle* h = B.h;
+  const long long N = a->N;
+  for (int b = 0; b < a->nb; ++b) {
+    const BlockMap& bm = h->blocks[a->ip][b];
+    const double* w = h->d_w + (size_t)bm.field * N;
+    const double* psi = (bm.charge_field >= 0) ? h->d_psi + (size_t)bm.charge_field * N : nullptr;
+    const double facz = bm.facz;
+    ops.push_back([=](cudaStream_t st) {
+      adj_dotw_kernel<<<kAdjRB, kAdjRT, 0, st>>>(w, psi, facz, a->gwb + (size_t)b * N, N, a->row(a->W_row + b));
+      return cudaGetLastError();
+    });
+  }
+}
+
+// Partials of `steps` adjoint steps.
+static int alloc_partials(ps_adj* a, size_t steps) {
+  ps_handle* h = a->h;
+  a->stride = std::max(std::max(kAdjRB, h->n[0]), adj_x_tiles(h->n[0], h->n[1] * h->nzh));
+  a->E_row = steps * 4;
+  a->W_row = a->E_row + (size_t)a->nb;
+  a->gq_row = a->W_row + (size_t)a->nb;
+  a->rows = a->gq_row + 1;
+  const size_t n = a->rows * (size_t)a->stride;
+  PA_CUDA(a, cudaMalloc((void**)&a->part, sizeof(double) * n));
+  PA_CUDA(a, cudaMemset(a->part, 0, sizeof(double) * n));
+  PA_CUDA(a, cudaMalloc((void**)&a->d_sum, sizeof(double) * a->rows));
+  PA_CUDA(a, cudaMallocHost((void**)&a->h_sum, sizeof(double) * a->rows));
+  return PS_OK;
+}
 
 // Branched chain (see the header): every slice stored by the engine's sweeps.
 static int tree_build(ps_adj* a, int ec) {
@@ -718,27 +876,18 @@ static int tree_build(ps_adj* a, int ec) {
   PA_CUDA(a, cudaMalloc((void**)&a->gphi, NB * a->nf));
   PA_CUDA(a, cudaMemset(a->gphi, 0, NB * a->nf));
   PA_CUDA(a, cudaMalloc((void**)&a->gq, sizeof(double)));
-  a->E_off = (size_t)steps_total * 4 * kAdjRB;
-  a->gq_off = a->E_off + (size_t)a->nb * kAdjRB;
-  a->part_len = a->gq_off + kAdjRB;
-  PA_CUDA(a, cudaMalloc((void**)&a->part, sizeof(double) * a->part_len));
-  PA_CUDA(a, cudaMemset(a->part, 0, sizeof(double) * a->part_len));
-  PA_CUDA(a, cudaMallocHost((void**)&a->h_part, sizeof(double) * a->part_len));
+  {
+    int rp = alloc_partials(a, (size_t)steps_total);
+    if (rp) return rp;
+  }
   // a->P was sized before the accumulation entries pointed at it
-  Builder B;
-  B.a = a;
-  B.h = h;
-  B.nx = h->n[0];
-  B.ny = h->n[1];
-  B.nz = h->n[2];
-  B.nzh = h->nzh;
-  B.fused = plane_fused_supported(8, h->n[1], h->n[2]);
+  Builder B(a, h);
   const BlockFieldMap fm = field_map(a);
 
   // ---- forward: the engine's sweeps (every slice stored), Q, quadrature
   a->fwd.push_back([h](cudaStream_t) {
     long long nl = 0;
-    return engine_sweeps(h, &nl, 0) == PS_OK ? cudaSuccess : cudaErrorLaunchFailure;
+    return engine_sweeps(h, &nl, VARIANT_FUSE_Z | VARIANT_FUSE_K) == PS_OK ? cudaSuccess : cudaErrorLaunchFailure;
   });
   {
     const double* qx = S(qh_sw, qh_i);
@@ -763,14 +912,14 @@ static int tree_build(ps_adj* a, int ec) {
   {
     const long long nfN = (long long)a->nf * N;
     a->bwd.push_back([=](cudaStream_t st) {
-      adj_dot_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->gphi, h->d_phi, nfN, a->part + a->gq_off);
+      adj_dot_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->gphi, h->d_phi, nfN, a->row(a->gq_row));
       return cudaGetLastError();
     });
     for (int b = 0; b < a->nb; ++b) {
       const int f = h->blocks[ip][b].field;
       a->bwd.push_back([=](cudaStream_t st) {
         adj_dot_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->gphi + (size_t)f * N, a->P + (size_t)b * N, N,
-                                                  a->part + a->E_off + (size_t)b * kAdjRB);
+                                                  a->row(a->E_row + b));
         return cudaGetLastError();
       });
     }
@@ -786,7 +935,34 @@ static int tree_build(ps_adj* a, int ec) {
       const int T = swp.total;
       const bool junction = !swp.jin.empty();
       int cur = 0;
-      {
+      if (B.adj) {
+        // fused steps; every slice is stored, so q's transform always goes along
+        const std::vector<int>& bl = a->tblk[t];
+        AdjPoint p0;
+        memset(&p0, 0, sizeof(p0));
+        p0.lam_out = a->lam[cur];
+        p0.q_s = S(sw, T);
+        p0.gwb2 = a->gwb + (size_t)bl[T - 1] * N;
+        p0.half_ds2 = 0.5 * h->blocks[ip][bl[T - 1]].ds;
+        fill(p0, t, T);
+        p0.extra = a->jacc[t];
+        B.lambda_pass(a->bwd, MODE_ADJ_INIT, p0, nullptr, B.wf(bl[T - 1]), S(sw, T - 1), B.wf(bl[T - 1]));
+        for (int st_ = T - 1; st_ >= 0; --st_) {
+          const int slot = (int)a->slot_block.size();
+          a->slot_block.push_back(bl[st_]);
+          B.stress_x(a->bwd, bl[st_], slot);
+          AdjPoint src_;
+          memset(&src_, 0, sizeof(src_));
+          const bool out = (st_ >= 1) || junction;
+          if (out) fill(src_, t, st_);
+          const AdjPoint p = step_point(B, bl[st_], slot, S(sw, st_), S(sw, st_ + 1), a->lam[cur],
+                                        out ? a->lam[1 - cur] : nullptr, src_, st_ >= 1 ? bl[st_ - 1] : -1);
+          const double* wn = (st_ >= 1) ? B.wf(bl[st_ - 1]) : nullptr;
+          B.lambda_pass(a->bwd, st_ >= 1 ? MODE_ADJ_MID : MODE_ADJ_LAST, p, B.wf(bl[st_]), wn,
+                        st_ >= 1 ? S(sw, st_ - 1) : nullptr, wn);
+          if (out) cur = 1 - cur;
+        }
+      } else {
         AdjPoint p;
         memset(&p, 0, sizeof(p));
         p.lam_out = a->lam[cur];
@@ -799,7 +975,7 @@ static int tree_build(ps_adj* a, int ec) {
           return cudaGetLastError();
         });
       }
-      for (int st_ = T - 1; st_ >= 0; --st_) {
+      for (int st_ = T - 1; st_ >= 0 && !B.adj; --st_) {
         AdjPoint p;
         memset(&p, 0, sizeof(p));
         const bool out = (st_ >= 1) || junction;
@@ -826,10 +1002,12 @@ static int tree_build(ps_adj* a, int ec) {
       }
     }
   }
+  push_dotw(B, a->bwd);
   int r2 = adj_upload(a, &a->d_pw, a->h_pw);
   if (!r2) r2 = adj_upload(a, &a->d_xw, a->h_xw);
   if (!r2) r2 = adj_upload(a, &a->d_acc, a->h_acc);
   if (!r2) r2 = adj_upload(a, &a->d_pt, a->h_pt);
+  if (!r2) r2 = adj_upload(a, &a->d_ax, a->h_ax);
   if (!r2) r2 = adj_upload(a, &a->d_jn, a->h_jn);
   return r2;
 }
@@ -947,6 +1125,7 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
     if (C > 1) PA_CUDA(a, cudaMalloc((void**)&a->seg[sg], NB * (C + 1)));
     PA_CUDA(a, cudaMalloc((void**)&a->lam[sg], NB));
     PA_CUDA(a, cudaMalloc((void**)&a->spec[sg], sizeof(double2) * nspec));
+    PA_CUDA(a, cudaMalloc((void**)&a->rspec[sg], sizeof(double2) * nspec));
   }
   a->storage_bytes = NB * (2 * (size_t)a->J + 2 + (C > 1 ? 2 * (size_t)(C + 1) : 0));
   PA_CUDA(a, cudaMalloc((void**)&a->mu, NB));
@@ -955,21 +1134,12 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
   PA_CUDA(a, cudaMalloc((void**)&a->gphi, NB * a->nf));
   PA_CUDA(a, cudaMemset(a->gphi, 0, NB * a->nf));
   PA_CUDA(a, cudaMalloc((void**)&a->gq, sizeof(double)));
-  a->E_off = (size_t)2 * M * 4 * kAdjRB;
-  a->gq_off = a->E_off + (size_t)a->nb * kAdjRB;
-  a->part_len = a->gq_off + kAdjRB;
-  PA_CUDA(a, cudaMalloc((void**)&a->part, sizeof(double) * a->part_len));
-  PA_CUDA(a, cudaMemset(a->part, 0, sizeof(double) * a->part_len));
-  PA_CUDA(a, cudaMallocHost((void**)&a->h_part, sizeof(double) * a->part_len));
+  {
+    int rp = alloc_partials(a, (size_t)2 * M);
+    if (rp) return rp;
+  }
 
-  Builder B;
-  B.a = a;
-  B.h = h;
-  B.nx = h->n[0];
-  B.ny = h->n[1];
-  B.nz = h->n[2];
-  B.nzh = h->nzh;
-  B.fused = plane_fused_supported(8, h->n[1], h->n[2]);
+  Builder B(a, h);
   const BlockFieldMap fm = field_map(a);
   const long long N = a->N;
 
@@ -1025,14 +1195,14 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
   {
     const long long nfN = (long long)a->nf * N;
     a->bwd.push_back([=](cudaStream_t st) {
-      adj_dot_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->gphi, h->d_phi, nfN, a->part + a->gq_off);
+      adj_dot_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->gphi, h->d_phi, nfN, a->row(a->gq_row));
       return cudaGetLastError();
     });
     for (int b = 0; b < a->nb; ++b) {
       const int f = h->blocks[a->ip][b].field;
       a->bwd.push_back([=](cudaStream_t st) {
         adj_dot_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->gphi + (size_t)f * N, a->P + (size_t)b * N, N,
-                                                  a->part + a->E_off + (size_t)b * kAdjRB);
+                                                  a->row(a->E_row + b));
         return cudaGetLastError();
       });
     }
@@ -1041,6 +1211,10 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
     int cur = 0;
     for (int j = a->J - 1; j >= 0; --j) {
       recompute(B, a->bwd, j);
+      if (B.adj) {
+        adjoint_segment(B, a->bwd, 0, j, a->seg_a[j], a->seg_b[j], j == a->J - 1, cur);
+        continue;
+      }
       if (j == a->J - 1) adjoint_init(a, a->bwd, 0, j, cur);
       for (int s = a->seg_b[j] - 1; s >= a->seg_a[j]; --s) {
         adjoint_step(B, a->bwd, 0, s, j, cur);
@@ -1051,6 +1225,10 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
     cur = 0;
     for (int j = 0; j < a->J; ++j) {
       recompute(B, a->bwd, j);
+      if (B.adj) {
+        adjoint_segment(B, a->bwd, 1, j, M - a->seg_b[j], M - a->seg_a[j], j == 0, cur);
+        continue;
+      }
       if (j == 0) adjoint_init(a, a->bwd, 1, j, cur);
       for (int m = M - a->seg_a[j] - 1; m >= M - a->seg_b[j]; --m) {
         adjoint_step(B, a->bwd, 1, m, j, cur);
@@ -1058,10 +1236,12 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
       }
     }
   }
+  push_dotw(B, a->bwd);
   int r2 = adj_upload(a, &a->d_pw, a->h_pw);
   if (!r2) r2 = adj_upload(a, &a->d_xw, a->h_xw);
   if (!r2) r2 = adj_upload(a, &a->d_acc, a->h_acc);
   if (!r2) r2 = adj_upload(a, &a->d_pt, a->h_pt);
+  if (!r2) r2 = adj_upload(a, &a->d_ax, a->h_ax);
   return r2;
 }
 
@@ -1077,6 +1257,7 @@ static void adj_free(ps_adj* a) {
     f(a->seg[sg]);
     f(a->lam[sg]);
     f(a->spec[sg]);
+    f(a->rspec[sg]);
   }
   f(a->mu);
   f(a->P);
@@ -1084,7 +1265,9 @@ static void adj_free(ps_adj* a) {
   f(a->gphi);
   f(a->gq);
   f(a->part);
-  if (a->h_part) cudaFreeHost(a->h_part);
+  f(a->d_sum);
+  f(a->d_ax);
+  if (a->h_sum) cudaFreeHost(a->h_sum);
   f(a->d_pw);
   f(a->d_xw);
   f(a->d_acc);
@@ -1244,13 +1427,15 @@ int ps_adj_backward(ps_adj* a, const double* g_phi, double g_log_q, double* g_w,
   PA_CUDA(a, cudaMemcpyAsync(a->gphi, g_phi, sizeof(double) * (size_t)a->nf * N, cudaMemcpyDeviceToDevice,
                              h->st));
   PA_CUDA(a, a->bwd[0](h->st));
-  adj_gq_kernel<<<1, kAdjRT, 0, h->st>>>(a->part + a->gq_off, g_log_q, h->d_sc, a->gq);
+  adj_gq_kernel<<<1, kAdjRT, 0, h->st>>>(a->row(a->gq_row), g_log_q, h->d_sc, a->gq);
   PA_CUDA(a, cudaGetLastError());
   int rc = run_ops(a, a->bwd, 1);
   if (rc) return rc;
   adj_sum_blocks_kernel<<<kAdjRB, kAdjRT, 0, h->st>>>(a->gwb, field_map(a), N, g_w);
   PA_CUDA(a, cudaGetLastError());
-  PA_CUDA(a, cudaMemcpyAsync(a->h_part, a->part, sizeof(double) * a->part_len, cudaMemcpyDeviceToHost, h->st));
+  adj_rows_kernel<<<(unsigned)a->rows, kAdjRT, 0, h->st>>>(a->part, a->stride, a->d_sum);
+  PA_CUDA(a, cudaGetLastError());
+  PA_CUDA(a, cudaMemcpyAsync(a->h_sum, a->d_sum, sizeof(double) * a->rows, cudaMemcpyDeviceToHost, h->st));
   PA_CUDA(a, cudaStreamSynchronize(h->st));
   // host sums in a fixed order
   double gbox[3] = {0.0, 0.0, 0.0};
@@ -1259,19 +1444,15 @@ int ps_adj_backward(ps_adj* a, const double* g_phi, double g_log_q, double* g_w,
   for (size_t slot = 0; slot < a->slot_block.size(); ++slot) {
     const int b = a->slot_block[slot];
     const BlockMap& bm = h->blocks[a->ip][b];
-    const double* p = a->h_part + slot * 4 * kAdjRB;
-    double R[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int q = 0; q < 4; ++q)
-      for (int i = 0; i < kAdjRB; ++i) R[q] += p[q * kAdjRB + i];
+    const double* R = a->h_sum + slot * 4;
     const double b2 = bm.bseg * bm.bseg;
     for (int d = 0; d < 3; ++d) gbox[d] += 2.0 * bm.ds * b2 / L[d] * R[d];
     gds[b] += -b2 * (R[0] + R[1] + R[2]) + R[3];
   }
-  for (int b = 0; b < a->nb; ++b) {
-    double E = 0.0;
-    for (int i = 0; i < kAdjRB; ++i) E += a->h_part[a->E_off + (size_t)b * kAdjRB + i];
-    gds[b] += E / h->blocks[a->ip][b].ds;
-  }
+  // the fused steps' explicit ds derivative: sum over the block's steps of -1/2 (w, t)
+  // with dL/dw = sum of -ds/2 t
+  for (int b = 0; b < a->nb; ++b)
+    gds[b] += (a->h_sum[a->E_row + b] + a->h_sum[a->W_row + b]) / h->blocks[a->ip][b].ds;
   if (g_box)
     for (int d = 0; d < 3; ++d) g_box[d] = gbox[d];
   if (g_ds)

@@ -40,6 +40,7 @@
 // to the k^2 table kyzc: exact, and four multiplies fewer per pair).
 #pragma once
 
+#include "adjoint.cuh"
 #include "step_common.cuh"
 
 namespace psb {
@@ -110,6 +111,12 @@ template <typename T, int U> struct RealRun {
 #pragma unroll
     for (int i = 0; i < U; ++i) v[i] = reinterpret_cast<const T*>(&x)[i];
   }
+  __device__ __forceinline__ void load_plain(const T* p) {
+    using V = typename Reals<T, U>::type;
+    const V x = *reinterpret_cast<const V*>(p);
+#pragma unroll
+    for (int i = 0; i < U; ++i) v[i] = reinterpret_cast<const T*>(&x)[i];
+  }
   __device__ __forceinline__ void store(T* p) const {
     using V = typename Reals<T, U>::type;
     V x;
@@ -119,15 +126,101 @@ template <typename T, int U> struct RealRun {
   }
 };
 
-template <typename T, int NY, int NZ>
-__global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, NZ>::MINB))
+// The real-space part of an adjoint step (adjoint.cuh) at M runs of U adjacent
+// points.  load() fetches every stream before any is used (one run at a time the
+// pass was a chain of L2 latencies: 30 us at 64^3); apply() turns mu (has_mu) into
+// the next lambda, in x.
+template <int U, int M> struct AdjRuns {
+  using Run = RealRun<double, U>;
+  Run q[M], gp[M], pt[M], gw[M];
+  __device__ __forceinline__ void fetch(Run (&r)[M], const double* base, const size_t (&at)[M]) {
+#pragma unroll
+    for (int m = 0; m < M; ++m) r[m].load(base + at[m]);
+  }
+  __device__ __forceinline__ void load(const AdjPoint& p, const size_t (&at)[M]) {
+    fetch(q, p.q_s, at);
+    if (p.lam_out && p.n_src > 0) {
+      fetch(gp, p.src[0].gphi, at);
+      fetch(pt, p.src[0].partner, at);
+    }
+    const double* g = p.gwb ? p.gwb : p.gwb2;
+#pragma unroll
+    for (int m = 0; m < M; ++m) gw[m].load_plain(g + at[m]);
+  }
+  __device__ __forceinline__ void apply(const AdjPoint& p, const AdjGlobals& g, const size_t (&at)[M], bool has_mu,
+                                        Run (&x)[M]) {
+    const bool lam = p.lam_out != nullptr, src = lam && p.n_src > 0;
+    Run l[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (!has_mu) x[m].v[u] = 0.0;
+        l[m].v[u] = src ? x[m].v[u] + (g.inv_q * p.src[0].coef) * (gp[m].v[u] * pt[m].v[u]) : x[m].v[u];
+      }
+    if (lam) {
+      for (int i = 1; i < p.n_src; ++i) {  // a block joint: two quadrature pairs
+        fetch(gp, p.src[i].gphi, at);
+        fetch(pt, p.src[i].partner, at);
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+          for (int u = 0; u < U; ++u) l[m].v[u] += (g.inv_q * p.src[i].coef) * (gp[m].v[u] * pt[m].v[u]);
+      }
+      if (p.q_partner) {
+        fetch(gp, p.q_partner, at);
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+          for (int u = 0; u < U; ++u) l[m].v[u] += g.gq_n * gp[m].v[u];
+      }
+      if (p.extra) {
+        fetch(gp, p.extra, at);
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+          for (int u = 0; u < U; ++u) l[m].v[u] += gp[m].v[u];
+      }
+#pragma unroll
+      for (int m = 0; m < M; ++m) l[m].store(p.lam_out + at[m]);
+    }
+    const bool one = (p.gwb == p.gwb2);
+    if (p.gwb) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          gw[m].v[u] -= p.half_ds * q[m].v[u] * (one ? x[m].v[u] + l[m].v[u] : x[m].v[u]);
+        gw[m].store(p.gwb + at[m]);
+      }
+    }
+    if (p.gwb2 && !one) {
+      if (p.gwb) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) gw[m].load_plain(p.gwb2 + at[m]);
+      }
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) gw[m].v[u] -= p.half_ds2 * q[m].v[u] * l[m].v[u];
+        gw[m].store(p.gwb2 + at[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) x[m] = l[m];
+  }
+};
+
+// ADJ (FP64): works in the adjoint modes of adjoint.cuh beside FIRST ones.
+template <typename T, int NY, int NZ, bool ADJ>
+__global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (ADJ ? 1 : StepPlane<T, NY, NZ>::MINB))
     step_plane_kernel(const PlaneWork<T>* __restrict__ works, const c2_t<T>* __restrict__ tw_y,
-                      const c2_t<T>* __restrict__ tw_z) {
+                      const c2_t<T>* __restrict__ tw_z, AdjArgs adj) {
   using P = StepPlane<T, NY, NZ>;
   using C = c2_t<T>;
   constexpr int H = P::H, PR = P::PR, S = P::S, TH = P::TH, CG = P::CG, PA = P::PA;
   constexpr int GY = P::GY, RY = P::RY, UY = P::UY, GZ = P::GZ, RZ = P::RZ, UZ = P::UZ;
-  constexpr int GH = GY / 2, CH = P::CH;
+  constexpr int GH = GY / 2, CH = (ADJ && UZ == 2) ? 1 : P::CH;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
   C* s_nyq = buf + PR * S;  // column 0 on its way out, to separate the Nyquist column
@@ -144,7 +237,10 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
   const int mc = (c == 0) ? H : NZ - c;
   C* const spec = w.spec + (size_t)blockIdx.x * (NY * (H + 1)) + c;
   const size_t roff = (size_t)blockIdx.x * (NY * NZ);
-  const bool dc_sum = (w.mode != MODE_LAST) && (w.dc_out != nullptr);
+  const bool adj_on = ADJ && w.mode >= MODE_ADJ_INIT;
+  const bool inverse = w.mode != MODE_FIRST && !(ADJ && w.mode == MODE_ADJ_INIT);
+  const bool forward = w.mode != MODE_LAST && !(ADJ && w.mode == MODE_ADJ_LAST);
+  const bool dc_sum = forward && (w.dc_out != nullptr);
 
   for (int i = tid; i < NY; i += TH) s_tw_y[i] = tw_y[i];
   for (int i = tid; i < NZ; i += TH) s_tw_z[i] = tw_z[i];
@@ -153,7 +249,7 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
 
   // exchange slot d of column c: row d % (ny/2) of column c, or of its mirror
   C* const slot_j = buf + (j % GH) * RY * S + (j < GH ? c : mc);  // slots j RY + r
-  if (w.mode != MODE_FIRST) {
+  if (inverse) {
     dc_hilo_store<T>(w.dc_in);  // used after the barriers below
     C v[RY];
 #pragma unroll
@@ -198,6 +294,14 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
 
   // z rows: inverse, real-space step, forward
   T acc = T(0);
+  const AdjPoint* const point = ADJ ? adj.points + blockIdx.y : nullptr;
+  AdjGlobals globals{0.0, 0.0};
+  if constexpr (ADJ) {
+    if (adj_on) {
+      globals.inv_q = 1.0 / *adj.q;
+      globals.gq_n = *adj.gq / adj.n;
+    }
+  }
 #pragma unroll 1
   for (int task = tid; task < P::TASKS; task += TH) {
     const int b = task / GZ, jz = task % GZ;
@@ -209,7 +313,7 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
     // the Boltzmann factors (FIRST: the initial q) of CH positions at a time: the
     // first ones are loaded ahead of the exchange, the next while the previous
     // ones are used
-    const T* const lead = (w.mode == MODE_FIRST) ? w.src : w.wfac_in;
+    const T* const lead = inverse ? w.wfac_in : w.src;
     const bool lead_on = on && lead;
     RealRun<T, UZ> f[2][CH], f2[2][CH];
     auto load_lead = [&](int s, int r0) {
@@ -224,7 +328,24 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
       }
     };
     load_lead(0, 0);
-    if (w.mode != MODE_FIRST) {
+    // ADJ: the pointwise streams, where registers allow one chunk ahead
+    constexpr bool AHEAD = ADJ && UZ == 1;
+    AdjRuns<UZ, ADJ ? 2 * CH : 1> runs[AHEAD ? 2 : 1];
+    auto adj_load = [&](int i, int r0) {
+      if constexpr (ADJ) {
+        size_t at[2 * CH];
+#pragma unroll
+        for (int k = 0; k < CH; ++k) {
+          at[2 * k] = ra + RZ * (r0 + k);
+          at[2 * k + 1] = at[2 * k] + (size_t)PR * NZ;
+        }
+        runs[i].load(*point, at);
+      }
+    };
+    if constexpr (AHEAD) {
+      if (adj_on && on) adj_load(0, 0);
+    }
+    if (inverse) {
       C v[RZ];
 #pragma unroll
       for (int r = 0; r < RZ; ++r) v[r] = row[jz + GZ * r];
@@ -265,40 +386,53 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
         for (int r = 0; r < GZ; ++r) q[u][r] = C{T(1), T(1)};
     }
     if (on) {
-      const bool same = (w.wfac_in == w.wfac_out) && w.mode != MODE_FIRST;
-      const bool dc_in = (w.mode != MODE_FIRST) && w.dc_in;
+      const bool same = (w.wfac_in == w.wfac_out) && inverse;
+      const bool dc_in = inverse && w.dc_in;
 #pragma unroll
       for (int r0 = 0; r0 < GZ; r0 += CH) {
         const int s = (r0 / CH) & 1;
         if (r0 + CH < GZ) load_lead(s ^ 1, r0 + CH);
+RealRun<T, UZ> xs[2 * CH];  // the rows' values at the chunk's positions
+        size_t at[2 * CH];
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
           const int r = r0 + i;
-          const size_t at = ra + RZ * r, at2 = at + (size_t)PR * NZ;
-          RealRun<T, UZ> x, x2;
+          at[2 * i] = ra + RZ * r;
+          at[2 * i + 1] = at[2 * i] + (size_t)PR * NZ;
 #pragma unroll
           for (int u = 0; u < UZ; ++u) {
             const C a = dc_in ? dc_add2<T>(q[u][r]) : q[u][r];
-            x.v[u] = a.x * f[s][i].v[u];
-            x2.v[u] = a.y * f2[s][i].v[u];
+            xs[2 * i].v[u] = a.x * f[s][i].v[u];
+            xs[2 * i + 1].v[u] = a.y * f2[s][i].v[u];
           }
+        }
+        if constexpr (ADJ) {
+          if (adj_on) {
+            if (AHEAD && r0 + CH < GZ) adj_load((r0 / CH + 1) & 1, r0 + CH);
+            if (!AHEAD) adj_load(0, r0);
+            runs[AHEAD ? (r0 / CH) & 1 : 0].apply(*point, globals, at, inverse, xs);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+          const int r = r0 + i;
           if (w.store) {
-            x.store(w.store + at);
-            x2.store(w.store + at2);
+            xs[2 * i].store(w.store + at[2 * i]);
+            xs[2 * i + 1].store(w.store + at[2 * i + 1]);
           }
           if (!same) {
             f[s][i].ones();
             f2[s][i].ones();
-            if (w.wfac_out && w.mode != MODE_LAST) {
-              f[s][i].load(w.wfac_out + at);
-              f2[s][i].load(w.wfac_out + at2);
+            if (w.wfac_out && forward) {
+              f[s][i].load(w.wfac_out + at[2 * i]);
+              f2[s][i].load(w.wfac_out + at[2 * i + 1]);
             }
           }
 #pragma unroll
-          for (int u = 0; u < UZ; ++u) q[u][r] = C{x.v[u] * f[s][i].v[u], x2.v[u] * f2[s][i].v[u]};
+          for (int u = 0; u < UZ; ++u) q[u][r] = C{xs[2 * i].v[u] * f[s][i].v[u], xs[2 * i + 1].v[u] * f2[s][i].v[u]};
         }
       }
-      if (w.mode != MODE_LAST) {
+      if (forward) {
 #pragma unroll
         for (int u = 0; u < UZ; ++u) {
           Dft<GZ, false, C>::run(q[u]);
@@ -316,7 +450,7 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
         }
       }
     }
-    if (w.mode == MODE_LAST) continue;
+    if (!forward) continue;
     __syncwarp();
     C v[RZ];
     if constexpr (P::V2) {
@@ -337,7 +471,7 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (StepPlane<T, NY, 
 #pragma unroll
     for (int r = 0; r < RZ; ++r) row[jz + GZ * r] = v[r];
   }
-  if (w.mode == MODE_LAST) return;  // uniform over the CTA
+  if (!forward) return;  // uniform over the CTA
   if (dc_sum) dc_warp_sum((double)acc);
   __syncthreads();  // every column complete
 
@@ -398,11 +532,11 @@ template <typename T, int NY, int NZ>
 cudaError_t launch_step_plane_t(const PlaneWork<T>* d_works, int nworks, int nx, const c2_t<T>* tw_y,
                                 const c2_t<T>* tw_z, cudaStream_t st) {
   using P = StepPlane<T, NY, NZ>;
-  auto kern = step_plane_kernel<T, NY, NZ>;
+  auto kern = step_plane_kernel<T, NY, NZ, false>;
   static unsigned attr_mask = 0;
   cudaError_t e = ensure_smem_attr(kern, P::SMEM, &attr_mask);
   if (e != cudaSuccess) return e;
-  return launch_sweep_kernel(kern, dim3(nx, nworks), dim3(P::TH), P::SMEM, st, d_works, tw_y, tw_z);
+  return launch_sweep_kernel(kern, dim3(nx, nworks), dim3(P::TH), P::SMEM, st, d_works, tw_y, tw_z, AdjArgs{});
 }
 
 // Planes of NY rows, for every nz of kStepExtents (one translation unit per NY).
