@@ -264,7 +264,12 @@ static int build_device_tables(ps_handle* h) {
     if (!h->no_slices) PS_CUDA(h, cudaMalloc((void**)&sl, sizeof(T) * (size_t)(sw.total + 1) * N));
     B.slices.push_back(sl);
     c2_t<T>* sp = nullptr;
-    PS_CUDA(h, cudaMalloc((void**)&sp, sizeof(c2_t<T>) * (size_t)h->n[0] * h->n[1] * h->nzh));
+    size_t ns = (size_t)h->n[0] * h->n[1] * h->nzh;
+    if (step_split_supported(h->n[1], h->n[2]))
+      ns = std::max(ns, step_split_spectrum((int)sizeof(T), h->n[0], h->n[1], h->n[2]));
+    PS_CUDA(h, cudaMalloc((void**)&sp, sizeof(c2_t<T>) * ns));
+    // the split layout's padding columns are transformed with the others
+    if (step_split_supported(h->n[1], h->n[2])) PS_CUDA(h, cudaMemset(sp, 0, sizeof(c2_t<T>) * ns));
     B.spec.push_back(sp);
   }
   for (size_t i = 0; i < h->wfac_keys.size(); ++i) {
@@ -388,6 +393,7 @@ static int build_device_tables(ps_handle* h) {
         PencilWork<T> x;
         memset(&x, 0, sizeof(x));
         x.spec = B.spec[e];
+        x.status = &h->d_sc->error_flags;
         x.kx = B.kx[seg_of(sw, kl).ktab_id];
         x.kyz = B.kyz[seg_of(sw, kl).ktab_id];
         x.kyzc = B.kyzc[seg_of(sw, kl).ktab_id];

@@ -66,6 +66,7 @@ template <typename T> struct PencilWork {
   double* dc_err;          // ... the rounding the previous step's mean lost (error feedback)
   double dc_scale;         // 1 / N
   int dc_first;            // the sweep's first step: no error to feed back
+  int* status;             // error word: bit 2 set when a bulk copy did not land in time
 };
 
 // One whole sweep (sweep_cluster.cuh): its blocks in order, with the global step
@@ -104,7 +105,8 @@ bool plane_fused_supported(int prec_bytes, int ny, int nz);
 // bit 0: the plane pass with group-local FFTs (step_plane.cuh), for every y-z
 // plane of extents 16 to 128, square or not; bit 1: the x pass in registers
 // (step_pencil.cu) instead of the shared-memory pencil pass; both, on a grid
-// that has one: every sweep in one launch (sweep_cluster.cuh).
+// that has one: every sweep in one launch (sweep_cluster.cuh), and on 256 x 256
+// planes without bit 4: the step with the y transform split (step_split.cuh).
 // bit 2: the sweeps use the row + x-y plane design (transposed half spectrum
 // S[kz][x][y]) instead of the y-z plane + x pencil design.
 // bit 3: each sweep of an instance runs as its own chain of launches on its
@@ -161,6 +163,17 @@ cudaError_t launch_step_plane(const PlaneWork<T>* d_works, int nworks, int nx, i
 template <typename T>
 cudaError_t launch_step_pencil(const PencilWork<T>* d_works, int nworks, int L, int inner, bool compact,
                                const c2_t<T>* tw, cudaStream_t st);
+
+// The step with the y transform split over the two passes (step_split.cuh), and the
+// complex values its spectrum takes.
+bool step_split_supported(int ny, int nz);
+size_t step_split_spectrum(int prec_bytes, int nx, int ny, int nz);
+template <typename T>
+cudaError_t launch_split_plane(const PlaneWork<T>* d_works, int nworks, int nx, const c2_t<T>* tw_y,
+                               const c2_t<T>* tw_z, cudaStream_t st);
+template <typename T>
+cudaError_t launch_split_pencil(const PencilWork<T>* d_works, int nworks, int nx, int nz, const c2_t<T>* tw_x,
+                                cudaStream_t st);
 
 // Pencils of length L along an axis of stride `inner` (elements), `outer`
 // independent groups of L*inner elements; dims used only by PENCIL_KFULL.

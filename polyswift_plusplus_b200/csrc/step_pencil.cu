@@ -34,6 +34,7 @@ __global__ void __launch_bounds__((PencilG<T, L>::TH))
   constexpr int G = P::G, R = P::R, U = P::U, TK = P::TK, TH = P::TH;
   __shared__ C buf[L * TK];
   __shared__ C s_tw[L];
+  __shared__ T s_kx[L];
   const PencilWork<T> w = works[blockIdx.y];
   const int tid = threadIdx.x;
   const int cc = tid % TK, j = tid / TK;
@@ -41,12 +42,15 @@ __global__ void __launch_bounds__((PencilG<T, L>::TH))
   const bool in = c < inner;
   C* const base = w.spec + c;
   const bool dc0 = w.dc_total && blockIdx.x == 0;  // mean-mode carry: see PlaneWork
-  for (int i = tid; i < L; i += TH) s_tw[i] = tw[i];
+  for (int i = tid; i < L; i += TH) {
+    s_tw[i] = tw[i];
+    s_kx[i] = __ldg(w.kx + i);
+  }
+  const T fyz = in ? __ldg((compact ? w.kyzc : w.kyz) + c) : T(0);
   pdl_wait();  // before any read or write of the spectrum
   C v[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) v[r] = in ? __ldcg(base + (size_t)(j + G * r) * inner) : C{T(0), T(0)};
-  const T fyz = in ? __ldg((compact ? w.kyzc : w.kyz) + c) : T(0);
   DcFinish<T> dcf;
   if (dc0 && tid < 32) dcf.load(w);
   Dft<R, false, C>::run(v);
@@ -67,7 +71,7 @@ __global__ void __launch_bounds__((PencilG<T, L>::TH))
       Dft<G, false, C>::run(b);
 #pragma unroll
       for (int r = 0; r < G; ++r) {
-        const T f = __ldg(w.kx + jp + R * r) * fyz;
+        const T f = s_kx[jp + R * r] * fyz;
         b[r] = C{b[r].x * f, b[r].y * f};
       }
       if (dc0 && c == 0 && jp == 0) b[0] = C{T(0), T(0)};

@@ -74,7 +74,7 @@ template <typename T, int NY, int NZ> struct StepPlane {
   // 18.1 with one and 19.3 with four), the others for four (64^2 FP64: 5.8 us
   // for 128 planes, 6.0 with one; 128^2 FP64: 40.0, 42.3)
   static constexpr int CH = (sizeof(T) == 4 && UZ == 2 && GZ == 8) ? 2 : 4;
-  static constexpr size_t SMEM = sizeof(c2_t<T>) * ((size_t)PR * S + 2 * NY + NZ);
+  static constexpr size_t SMEM = sizeof(c2_t<T>) * ((size_t)PR * S + 2 * NY + 2 * NZ);
   // registers: FP32 64 and FP64 128 a thread
   static constexpr int BY_REG = 65536 / (TH * (sizeof(T) == 4 ? 64 : 128));
   static constexpr int BY_SMEM = (int)((size_t)224 * 1024 / (SMEM + 1024));
@@ -225,7 +225,8 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (ADJ ? 1 : StepPla
   C* buf = reinterpret_cast<C*>(smem_raw);
   C* s_nyq = buf + PR * S;  // column 0 on its way out, to separate the Nyquist column
   C* s_tw_y = s_nyq + NY;
-  C* s_tw_z = s_tw_y + NY;
+  C* s_twb = s_tw_y + NY;  // exp(-2 pi i r j / nz) as [r][j] for the radix-GZ passes
+  C* s_twf = s_twb + NZ;   // ... and for the radix-RZ ones: consecutive lanes, consecutive banks
 
   const PlaneWork<T> w = works[blockIdx.y];
   const int tid = threadIdx.x;
@@ -243,7 +244,10 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (ADJ ? 1 : StepPla
   const bool dc_sum = forward && (w.dc_out != nullptr);
 
   for (int i = tid; i < NY; i += TH) s_tw_y[i] = tw_y[i];
-  for (int i = tid; i < NZ; i += TH) s_tw_z[i] = tw_z[i];
+  for (int i = tid; i < NZ; i += TH) {
+    s_twb[i] = tw_z[(i / RZ) * (i % RZ)];
+    s_twf[i] = tw_z[(i / GZ) * (i % GZ)];
+  }
   __syncthreads();  // the groups below read tables that other groups wrote
   pdl_wait();       // before any read of the spectrum, src or wfac, and any write
 
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (ADJ ? 1 : StepPla
 #pragma unroll
         for (int u = 0; u < UZ; ++u) {
 #pragma unroll
-          for (int r = 1; r < GZ; ++r) q[u][r] = cmulc(q[u][r], s_tw_z[r * (j0 + u)]);
+          for (int r = 1; r < GZ; ++r) q[u][r] = cmulc(q[u][r], s_twb[r * RZ + j0 + u]);
           Dft<GZ, true, C>::run(q[u]);
         }
       }
@@ -465,7 +469,7 @@ RealRun<T, UZ> xs[2 * CH];  // the rows' values at the chunk's positions
       for (int r = 0; r < RZ; ++r) v[r] = row[jz * PA + r];
     }
 #pragma unroll
-    for (int r = 1; r < RZ; ++r) v[r] = cmul(v[r], s_tw_z[r * jz]);
+    for (int r = 1; r < RZ; ++r) v[r] = cmul(v[r], s_twf[r * GZ + jz]);
     Dft<RZ, false, C>::run(v);
     __syncwarp();
 #pragma unroll

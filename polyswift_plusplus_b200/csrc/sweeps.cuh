@@ -80,6 +80,12 @@ template <typename T>
 inline bool compact_path(const SweepSet<T>& s, int variant) {
   return (variant & VARIANT_FUSE_Z) && step_plane_supported(s.n[1], s.n[2]);
 }
+// The y transform split over the two passes.
+template <typename T>
+inline bool split_path(const SweepSet<T>& s, int variant) {
+  constexpr int both = VARIANT_FUSE_Z | VARIANT_FUSE_K;
+  return (variant & both) == both && !(variant & VARIANT_CLUSTER) && step_split_supported(s.n[1], s.n[2]);
+}
 template <typename T>
 inline cudaError_t launch_x_pass(const SweepSet<T>& s, const PencilWork<T>* w, int nw, bool compact, int variant,
                                  cudaStream_t st) {
@@ -121,6 +127,9 @@ cudaError_t launch_sweep_set(const SweepSet<T>& s, int variant, cudaStream_t st,
     if ((variant & VARIANT_XY) && s.xy_ok) {
       PSB_L(launch_rows_t<T>(pw, np, nx, ny, nz, s.tw_zh, s.tw_z, st));
       if (nxw > 0) PSB_L(launch_xy<T>(xw, nxw, nx, s.nzh, s.tw_x, variant, st));
+    } else if (split_path(s, variant)) {
+      PSB_L(launch_split_plane<T>(pw, np, nx, s.tw_y, s.tw_z, st));
+      if (nxw > 0) PSB_L(launch_split_pencil<T>(xw, nxw, nx, nz, s.tw_x, st));
     } else if (compact_path(s, variant)) {
       PSB_L(launch_step_plane<T>(pw, np, nx, ny, nz, s.tw_y, s.tw_z, st));
       if (nxw > 0) PSB_L(launch_x_pass<T>(s, xw, nxw, true, variant, st));
