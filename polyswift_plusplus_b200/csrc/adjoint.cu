@@ -893,9 +893,11 @@ static int tree_build(ps_adj* a, int ec) {
     const double* qx = S(qh_sw, qh_i);
     const double* qy = S(qt_sw, qt_i);
     a->fwd.push_back([=](cudaStream_t st) {
-      cudaError_t e = launch_dot_partials<double>(qx, qy, N, h->d_qpart, st);
-      if (e == cudaSuccess) e = launch_finalize_q(h->d_qpart, (double)N, 0, h->d_sc, st);
-      return e;
+      BigQSet<double> set;
+      set.n = 1;
+      set.a[0] = qx;
+      set.b[0] = qy;
+      return launch_big_q<double>(set, N, h->d_qpart, h->d_count, h->d_sc, st);
     });
     a->fwd.push_back([=](cudaStream_t st) { return cudaMemsetAsync(a->P, 0, sizeof(double) * N * a->nb, st); });
     const int ne = (int)a->h_acc.size();
@@ -1160,9 +1162,11 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
     const double* qx = (a->n0 == 0) ? a->ck[0] : a->endq[0];
     const double* qy = (a->n0 == 0) ? a->endq[1] : a->ck[1] + (size_t)(a->J - 1) * N;
     a->fwd.push_back([=](cudaStream_t st) {
-      cudaError_t e = launch_dot_partials<double>(qx, qy, N, h->d_qpart, st);
-      if (e == cudaSuccess) e = launch_finalize_q(h->d_qpart, (double)N, 0, h->d_sc, st);
-      return e;
+      BigQSet<double> set;
+      set.n = 1;
+      set.a[0] = qx;
+      set.b[0] = qy;
+      return launch_big_q<double>(set, N, h->d_qpart, h->d_count, h->d_sc, st);
     });
     // quadrature, segment by segment
     a->fwd.push_back([=](cudaStream_t st) { return cudaMemsetAsync(a->P, 0, sizeof(double) * N * a->nb, st); });

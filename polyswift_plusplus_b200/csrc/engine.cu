@@ -513,24 +513,44 @@ static int launch_sweeps(ps_handle* h, long long* nlaunch, int variant) {
   return PS_OK;
 }
 
+// One quadrature launch covers every block (charged ones read their field's phi
+// between blocks), and it writes phi outright when nothing was added before.
+static bool quadrature_in_one(const ps_handle* h) {
+  size_t n = 0;
+  for (const auto& bs : h->blocks)
+    for (const BlockMap& b : bs) {
+      if (b.charge_field >= 0) return false;
+      ++n;
+    }
+  return n <= (size_t)kQuadMax;
+}
+static bool quadrature_overwrites(const ps_handle* h) { return quadrature_in_one(h) && h->cfg.n_solvents == 0; }
+
 template <typename T>
 static int launch_pre(ps_handle* h, long long* nlaunch) {
   Buffers<T>& B = bufs<T>(h);
   const long long N = h->N;
-  PS_CUDA(h, launch_zero(h->d_phi, (long long)h->nf * N, h->st));
-  ++*nlaunch;
+  if (!quadrature_overwrites(h)) {
+    PS_CUDA(h, launch_zero(h->d_phi, (long long)h->nf * N, h->st));
+    ++*nlaunch;
+  }
   if (h->nq > 0) {
     // PsChargeDens::update: resetDensField (psphysf/PsChargeDens.cpp:180-190)
     PS_CUDA(h, launch_zero(h->d_rho, (long long)h->nq * N, h->st));
     ++*nlaunch;
   }
-  for (size_t i = 0; i < h->wfac_keys.size(); ++i) {
-    const WfacKey& k = h->wfac_keys[i];
-    if (k.charge_field < 0)
-      PS_CUDA(h, launch_wfac<T>(h->d_w + (size_t)k.field * N, B.wfac[i], -0.5 * k.ds, N, h->st));
-    else
-      PS_CUDA(h, launch_wfac_charged<T>(h->d_w + (size_t)k.field * N, h->d_psi + (size_t)k.charge_field * N,
-                                        B.wfac[i], -0.5 * k.ds, k.facz, N, h->st));
+  for (size_t i0 = 0; i0 < h->wfac_keys.size(); i0 += kWfacMax) {
+    WfacSet<T> set;
+    set.n = (int)std::min<size_t>(kWfacMax, h->wfac_keys.size() - i0);
+    for (int i = 0; i < set.n; ++i) {
+      const WfacKey& k = h->wfac_keys[i0 + i];
+      set.key[i].w = h->d_w + (size_t)k.field * N;
+      set.key[i].psi = k.charge_field < 0 ? nullptr : h->d_psi + (size_t)k.charge_field * N;
+      set.key[i].out = B.wfac[i0 + i];
+      set.key[i].ds2 = -0.5 * k.ds;
+      set.key[i].facz = k.facz;
+    }
+    PS_CUDA(h, launch_wfac<T>(set, N, h->st));
     ++*nlaunch;
   }
   return PS_OK;
@@ -577,19 +597,34 @@ static int launch_post(ps_handle* h, long long* nlaunch) {
                                 h->d_qpart, h->d_sc, h->d_phi + (size_t)S.field * N, h->st));
     *nlaunch += 3;
   }
+  BigQSet<T> qset;
+  qset.n = h->cfg.n_polymers;
   for (int ip = 0; ip < h->cfg.n_polymers; ++ip) {
     const BlockMap& b0 = h->blocks[ip][0];
-    PS_CUDA(h, launch_dot_partials<T>(slice(b0.sweep_head, b0.off_head),
-                                      slice(b0.sweep_tail, b0.off_tail + b0.steps), N, h->d_qpart,
-                                      h->st));
-    PS_CUDA(h, launch_finalize_q(h->d_qpart, (double)N, ip, h->d_sc, h->st));
-    *nlaunch += 2;
+    qset.a[ip] = slice(b0.sweep_head, b0.off_head);
+    qset.b[ip] = slice(b0.sweep_tail, b0.off_tail + b0.steps);
   }
+  PS_CUDA(h, launch_big_q<T>(qset, N, h->d_qpart, h->d_count, h->d_sc, h->st));
+  ++*nlaunch;
+  const bool in_one = quadrature_in_one(h);
+  QuadSet<T> quad;
   for (int ip = 0; ip < h->cfg.n_polymers; ++ip) {
     // densWt vf / lengthRatio (pspolymer/PsBlock.cpp:164-172); densWt = 1 or w_k / Gamma(alpha)
     const double densfac = h->chain_dwt[ip] * h->chain_vf[ip] / h->alpha[ip];
     for (size_t ib = 0; ib < h->blocks[ip].size(); ++ib) {
       const BlockMap& b = h->blocks[ip][ib];
+      if (in_one) {
+        auto& q = quad.block[quad.n++];
+        q.qs = slice(b.sweep_head, b.off_head);
+        q.qts = slice(b.sweep_tail, b.off_tail);
+        q.steps = b.steps;
+        q.simp = 0.33333 * b.ds;
+        q.trap = b.ds * 0.5;
+        q.densfac = densfac;
+        q.ip = ip;
+        q.field = b.field;
+        continue;
+      }
       PS_CUDA(h, launch_quadrature<T>(slice(b.sweep_head, b.off_head), slice(b.sweep_tail, b.off_tail),
                                       b.steps, N, b.ds, densfac, h->d_sc, ip,
                                       h->d_phi + (size_t)b.field * N, h->st));
@@ -602,6 +637,10 @@ static int launch_post(ps_handle* h, long long* nlaunch) {
         ++*nlaunch;
       }
     }
+  }
+  if (in_one) {
+    PS_CUDA(h, launch_quadrature_all<T>(quad, N, h->nf, h->d_sc, h->d_phi, !quadrature_overwrites(h), h->st));
+    ++*nlaunch;
   }
   // the field update is the first reader of p: wait for an asynchronous upload
   // of it (an external event-wait node when this is being captured)
@@ -627,15 +666,14 @@ static int launch_post(ps_handle* h, long long* nlaunch) {
     const int m = h->cfg.updater.anderson_depth;
     PS_CUDA(h, launch_am_residual(h->fm, fp, h->d_hw, h->d_hd, h->am_slots, h->d_sc, h->d_upart, h->st));
     PS_CUDA(h, launch_am_gram((long long)h->nf * N, h->d_hd, h->am_slots, m, h->d_sc, h->d_gpart, h->st));
-    PS_CUDA(h, launch_am_solve(h->d_gpart, h->d_gram, h->am_slots, m, h->cfg.updater.anderson_start,
+    PS_CUDA(h, launch_am_solve((long long)h->nf * N, h->d_gpart, h->d_gram, h->am_slots, m, h->cfg.updater.anderson_start,
                                h->cfg.updater.anderson_mix, h->cfg.updater.lambda0, h->d_sc, h->st));
-    PS_CUDA(h, launch_am_mix(h->fm, fp, h->d_hw, h->d_hd, h->am_slots, h->d_sc, h->d_upart, h->st));
-    PS_CUDA(h, launch_update_finalize_am(h->fm, h->d_upart, h->d_sc, h->st));
-    *nlaunch += 5;
+    PS_CUDA(h, launch_am_mix(h->fm, fp, h->d_hw, h->d_hd, h->am_slots, h->d_sc, h->d_upart,
+                             h->d_count + PS_MAX_POLYMERS, h->st));
+    *nlaunch += 4;
   } else {
-    PS_CUDA(h, launch_sd_update(h->fm, fp, h->d_upart, h->st));
-    PS_CUDA(h, launch_update_finalize(h->fm, h->d_upart, h->d_sc, h->st));
-    *nlaunch += 2;
+    PS_CUDA(h, launch_sd_update(h->fm, fp, h->d_upart, h->d_count + PS_MAX_POLYMERS, h->d_sc, h->st));
+    ++*nlaunch;
   }
   PS_CUDA(h, launch_pressure_shift(h->d_p, N, h->d_sc, h->st));
   ++*nlaunch;
@@ -755,7 +793,7 @@ static void free_all(ps_handle* h) {
   f(h->d_w); f(h->d_phi); f(h->d_p); f(h->d_noise); f(h->d_rho); f(h->d_psi);
   free_buffers(h->bf);
   free_buffers(h->bd);
-  f(h->d_qpart); f(h->d_upart); f(h->d_sc);
+  f(h->d_qpart); f(h->d_count); f(h->d_upart); f(h->d_sc);
   if (h->h_sc) cudaFreeHost(h->h_sc);
   f(h->d_hw); f(h->d_hd); f(h->d_gram); f(h->d_gpart);
   if (h->ev_cap_start) cudaEventDestroy(h->ev_cap_start);
@@ -1137,7 +1175,9 @@ static int create_impl(ps_handle* h, const ps_config* ucfg) {
     int rn = noise_setup(h);
     if (rn) return rn;
   }
-  PS_CUDA(h, cudaMalloc((void**)&h->d_qpart, sizeof(double) * kRedBlocks));
+  PS_CUDA(h, cudaMalloc((void**)&h->d_qpart, sizeof(double) * kRedBlocks * (size_t)std::max(1, c.n_polymers)));
+  PS_CUDA(h, cudaMalloc((void**)&h->d_count, sizeof(unsigned) * (PS_MAX_POLYMERS + 1)));
+  PS_CUDA(h, cudaMemset(h->d_count, 0, sizeof(unsigned) * (PS_MAX_POLYMERS + 1)));
   PS_CUDA(h, cudaMalloc((void**)&h->d_upart, sizeof(double) * kRedBlocks * kUpdQ));
   PS_CUDA(h, cudaMemset(h->d_upart, 0, sizeof(double) * kRedBlocks * kUpdQ));
   PS_CUDA(h, cudaMalloc((void**)&h->d_sc, sizeof(DevScalars)));

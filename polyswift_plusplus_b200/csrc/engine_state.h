@@ -140,6 +140,7 @@ struct ps_handle {
   psb::Buffers<double> bd;
 
   double* d_qpart = nullptr;
+  unsigned* d_count = nullptr;  // finished CTAs: one per polymer's Q, one for the update (0 between launches)
   double* d_upart = nullptr;
   psb::DevScalars* d_sc = nullptr;
   psb::DevScalars* h_sc = nullptr;  // pinned

@@ -8,6 +8,7 @@
 #include <math.h>
 
 #include "field_kernels.cuh"
+#include "step_common.cuh"
 
 namespace psb {
 
@@ -67,29 +68,87 @@ __device__ double cta_reduce_partials(const double* p, int n, int stride, bool i
   return r;
 }
 
+// The same sums (or maxima, by bit of max_mask) of NQ interleaved quantities at
+// once: each is added in cta_reduce_partials' order.  L2 loads: other CTAs of this
+// launch wrote the partials.
+template <int NQ>
+__device__ __forceinline__ void cta_reduce_many(const double* p, int n, int stride, unsigned max_mask,
+                                                double (&out)[NQ]) {
+  __shared__ double sh[NQ][kRedThreads];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    double x = 0.0;
+    for (int i = threadIdx.x; i < n; i += kRedThreads) {
+      const double y = __ldcg(p + (size_t)i * stride + q);
+      x = ((max_mask >> q) & 1u) ? fmax(x, y) : x + y;
+    }
+    sh[q][threadIdx.x] = x;
+  }
+  __syncthreads();
+  for (int s = kRedThreads / 2; s > 0; s >>= 1) {
+    if (threadIdx.x < s) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const double a = sh[q][threadIdx.x], b = sh[q][threadIdx.x + s];
+        sh[q][threadIdx.x] = ((max_mask >> q) & 1u) ? fmax(a, b) : a + b;
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) out[q] = sh[q][0];
+  __syncthreads();
+}
+
+// True in every thread of the CTA that finishes last of `blocks` (its threads then
+// see what the others wrote before); resets the count for the next launch.
+__device__ __forceinline__ bool last_block(unsigned* count, unsigned blocks) {
+  __shared__ unsigned s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = (atomicAdd(count, 1u) == blocks - 1) ? 1u : 0u;
+    if (s_last) *count = 0;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last != 0;
+}
+
+// CTAs of a reduction over n points: those beyond would only add zeros.
+static inline int red_blocks(long long n) {
+  const long long b = (n + kRedThreads - 1) / kRedThreads;
+  return (int)(b < 1 ? 1 : (b > kRedBlocks ? kRedBlocks : b));
+}
+
 // ---------------------------------------------------------------------------
 // wfac = exp(-ds/2 w)   (pspolymer/PsFlexPseudoSpec.cpp:170-177)
 // ---------------------------------------------------------------------------
+// Charged blocks (pspolymer/PsChargeFlexPseudoSpec.cpp:97-130): times
+// exp(facZ ds2 psi), facZ = za alpha L.  One launch covers every (field, ds) table.
 template <typename T>
-__global__ void wfac_kernel(const double* __restrict__ w, T* __restrict__ wfac, double ds2,
-                            long long N) {
+__global__ void wfac_kernel(WfacSet<T> set, long long N) {
+  pdl_wait();
+  const typename WfacSet<T>::Key k = set.key[blockIdx.y];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
-       i += (long long)gridDim.x * blockDim.x)
-    wfac[i] = (T)exp(ds2 * w[i]);
+       i += (long long)gridDim.x * blockDim.x) {
+    const double e = exp(k.ds2 * k.w[i]);
+    k.out[i] = (T)(k.psi ? e * exp(k.facz * k.ds2 * k.psi[i]) : e);
+  }
 }
 
 template <typename T>
-cudaError_t launch_wfac(const double* w, T* wfac, double ds2, long long N, cudaStream_t st) {
+cudaError_t launch_wfac(const WfacSet<T>& set, long long N, cudaStream_t st) {
   int blocks = (int)((N + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
-  wfac_kernel<T><<<blocks, 256, 0, st>>>(w, wfac, ds2, N);
-  return cudaGetLastError();
+  return launch_sweep_kernel(wfac_kernel<T>, dim3(blocks, set.n), dim3(256), 0, st, set, N);
 }
-template cudaError_t launch_wfac<float>(const double*, float*, double, long long, cudaStream_t);
-template cudaError_t launch_wfac<double>(const double*, double*, double, long long, cudaStream_t);
+template cudaError_t launch_wfac<float>(const WfacSet<float>&, long long, cudaStream_t);
+template cudaError_t launch_wfac<double>(const WfacSet<double>&, long long, cudaStream_t);
 
 template <typename T>
 __global__ void junction_kernel(JunctionIn<T> in, long long N, T* __restrict__ out) {
+  pdl_wait();
   for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < N;
        r += (long long)gridDim.x * blockDim.x) {
     T p = T(1);
@@ -102,8 +161,7 @@ template <typename T>
 cudaError_t launch_junction(const JunctionIn<T>& in, long long N, T* out, cudaStream_t st) {
   int blocks = (int)((N + 255) / 256);
   if (blocks > 148 * 8) blocks = 148 * 8;
-  junction_kernel<T><<<blocks, 256, 0, st>>>(in, N, out);
-  return cudaGetLastError();
+  return launch_sweep_kernel(junction_kernel<T>, dim3(blocks), dim3(256), 0, st, in, N, out);
 }
 template cudaError_t launch_junction<float>(const JunctionIn<float>&, long long, float*, cudaStream_t);
 template cudaError_t launch_junction<double>(const JunctionIn<double>&, long long, double*, cudaStream_t);
@@ -124,43 +182,43 @@ cudaError_t launch_zero(double* p, long long n, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Q = <qHeadInitial * qHeadFinal>  (pspolymer/PsBlock.cpp:204-237)
 // ---------------------------------------------------------------------------
+// One launch for every polymer: partial sums, and the last CTA of each polymer turns
+// them into Q.
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads)
-    dot_partials_kernel(const T* __restrict__ a, const T* __restrict__ b, long long N,
-                        double* __restrict__ partials) {
+    big_q_kernel(BigQSet<T> set, long long N, double* __restrict__ partials, unsigned* __restrict__ count,
+                 DevScalars* __restrict__ sc) {
+  pdl_wait();
+  const int ip = blockIdx.y;
+  const T* __restrict__ a = set.a[ip];
+  const T* __restrict__ b = set.b[ip];
+  double* const part = partials + (size_t)ip * kRedBlocks;
   double v[1] = {0.0};
   for (long long i = blockIdx.x * (long long)kRedThreads + threadIdx.x; i < N;
-       i += (long long)kRedBlocks * kRedThreads)
+       i += (long long)gridDim.x * kRedThreads)
     v[0] += (0.0 + (double)a[i]) * (double)b[i];
-  block_reduce_write<1>(v, 0u, partials + blockIdx.x);
-}
-
-template <typename T>
-cudaError_t launch_dot_partials(const T* a, const T* b, long long N, double* partials,
-                                cudaStream_t st) {
-  dot_partials_kernel<T><<<kRedBlocks, kRedThreads, 0, st>>>(a, b, N, partials);
-  return cudaGetLastError();
-}
-template cudaError_t launch_dot_partials<float>(const float*, const float*, long long, double*,
-                                                cudaStream_t);
-template cudaError_t launch_dot_partials<double>(const double*, const double*, long long, double*,
-                                                 cudaStream_t);
-
-__global__ void finalize_q_kernel(const double* partials, double N, int ip, DevScalars* sc) {
-  double tot = cta_reduce_partials(partials, kRedBlocks, 1, false);
+  block_reduce_write<1>(v, 0u, part + blockIdx.x);
+  if (!last_block(count + ip, gridDim.x)) return;
+  double tot[1];
+  cta_reduce_many<1>(part, gridDim.x, 1, 0u, tot);
   if (threadIdx.x == 0) {
-    double q = tot / (1.0 * N);
+    const double q = tot[0] / (1.0 * (double)N);
     sc->q[ip] = q;
     sc->log_q[ip] = log(q);
-    if (q != q) sc->error_flags |= 1;
+    if (q != q) atomicOr(&sc->error_flags, 1);
   }
 }
 
-cudaError_t launch_finalize_q(const double* partials, double N, int ip, DevScalars* sc,
-                              cudaStream_t st) {
-  finalize_q_kernel<<<1, kRedThreads, 0, st>>>(partials, N, ip, sc);
-  return cudaGetLastError();
+template <typename T>
+cudaError_t launch_big_q(const BigQSet<T>& set, long long N, double* partials, unsigned* count, DevScalars* sc,
+                         cudaStream_t st) {
+  return launch_sweep_kernel(big_q_kernel<T>, dim3(red_blocks(N), set.n), dim3(kRedThreads), 0, st, set, N, partials,
+                             count, sc);
 }
+template cudaError_t launch_big_q<float>(const BigQSet<float>&, long long, double*, unsigned*, DevScalars*,
+                                         cudaStream_t);
+template cudaError_t launch_big_q<double>(const BigQSet<double>&, long long, double*, unsigned*, DevScalars*,
+                                          cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // simpleSolvent: wFactor = exp(-w / L), Q = sum(wFactor) / N, phi += (vf / Q) wFactor
@@ -208,31 +266,6 @@ cudaError_t launch_solvent(const double* w, double neg_inv_len, double volfrac, 
   solvent_density_kernel<<<blocks, 256, 0, st>>>(w, neg_inv_len, volfrac, N, is, sc, phi);
   return cudaGetLastError();
 }
-
-// ---------------------------------------------------------------------------
-// chargeFlexPseudoSpec Boltzmann factor (pspolymer/PsChargeFlexPseudoSpec.cpp:97-130):
-// wfac = exp(ds2 w) exp(facZ ds2 psi), facZ = za alpha L.
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void wfac_charged_kernel(const double* __restrict__ w, const double* __restrict__ psi,
-                                    T* __restrict__ wfac, double ds2, double facz, long long N) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
-       i += (long long)gridDim.x * blockDim.x)
-    wfac[i] = (T)(exp(ds2 * w[i]) * exp(facz * ds2 * psi[i]));
-}
-
-template <typename T>
-cudaError_t launch_wfac_charged(const double* w, const double* psi, T* wfac, double ds2, double facz,
-                                long long N, cudaStream_t st) {
-  int blocks = (int)((N + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  wfac_charged_kernel<T><<<blocks, 256, 0, st>>>(w, psi, wfac, ds2, facz, N);
-  return cudaGetLastError();
-}
-template cudaError_t launch_wfac_charged<float>(const double*, const double*, float*, double, double,
-                                                long long, cudaStream_t);
-template cudaError_t launch_wfac_charged<double>(const double*, const double*, double*, double, double,
-                                                 long long, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // simpleIons (pssolvent/PsSimpleIons.cpp:90-160): e = exp(-zc psi),
@@ -430,6 +463,139 @@ template cudaError_t launch_quadrature<double>(const double*, const double*, int
                                                double, const DevScalars*, int, double*,
                                                cudaStream_t);
 
+// The contour sums of every block in one launch.  A thread takes VEC adjacent points
+// of one field, its blocks in order, and writes phi once (the separate launches read
+// and wrote phi per block after a launch that zeroed it).  A panel's last product is
+// the next one's first: two loads of each slice pair instead of three.  Small grids
+// split a block's panels over S threads, whose sums are added in order: one thread
+// per point left most of the chip idle (16^3, three blocks: 30 -> 5 us).
+template <typename T, int VEC> struct QuadVec;
+template <> struct QuadVec<float, 1> { using type = float; };
+template <> struct QuadVec<float, 4> { using type = float4; };
+template <> struct QuadVec<double, 1> { using type = double; };
+template <> struct QuadVec<double, 2> { using type = double2; };
+
+template <typename T, int VEC, int S>
+__global__ void __launch_bounds__(256)
+    quadrature_all_kernel(QuadSet<T> set, long long NV, const DevScalars* __restrict__ sc, double* __restrict__ phi,
+                          int add) {
+  using V = typename QuadVec<T, VEC>::type;
+  constexpr int PT = 256 / S;
+  __shared__ double red[S > 1 ? S : 1][S > 1 ? PT * VEC : 1];
+  pdl_wait();
+  const int field = blockIdx.y;
+  const int t = threadIdx.x % PT, s = threadIdx.x / PT;
+  const long long r = (long long)blockIdx.x * PT + t;
+  const bool in = r < NV;
+  double* const out = phi + ((size_t)field * NV + r) * VEC;
+  double total[VEC];
+#pragma unroll
+  for (int c = 0; c < VEC; ++c) total[c] = (in && add) ? out[c] : 0.0;
+  for (int b = 0; b < set.n; ++b) {
+    if (set.block[b].field != field) continue;
+    const V* __restrict__ qs = reinterpret_cast<const V*>(set.block[b].qs) + r;
+    const V* __restrict__ qts = reinterpret_cast<const V*>(set.block[b].qts) + r;
+    const int num = set.block[b].steps + 1;
+    const bool even = (num % 2) == 0;
+    const int panels = (even ? num - 4 : num - 3) / 2 + 1;
+    const int p0 = (int)((long long)panels * s / S), p1 = (int)((long long)panels * (s + 1) / S);
+    auto product = [&](int n, double (&p)[VEC]) {
+      const V x = qs[n * NV], y = qts[(num - 1 - n) * NV];
+#pragma unroll
+      for (int c = 0; c < VEC; ++c)
+        p[c] = (double)reinterpret_cast<const T*>(&x)[c] * (double)reinterpret_cast<const T*>(&y)[c];
+    };
+    double acc[VEC];
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) acc[c] = 0.0;
+    if (in && p0 < p1) {
+      double a[VEC];
+      product(2 * p0, a);
+#pragma unroll 4
+      for (int p = p0; p < p1; ++p) {
+        double m[VEC], e[VEC];
+        product(2 * p + 1, m);
+        product(2 * p + 2, e);
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) {
+          acc[c] = acc[c] + a[c];
+          acc[c] = acc[c] + m[c] * 4.0;
+          acc[c] = acc[c] + e[c];
+          a[c] = e[c];
+        }
+      }
+    }
+    if constexpr (S > 1) {
+      __syncthreads();
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) red[s][t * VEC + c] = acc[c];
+      __syncthreads();
+      if (s == 0) {
+        for (int k = 1; k < S; ++k)
+#pragma unroll
+          for (int c = 0; c < VEC; ++c) acc[c] = acc[c] + red[k][t * VEC + c];
+      }
+    }
+    if (s == 0 && in) {
+      const double inv_bq = 1.0 / sc->q[set.block[b].ip];
+      double tail[VEC];
+      if (even) {
+        double l[VEC], e[VEC];
+        product(num - 2, l);
+        product(num - 1, e);
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) {
+          double x = 0.0;
+          x = x + l[c];
+          x = x + e[c];
+          tail[c] = x * set.block[b].trap;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) {
+        double x = acc[c] * set.block[b].simp;
+        if (even) x = x + tail[c];
+        const double qqt = inv_bq * x;
+        total[c] = total[c] + set.block[b].densfac * qqt;
+      }
+    }
+  }
+  if (s == 0 && in) {
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) out[c] = total[c];
+  }
+}
+
+template <typename T, int VEC>
+static cudaError_t launch_quadrature_vec(const QuadSet<T>& set, long long NV, int nf, const DevScalars* sc, double* phi,
+                                         bool add, cudaStream_t st) {
+  // as many splits as it takes to give every SM 1024 threads
+  int S = 1;
+  while (S < 16 && NV * nf * S < 148LL * 1024) S *= 2;
+#define PSB_QUAD(SS)                                                                                              \
+  if (S == SS)                                                                                                    \
+    return launch_sweep_kernel(quadrature_all_kernel<T, VEC, SS>, dim3((unsigned)((NV * SS + 255) / 256), nf),    \
+                               dim3(256), 0, st, set, NV, sc, phi, add ? 1 : 0);
+  PSB_QUAD(1) PSB_QUAD(2) PSB_QUAD(4) PSB_QUAD(8) PSB_QUAD(16)
+#undef PSB_QUAD
+  return cudaErrorInvalidValue;
+}
+
+template <typename T>
+cudaError_t launch_quadrature_all(const QuadSet<T>& set, long long N, int nf, const DevScalars* sc, double* phi,
+                                  bool add, cudaStream_t st) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  bool wide = N % VEC == 0 && ((uintptr_t)phi % 16) == 0;
+  for (int b = 0; b < set.n; ++b)
+    wide = wide && ((uintptr_t)set.block[b].qs % 16) == 0 && ((uintptr_t)set.block[b].qts % 16) == 0;
+  if (wide) return launch_quadrature_vec<T, VEC>(set, N / VEC, nf, sc, phi, add, st);
+  return launch_quadrature_vec<T, 1>(set, N, nf, sc, phi, add, st);
+}
+template cudaError_t launch_quadrature_all<float>(const QuadSet<float>&, long long, int, const DevScalars*, double*,
+                                                  bool, cudaStream_t);
+template cudaError_t launch_quadrature_all<double>(const QuadSet<double>&, long long, int, const DevScalars*, double*,
+                                                   bool, cudaStream_t);
+
 // ---------------------------------------------------------------------------
 // Field update pieces shared by the steepest-descent and Anderson updaters.
 // ---------------------------------------------------------------------------
@@ -570,12 +736,40 @@ __device__ __forceinline__ double incomp(const double (&phi_r)[NF]) {
   return fabs(t - 1.0);
 }
 
+// Finalisation by the last CTA of the update: mean pressure, F, diagnostics.
+__device__ __forceinline__ void update_finalize(const FieldModel& fm, const double* partials, int blocks,
+                                                DevScalars* sc, bool anderson) {
+  double r[5];  // sum p, sum fe, sum fe_nodis, sum dH^2, max incompressibility
+  cta_reduce_many<5>(partials, blocks, kUpdQ, 1u << 4, r);
+  if (threadIdx.x == 0) {
+    double sum_tmp = 0.0;
+    for (int ip = 0; ip < fm.npol; ++ip) {
+      const double logq = sc->log_q[ip];
+      sum_tmp = sum_tmp - ((fm.vf[ip] * logq) / fm.alpha[ip]);
+    }
+    for (int is = 0; is < fm.nsolv; ++is) {
+      const double logq = log(sc->solv_q[is]);
+      sum_tmp = sum_tmp - ((fm.solv_vf[is] * logq) / (1.0 / fm.scale_len));
+    }
+    sc->pressure_mean = r[0] / ((double)fm.N * 1.0);
+    sc->free_energy = sum_tmp + r[1];
+    sc->free_energy_nodis = sum_tmp + r[2];
+    sc->dh_norm = sqrt(r[3] / (double)fm.N);
+    sc->max_incomp = r[4];
+    if (!(sc->free_energy == sc->free_energy)) sc->error_flags |= 2;
+    sc->iteration += 1;
+    if (anderson) sc->am_k += 1;
+  }
+}
+
 template <int NF>
 __global__ void __launch_bounds__(kRedThreads)
-    sd_update_kernel(FieldModel fm, FieldPtrs fp, double* __restrict__ partials) {
+    sd_update_kernel(FieldModel fm, FieldPtrs fp, double* __restrict__ partials, unsigned* __restrict__ count,
+                     DevScalars* __restrict__ sc) {
+  pdl_wait();
   double acc[kUpdQ] = {0, 0, 0, 0, 0, 0};
   for (long long r = blockIdx.x * (long long)kRedThreads + threadIdx.x; r < fm.N;
-       r += (long long)kRedBlocks * kRedThreads) {
+       r += (long long)gridDim.x * kRedThreads) {
     double dh[NF], phi_r[NF], dir[NF], wn[NF];
     compute_dh<NF>(fm, fp, r, dh, phi_r);
 #pragma unroll
@@ -590,15 +784,13 @@ __global__ void __launch_bounds__(kRedThreads)
     finish_point<NF>(fm, fp, r, wn, phi_r, acc[0], acc[1], acc[2]);
   }
   block_reduce_write<kUpdQ>(acc, 1u << 4, partials + (size_t)blockIdx.x * kUpdQ);
+  if (last_block(count, gridDim.x)) update_finalize(fm, partials, gridDim.x, sc, false);
 }
 
-cudaError_t launch_sd_update(const FieldModel& fm, const FieldPtrs& fp, double* partials,
-                             cudaStream_t st) {
-  if (fm.nf == 3)
-    sd_update_kernel<3><<<kRedBlocks, kRedThreads, 0, st>>>(fm, fp, partials);
-  else
-    sd_update_kernel<2><<<kRedBlocks, kRedThreads, 0, st>>>(fm, fp, partials);
-  return cudaGetLastError();
+cudaError_t launch_sd_update(const FieldModel& fm, const FieldPtrs& fp, double* partials, unsigned* count,
+                             DevScalars* sc, cudaStream_t st) {
+  return launch_sweep_kernel(fm.nf == 3 ? sd_update_kernel<3> : sd_update_kernel<2>, dim3(red_blocks(fm.N)),
+                             dim3(kRedThreads), 0, st, fm, fp, partials, count, sc);
 }
 
 // ---------------------------------------------------------------------------
@@ -610,13 +802,14 @@ __global__ void __launch_bounds__(kRedThreads)
     am_residual_kernel(FieldModel fm, FieldPtrs fp, double* __restrict__ hist_w,
                        double* __restrict__ hist_d, int slots, const DevScalars* __restrict__ sc,
                        double* __restrict__ partials) {
+  pdl_wait();
   const int cur = (int)(sc->am_k % slots);
   const size_t nfN = (size_t)fm.nf * fm.N;
   double* Wc = hist_w + (size_t)cur * nfN;
   double* Dc = hist_d + (size_t)cur * nfN;
   double acc[2] = {0.0, 0.0};
   for (long long r = blockIdx.x * (long long)kRedThreads + threadIdx.x; r < fm.N;
-       r += (long long)kRedBlocks * kRedThreads) {
+       r += (long long)gridDim.x * kRedThreads) {
     double dh[NF], phi_r[NF], dir[NF];
     compute_dh<NF>(fm, fp, r, dh, phi_r);
 #pragma unroll
@@ -640,11 +833,9 @@ __global__ void __launch_bounds__(kRedThreads)
 cudaError_t launch_am_residual(const FieldModel& fm, const FieldPtrs& fp, double* hist_w,
                                double* hist_d, int slots, DevScalars* sc, double* partials,
                                cudaStream_t st) {
-  if (fm.nf == 3)
-    am_residual_kernel<3><<<kRedBlocks, kRedThreads, 0, st>>>(fm, fp, hist_w, hist_d, slots, sc, partials);
-  else
-    am_residual_kernel<2><<<kRedBlocks, kRedThreads, 0, st>>>(fm, fp, hist_w, hist_d, slots, sc, partials);
-  return cudaGetLastError();
+  return launch_sweep_kernel(fm.nf == 3 ? am_residual_kernel<3> : am_residual_kernel<2>, dim3(red_blocks(fm.N)),
+                             dim3(kRedThreads), 0, st, fm, fp, hist_w, hist_d, slots,
+                             static_cast<const DevScalars*>(sc), partials);
 }
 
 constexpr int kAmMax = 33;  // depth <= 32
@@ -655,6 +846,7 @@ template <int MAXJ>
 __global__ void __launch_bounds__(kRedThreads)
     am_gram_kernel(long long nfN, const double* __restrict__ hist_d, int slots, int m,
                    const DevScalars* __restrict__ sc, double* __restrict__ gram_partials) {
+  pdl_wait();
   const long long k = sc->am_k;
   const int nh = (int)(k < m ? k : m);
   const int cur = (int)(k % slots);
@@ -669,7 +861,7 @@ __global__ void __launch_bounds__(kRedThreads)
 #pragma unroll
   for (int j = 0; j < MAXJ; ++j) acc[j] = 0.0;
   for (long long t = blockIdx.x * (long long)kRedThreads + threadIdx.x; t < nfN;
-       t += (long long)kRedBlocks * kRedThreads) {
+       t += (long long)gridDim.x * kRedThreads) {
     const double d = Dc[t];
 #pragma unroll
     for (int j = 0; j < MAXJ; ++j)
@@ -681,98 +873,118 @@ __global__ void __launch_bounds__(kRedThreads)
 cudaError_t launch_am_gram(long long nfN, const double* hist_d, int slots, int m, DevScalars* sc,
                            double* gram_partials, cudaStream_t st) {
   if (m + 1 > kAmMax) return cudaErrorInvalidValue;
-  if (m + 1 <= 8)
-    am_gram_kernel<8><<<kRedBlocks, kRedThreads, 0, st>>>(nfN, hist_d, slots, m, sc, gram_partials);
-  else if (m + 1 <= 12)
-    am_gram_kernel<12><<<kRedBlocks, kRedThreads, 0, st>>>(nfN, hist_d, slots, m, sc, gram_partials);
-  else if (m + 1 <= 16)
-    am_gram_kernel<16><<<kRedBlocks, kRedThreads, 0, st>>>(nfN, hist_d, slots, m, sc, gram_partials);
-  else
-    am_gram_kernel<kAmMax><<<kRedBlocks, kRedThreads, 0, st>>>(nfN, hist_d, slots, m, sc, gram_partials);
-  return cudaGetLastError();
+  auto kern = (m + 1 <= 8) ? am_gram_kernel<8>
+                           : (m + 1 <= 12) ? am_gram_kernel<12> : (m + 1 <= 16) ? am_gram_kernel<16> : am_gram_kernel<kAmMax>;
+  return launch_sweep_kernel(kern, dim3(red_blocks(nfN)), dim3(kRedThreads), 0, st, nfN, hist_d, slots, m,
+                             static_cast<const DevScalars*>(sc), gram_partials);
 }
 
 // One CTA: finish the Gram row, build U c = V and solve it (partial pivoting,
 // the same elimination order as the oracle's restatement).
-__global__ void am_solve_kernel(const double* __restrict__ gram_partials, double* __restrict__ gram,
+__global__ void am_solve_kernel(const double* __restrict__ gram_partials, int blocks, double* __restrict__ gram,
                                 int slots, int m, int start, double mix, double lambda0,
                                 DevScalars* __restrict__ sc) {
+  pdl_wait();
   __shared__ double A[32 * 32];
   __shared__ double V[32];
   __shared__ double row[kAmMax];
   const long long k = sc->am_k;
   const int nh_all = (int)(k < m ? k : m);
   const int cur = (int)(k % slots);
-  for (int j = 0; j <= nh_all; ++j) {
-    double g = cta_reduce_partials(gram_partials + j, kRedBlocks, kAmMax, false);
-    if (threadIdx.x == 0) row[j] = g;
+  // the row's sums, eight at a time (the partials have kAmMax columns; those beyond
+  // nh_all are not used)
+  for (int j0 = 0; j0 <= nh_all; j0 += 8) {
+    double g[8];
+    if (j0 + 8 <= kAmMax) {
+      cta_reduce_many<8>(gram_partials + j0, blocks, kAmMax, 0u, g);
+      if (threadIdx.x == 0)
+        for (int j = 0; j < 8; ++j) row[j0 + j] = g[j];
+    } else {
+      double l[1];
+      cta_reduce_many<1>(gram_partials + j0, blocks, kAmMax, 0u, l);
+      if (threadIdx.x == 0) row[j0] = l[0];
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int j = 0; j <= nh_all; ++j) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    for (int j = lane; j <= nh_all; j += 32) {
       const int sj = (int)((k - j) % slots);
       gram[cur * slots + sj] = row[j];
       gram[sj * slots + cur] = row[j];
     }
+    __syncwarp();
     const int use = (k >= start) && nh_all > 0;
-    int nh = use ? nh_all : 0;
+    const int nh = use ? nh_all : 0;
     if (use) {
+      // one lane per column: every element's operations and their order are those of
+      // the elimination by one thread
       const double gkk = gram[cur * slots + cur];
       for (int a = 1; a <= nh; ++a) {
         const int sa = (int)((k - a) % slots);
-        V[a - 1] = gkk - gram[cur * slots + sa];
-        for (int b = 1; b <= nh; ++b) {
+        for (int b = 1 + lane; b <= nh; b += 32) {
           const int sb = (int)((k - b) % slots);
           A[(a - 1) * nh + (b - 1)] =
               gkk - gram[cur * slots + sa] - gram[cur * slots + sb] + gram[sa * slots + sb];
         }
+        if (lane == 0) V[a - 1] = gkk - gram[cur * slots + sa];
       }
+      __syncwarp();
       int singular = 0;
       for (int kk = 0; kk < nh && !singular; ++kk) {
         int piv = kk;
         double best = fabs(A[kk * nh + kk]);
         for (int i = kk + 1; i < nh; ++i)
           if (fabs(A[i * nh + kk]) > best) { best = fabs(A[i * nh + kk]); piv = i; }
-        if (!(best > 0.0)) { singular = 1; break; }
+        if (!(best > 0.0)) { singular = 1; break; }  // the same in every lane
+        __syncwarp();
         if (piv != kk) {
-          for (int j = 0; j < nh; ++j) {
+          for (int j = lane; j < nh; j += 32) {
             double t = A[kk * nh + j]; A[kk * nh + j] = A[piv * nh + j]; A[piv * nh + j] = t;
           }
-          double t = V[kk]; V[kk] = V[piv]; V[piv] = t;
+          if (lane == 0) { double t = V[kk]; V[kk] = V[piv]; V[piv] = t; }
+          __syncwarp();
         }
-        for (int i = kk + 1; i < nh; ++i) {
+        // one lane per row
+        for (int i = kk + 1 + lane; i < nh; i += 32) {
           double f = A[i * nh + kk] / A[kk * nh + kk];
           for (int j = kk; j < nh; ++j) A[i * nh + j] = A[i * nh + j] - f * A[kk * nh + j];
           V[i] = V[i] - f * V[kk];
         }
+        __syncwarp();
       }
-      if (!singular) {
-        for (int i = nh - 1; i >= 0; --i) {
-          double t = V[i];
-          for (int j = i + 1; j < nh; ++j) t = t - A[i * nh + j] * V[j];
-          V[i] = t / A[i * nh + i];
+      if (lane == 0) {
+        if (!singular) {
+          for (int i = nh - 1; i >= 0; --i) {
+            double t = V[i];
+            for (int j = i + 1; j < nh; ++j) t = t - A[i * nh + j] * V[j];
+            V[i] = t / A[i * nh + i];
+          }
         }
+        for (int a = 0; a < nh; ++a) sc->am_c[a] = singular ? 0.0 : V[a];
       }
-      for (int a = 0; a < nh; ++a) sc->am_c[a] = singular ? 0.0 : V[a];
     }
-    sc->am_nh = nh;
-    sc->am_use = use;
-    sc->am_mix = use ? mix : lambda0;
+    if (lane == 0) {
+      sc->am_nh = nh;
+      sc->am_use = use;
+      sc->am_mix = use ? mix : lambda0;
+    }
   }
 }
 
-cudaError_t launch_am_solve(const double* gram_partials, double* gram, int slots, int m, int start,
+cudaError_t launch_am_solve(long long nfN, const double* gram_partials, double* gram, int slots, int m, int start,
                             double mix, double lambda0, DevScalars* sc, cudaStream_t st) {
   if (m > 32) return cudaErrorInvalidValue;
-  am_solve_kernel<<<1, kRedThreads, 0, st>>>(gram_partials, gram, slots, m, start, mix, lambda0, sc);
-  return cudaGetLastError();
+  return launch_sweep_kernel(am_solve_kernel, dim3(1), dim3(kRedThreads), 0, st, gram_partials, red_blocks(nfN), gram,
+                             slots, m, start, mix, lambda0, sc);
 }
 
 template <int NF>
 __global__ void __launch_bounds__(kRedThreads)
     am_mix_kernel(FieldModel fm, FieldPtrs fp, const double* __restrict__ hist_w,
-                  const double* __restrict__ hist_d, int slots, const DevScalars* __restrict__ sc,
-                  double* __restrict__ partials) {
+                  const double* __restrict__ hist_d, int slots, DevScalars* __restrict__ sc,
+                  double* __restrict__ partials, unsigned* __restrict__ count) {
+  pdl_wait();
   const long long k = sc->am_k;
   const int cur = (int)(k % slots);
   const int nh = sc->am_nh;
@@ -780,7 +992,7 @@ __global__ void __launch_bounds__(kRedThreads)
   const size_t nfN = (size_t)fm.nf * fm.N;
   double acc[3] = {0.0, 0.0, 0.0};
   for (long long r = blockIdx.x * (long long)kRedThreads + threadIdx.x; r < fm.N;
-       r += (long long)kRedBlocks * kRedThreads) {
+       r += (long long)gridDim.x * kRedThreads) {
     double wn[NF], phi_r[NF];
 #pragma unroll
     for (int i = 0; i < NF; ++i) phi_r[i] = fp.phi[i][r];
@@ -822,63 +1034,19 @@ __global__ void __launch_bounds__(kRedThreads)
   if (threadIdx.x == 0) {
     for (int q = 0; q < 3; ++q) partials[(size_t)blockIdx.x * kUpdQ + q] = out[q];
   }
+  if (last_block(count, gridDim.x)) update_finalize(fm, partials, gridDim.x, sc, true);
 }
 
 cudaError_t launch_am_mix(const FieldModel& fm, const FieldPtrs& fp, const double* hist_w,
-                          const double* hist_d, int slots, DevScalars* sc, double* partials,
+                          const double* hist_d, int slots, DevScalars* sc, double* partials, unsigned* count,
                           cudaStream_t st) {
-  if (fm.nf == 3)
-    am_mix_kernel<3><<<kRedBlocks, kRedThreads, 0, st>>>(fm, fp, hist_w, hist_d, slots, sc, partials);
-  else
-    am_mix_kernel<2><<<kRedBlocks, kRedThreads, 0, st>>>(fm, fp, hist_w, hist_d, slots, sc, partials);
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Finalisation: mean pressure, F, diagnostics.
-// ---------------------------------------------------------------------------
-__global__ void update_finalize_kernel(FieldModel fm, const double* __restrict__ partials,
-                                       DevScalars* __restrict__ sc, int anderson) {
-  const double psum = cta_reduce_partials(partials + 0, kRedBlocks, kUpdQ, false);
-  const double fe = cta_reduce_partials(partials + 1, kRedBlocks, kUpdQ, false);
-  const double fend = cta_reduce_partials(partials + 2, kRedBlocks, kUpdQ, false);
-  const double dh2 = cta_reduce_partials(partials + 3, kRedBlocks, kUpdQ, false);
-  const double mx = cta_reduce_partials(partials + 4, kRedBlocks, kUpdQ, true);
-  if (threadIdx.x == 0) {
-    double sum_tmp = 0.0;
-    for (int ip = 0; ip < fm.npol; ++ip) {
-      const double logq = sc->log_q[ip];
-      sum_tmp = sum_tmp - ((fm.vf[ip] * logq) / fm.alpha[ip]);
-    }
-    for (int is = 0; is < fm.nsolv; ++is) {
-      const double logq = log(sc->solv_q[is]);
-      sum_tmp = sum_tmp - ((fm.solv_vf[is] * logq) / (1.0 / fm.scale_len));
-    }
-    sc->pressure_mean = psum / ((double)fm.N * 1.0);
-    sc->free_energy = sum_tmp + fe;
-    sc->free_energy_nodis = sum_tmp + fend;
-    sc->dh_norm = sqrt(dh2 / (double)fm.N);
-    sc->max_incomp = mx;
-    if (!(sc->free_energy == sc->free_energy)) sc->error_flags |= 2;
-    sc->iteration += 1;
-    if (anderson) sc->am_k += 1;
-  }
-}
-
-cudaError_t launch_update_finalize(const FieldModel& fm, const double* partials, DevScalars* sc,
-                                   cudaStream_t st) {
-  update_finalize_kernel<<<1, kRedThreads, 0, st>>>(fm, partials, sc, 0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_update_finalize_am(const FieldModel& fm, const double* partials, DevScalars* sc,
-                                      cudaStream_t st) {
-  update_finalize_kernel<<<1, kRedThreads, 0, st>>>(fm, partials, sc, 1);
-  return cudaGetLastError();
+  return launch_sweep_kernel(fm.nf == 3 ? am_mix_kernel<3> : am_mix_kernel<2>, dim3(red_blocks(fm.N)),
+                             dim3(kRedThreads), 0, st, fm, fp, hist_w, hist_d, slots, sc, partials, count);
 }
 
 __global__ void pressure_shift_kernel(double* __restrict__ p, long long N,
                                       const DevScalars* __restrict__ sc) {
+  pdl_wait();
   const double mean = sc->pressure_mean;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
        i += (long long)gridDim.x * blockDim.x)
@@ -888,8 +1056,7 @@ __global__ void pressure_shift_kernel(double* __restrict__ p, long long N,
 cudaError_t launch_pressure_shift(double* p, long long N, const DevScalars* sc, cudaStream_t st) {
   int blocks = (int)((N + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
-  pressure_shift_kernel<<<blocks, 256, 0, st>>>(p, N, sc);
-  return cudaGetLastError();
+  return launch_sweep_kernel(pressure_shift_kernel, dim3(blocks), dim3(256), 0, st, p, N, sc);
 }
 
 }  // namespace psb

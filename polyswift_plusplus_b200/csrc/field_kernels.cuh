@@ -57,17 +57,48 @@ struct FieldPtrs {
   const double* noise;  // nf*N Gaussian increments (already scaled) or nullptr
 };
 
-// wfac = exp(ds2 * w) rounded to T.
+// Boltzmann factors exp(ds2 w) [exp(facz ds2 psi) of charged blocks], rounded to T, of
+// up to kWfacMax tables in one launch.
+constexpr int kWfacMax = 16;
+template <typename T> struct WfacSet {
+  int n = 0;
+  struct Key {
+    const double* w;
+    const double* psi;  // nullptr: not charged
+    T* out;
+    double ds2, facz;
+  } key[kWfacMax];
+};
 template <typename T>
-cudaError_t launch_wfac(const double* w, T* wfac, double ds2, long long N, cudaStream_t st);
+cudaError_t launch_wfac(const WfacSet<T>& set, long long N, cudaStream_t st);
 
-// partials[b] = sum over the block's points of a*b (FP64).
+// Q of every polymer ip: sum over the points of a[ip] b[ip], over N, into sc->q and
+// log_q; sets the error flag on NaN.  partials: n x kRedBlocks; count: n zeros.
+template <typename T> struct BigQSet {
+  int n = 0;
+  const T* a[PS_MAX_POLYMERS];
+  const T* b[PS_MAX_POLYMERS];
+};
 template <typename T>
-cudaError_t launch_dot_partials(const T* a, const T* b, long long N, double* partials,
-                                cudaStream_t st);
-// Q = sum(partials) / N for polymer ip; sets error flag on NaN.
-cudaError_t launch_finalize_q(const double* partials, double N, int ip, DevScalars* sc,
-                              cudaStream_t st);
+cudaError_t launch_big_q(const BigQSet<T>& set, long long N, double* partials, unsigned* count, DevScalars* sc,
+                         cudaStream_t st);
+
+// phi_f (+)= sum over the blocks of field f, in order, of densfac Simpson(qs, qts) / Q
+// (pspolymer/PsBlock.cpp:255-380 + :153-196), up to kQuadMax blocks in one launch; add:
+// onto what phi holds, otherwise phi is overwritten.
+constexpr int kQuadMax = 32;
+template <typename T> struct QuadSet {
+  int n = 0;
+  struct Block {
+    const T* qs;
+    const T* qts;
+    double simp, trap, densfac;
+    int steps, ip, field, pad;
+  } block[kQuadMax];
+};
+template <typename T>
+cudaError_t launch_quadrature_all(const QuadSet<T>& set, long long N, int nf, const DevScalars* sc, double* phi,
+                                  bool add, cudaStream_t st);
 
 // phi += densfac * Simpson(qs, qts) / Q  (pspolymer/PsBlock.cpp:255-380 + :153-196).
 template <typename T>
@@ -91,11 +122,6 @@ cudaError_t launch_junction(const JunctionIn<T>& in, long long N, T* out, cudaSt
 cudaError_t launch_solvent(const double* w, double neg_inv_len, double volfrac, long long N, int is,
                            double* partials, DevScalars* sc, double* phi, cudaStream_t st);
 
-// chargeFlexPseudoSpec: wfac = exp(ds2 w) exp(facz ds2 psi) rounded to T.
-template <typename T>
-cudaError_t launch_wfac_charged(const double* w, const double* psi, T* wfac, double ds2, double facz,
-                                long long N, cudaStream_t st);
-
 // simpleIons (pssolvent/PsSimpleIons.cpp:90-160): Q = <exp(-zc psi)> into
 // sc->solv_q[is]; e = exp(-zc psi) (-neutral_factor / (Q zc)); block_rho = e
 // (when not null); rho += zc e.
@@ -107,26 +133,23 @@ cudaError_t launch_ions(const double* psi, double zc, double neutral_factor, lon
 cudaError_t launch_charge_accum(const double* phi, double alpha, double za, long long N, double* rho,
                                 cudaStream_t st);
 
-// Steepest-descent update, pressure rebuild and free-energy partial sums.
-cudaError_t launch_sd_update(const FieldModel& fm, const FieldPtrs& fp, double* partials,
-                             cudaStream_t st);
-// Anderson: residual + history store, Gram row, solve, mix (+ pressure / F partials).
+// Steepest-descent update, pressure rebuild and free-energy sums; the last CTA
+// (count: one zero) reduces them into DevScalars (F, mean p, diagnostics; iteration++).
+cudaError_t launch_sd_update(const FieldModel& fm, const FieldPtrs& fp, double* partials, unsigned* count,
+                             DevScalars* sc, cudaStream_t st);
+// Anderson: residual + history store, Gram row, solve, mix (+ pressure / F sums and the
+// same reduction).
 cudaError_t launch_am_residual(const FieldModel& fm, const FieldPtrs& fp, double* hist_w,
                                double* hist_d, int slots, DevScalars* sc, double* partials,
                                cudaStream_t st);
 cudaError_t launch_am_gram(long long nfN, const double* hist_d, int slots, int m, DevScalars* sc,
                            double* gram_partials, cudaStream_t st);
-cudaError_t launch_am_solve(const double* gram_partials, double* gram, int slots, int m,
+cudaError_t launch_am_solve(long long nfN, const double* gram_partials, double* gram, int slots, int m,
                             int start, double mix, double lambda0, DevScalars* sc,
                             cudaStream_t st);
 cudaError_t launch_am_mix(const FieldModel& fm, const FieldPtrs& fp, const double* hist_w,
-                          const double* hist_d, int slots, DevScalars* sc, double* partials,
+                          const double* hist_d, int slots, DevScalars* sc, double* partials, unsigned* count,
                           cudaStream_t st);
-// Reduce the update partials into DevScalars (F, mean p, diagnostics); iteration++.
-cudaError_t launch_update_finalize(const FieldModel& fm, const double* partials, DevScalars* sc,
-                                   cudaStream_t st);
-cudaError_t launch_update_finalize_am(const FieldModel& fm, const double* partials,
-                                      DevScalars* sc, cudaStream_t st);
 // p -= mean(p)
 cudaError_t launch_pressure_shift(double* p, long long N, const DevScalars* sc, cudaStream_t st);
 
