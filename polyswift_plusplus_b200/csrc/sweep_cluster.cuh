@@ -84,7 +84,7 @@ template <typename T, int NX, int NY, int NZ, int CL_> struct SweepCl {
   // four threads a column leave no lane idle at ny = 16 and 32 (32^3 FP64: 4.60 us a
   // step, 4.84 with eight)
   static constexpr int GY = (NY == 16 || NY == 32) ? 4 : GroupOf<NY>::v, RY = FILM ? 1 : NY / GY, UY = (RY + GY - 1) / GY;
-  static constexpr int GZ = RowGroup<PR, NZ>::v, RZ = NZ / GZ, UZ = (RZ + GZ - 1) / GZ;
+  static constexpr int GZ = (NZ < 16) ? 4 : RowGroup<PR, NZ>::v, RZ = NZ / GZ, UZ = (RZ + GZ - 1) / GZ;
   static constexpr int GX = (NX >= 64) ? 16 : 4, RX = NX / GX, UX = (RX + GX - 1) / GX;
   static constexpr bool V2 = sizeof(T) == 4 && RZ % 2 == 0;
   static constexpr int PA = V2 ? ((RZ / 2) % 2 ? RZ : RZ + 2) : RZ + 1;
@@ -92,16 +92,20 @@ template <typename T, int NX, int NY, int NZ, int CL_> struct SweepCl {
   static constexpr int S = (sizeof(T) == 4) ? S0 + ((24 - S0 % 16) % 16) : S0;
   static constexpr int NCOL = NY * (H + 1);
   static constexpr int COLS = (NCOL + CL - 1) / CL;     // columns of a CTA (the last may have fewer)
-  static constexpr int PTH = FILM ? PR * GZ : H * GY;   // threads of a plane
+  // threads of a plane's z rows and of a plane: whole warps.  At nz < 16 the last
+  // warp has lanes without a row (they take PRB - PR spare rows of the buffer along)
+  // or without a column.
+  static constexpr int ROWT = (PR * GZ + 31) / 32 * 32, PRB = ROWT / GZ;
+  static constexpr int COLT = FILM ? 0 : (H * GY + 31) / 32 * 32;
+  static constexpr int PTH = COLT > ROWT ? COLT : ROWT;
   static constexpr int TH0 = NP * PTH, THX = COLS * GX;
   static constexpr int TH1 = TH0 > THX ? TH0 : THX;
   static constexpr int TH = (TH1 + 31) / 32 * 32;
-  static constexpr int ROWT = PR * GZ;                  // z-row threads of a plane
-  static constexpr int BUF = NP * PR * S, AIN = PX * NCOL, BIN = NX * COLS;
+  static constexpr int BUF = NP * PRB * S, AIN = PX * NCOL, BIN = NX * COLS;
   static constexpr size_t SMEM =
       sizeof(c2_t<T>) * ((size_t)BUF + AIN + 2 * BIN + NP * NY + NX + NX / 2 + NY + NZ) +
       sizeof(double) * (CL * (TH / 32) + 1) + 2 * sizeof(uint64_t);
-  static_assert(PX * CL == NX && TH <= 1024 && ROWT <= PTH && ROWT % 32 == 0 && PTH % 32 == 0, "cluster sweep layout");
+  static_assert(PX * CL == NX && TH <= 1024 && PRB * GZ == ROWT && (!FILM || PRB == PR), "cluster sweep layout");
   static_assert(S >= NZ && RZ * GZ == NZ && RX * GX == NX && (FILM || RY * GY == NY) && UZ <= 2, "cluster sweep layout");
   static_assert(NP <= 15 && (!FILM || PX % 2 == 0) && CL * 2 <= TH, "cluster sweep layout");
 };
@@ -150,12 +154,13 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
   const int pl = tid / PTH, tp = tid - pl * PTH;
   const bool in_plane = pl < NP;
   const int c = FILM ? 0 : tp % H, j = FILM ? 0 : tp / H;
+  const bool in_y = (PTH == H * GY) || j < GY;
   const int mc = (c == 0) ? H : NZ - c;
-  C* const pbuf = buf + (in_plane ? pl : 0) * (PR * S);
+  C* const pbuf = buf + (in_plane ? pl : 0) * (P::PRB * S);
   // z part: row b of the plane's packed rows
   const bool in_row = in_plane && tp < P::ROWT;
   const int b = tp / GZ, jz = tp % GZ, j0 = jz * UZ;
-  const bool on = in_row && ((RZ % GZ == 0) || j0 < RZ);
+  const bool on = in_row && (P::PRB == PR || b < PR) && ((RZ % GZ == 0) || j0 < RZ);
   C* const row = pbuf + b * S;
   // the pair's real rows in memory: y and y + ny/2 of plane x0 + pl (film: x and x + PX/2)
   const size_t ra = (FILM ? (size_t)(x0 + b) * NZ : ((size_t)(x0 + pl) * NY + b) * NZ) + j0;
@@ -224,26 +229,28 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
     if (k > 0) wait(bar_a, (uint32_t)(k - 1), bytes_a, k < total);
     if (!FILM && k > 0) {
       if (in_plane) {
-        const C* const src = a_in + pl * NCOL + c;
-        C v[RY];
+        if (in_y) {
+          const C* const src = a_in + pl * NCOL + c;
+          C v[RY];
 #pragma unroll
-        for (int r = 0; r < RY; ++r) v[r] = src[(j + GY * r) * H];
-        if (c == 0) {
+          for (int r = 0; r < RY; ++r) v[r] = src[(j + GY * r) * H];
+          if (c == 0) {
 #pragma unroll
-          for (int r = 0; r < RY; ++r) {
-            const C n = src[NY * H + (j + GY * r)];
-            v[r] = C{v[r].x - n.y, v[r].y + n.x};
+            for (int r = 0; r < RY; ++r) {
+              const C n = src[NY * H + (j + GY * r)];
+              v[r] = C{v[r].x - n.y, v[r].y + n.x};
+            }
           }
-        }
-        Dft<RY, true, C>::run(v);
-        C* const slot_j = pbuf + (j % GH) * RY * S + (j < GH ? c : mc);
+          Dft<RY, true, C>::run(v);
+          C* const slot_j = pbuf + (j % GH) * RY * S + (j < GH ? c : mc);
 #pragma unroll
-        for (int r = 0; r < RY; ++r) slot_j[r * S] = v[r];
+          for (int r = 0; r < RY; ++r) slot_j[r * S] = v[r];
+        }
         plane_sync<TH == PTH, PTH>(pl);
 #pragma unroll
         for (int u = 0; u < UY; ++u) {
           const int jp = j + u * GY;
-          if (RY % GY == 0 || jp < RY) {
+          if (in_y && (RY % GY == 0 || jp < RY)) {
             C q[GY];
             C* const r0 = pbuf + jp * S;
 #pragma unroll
@@ -414,7 +421,7 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
 #pragma unroll
         for (int u = 0; u < UY; ++u) {
           const int jp = j + u * GY;
-          if (RY % GY == 0 || jp < RY) {
+          if (in_y && (RY % GY == 0 || jp < RY)) {
             C q[GY];
             C* const r0 = pbuf + jp * S;
 #pragma unroll
@@ -432,36 +439,40 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
           }
         }
         plane_sync<TH == PTH, PTH>(pl);
-        const C* const slot_j = pbuf + (j % GH) * RY * S + (j < GH ? c : mc);
         C v[RY];
-#pragma unroll
-        for (int r = 0; r < RY; ++r) v[r] = slot_j[r * S];
-#pragma unroll
-        for (int r = 1; r < RY; ++r) v[r] = cmul(v[r], s_tw_y[r * j]);
-        Dft<RY, false, C>::run(v);
-        const int x = x0 + pl;
-        // column 0: separate the Nyquist column (c = 0 threads of all j meet)
         C* const ny = s_nyq + pl * NY;
-        if (c == 0) {
+        if (in_y) {
+          const C* const slot_j = pbuf + (j % GH) * RY * S + (j < GH ? c : mc);
 #pragma unroll
-          for (int r = 0; r < RY; ++r) ny[j + GY * r] = v[r];
-        }
-        plane_sync<TH == PTH, PTH>(pl);
-        if (c == 0) {
+          for (int r = 0; r < RY; ++r) v[r] = slot_j[r * S];
 #pragma unroll
-          for (int r = 0; r < RY; ++r) {
-            const int ky = j + GY * r;
-            const C d = ny[(NY - ky) % NY], a = v[r];
-            v[r] = C{a.x + d.x, a.y - d.y};
-            const int col = NY * H + ky;
-            cl_store(cl_addr(b_in + x * COLS + col % COLS, col / COLS), cl_addr(bar_b, col / COLS),
-                     C{a.y + d.y, d.x - a.x});
+          for (int r = 1; r < RY; ++r) v[r] = cmul(v[r], s_tw_y[r * j]);
+          Dft<RY, false, C>::run(v);
+          // column 0: separate the Nyquist column (c = 0 threads of all j meet)
+          if (c == 0) {
+#pragma unroll
+            for (int r = 0; r < RY; ++r) ny[j + GY * r] = v[r];
           }
         }
+        plane_sync<TH == PTH, PTH>(pl);
+        if (in_y) {
+          const int x = x0 + pl;
+          if (c == 0) {
 #pragma unroll
-        for (int r = 0; r < RY; ++r) {
-          const int col = (j + GY * r) * H + c;
-          cl_store(cl_addr(b_in + x * COLS + col % COLS, col / COLS), cl_addr(bar_b, col / COLS), v[r]);
+            for (int r = 0; r < RY; ++r) {
+              const int ky = j + GY * r;
+              const C d = ny[(NY - ky) % NY], a = v[r];
+              v[r] = C{a.x + d.x, a.y - d.y};
+              const int col = NY * H + ky;
+              cl_store(cl_addr(b_in + x * COLS + col % COLS, col / COLS), cl_addr(bar_b, col / COLS),
+                       C{a.y + d.y, d.x - a.x});
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < RY; ++r) {
+            const int col = (j + GY * r) * H + c;
+            cl_store(cl_addr(b_in + x * COLS + col % COLS, col / COLS), cl_addr(bar_b, col / COLS), v[r]);
+          }
         }
       }
     } else {

@@ -94,7 +94,8 @@ def test_split_step_256(gpu, nx, precision):
     _compare((nx, 256, 256), precision, [3, 11], 0)
 
 
-ONE_LAUNCH = [(16, 16, 16), (24, 24, 24), (32, 32, 32), (16, 16, 1), (32, 32, 1), (64, 64, 1), (128, 128, 1)]
+ONE_LAUNCH = [(16, 16, 16), (24, 24, 24), (32, 32, 32), (16, 16, 1), (32, 32, 1), (64, 64, 1), (128, 128, 1),
+              (8, 8, 8), (12, 12, 12), (24, 24, 1), (48, 48, 1), (96, 96, 1)]
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
