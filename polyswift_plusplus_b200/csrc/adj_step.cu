@@ -4,10 +4,11 @@
 // What was slow: an adjoint step was seven launches (two forward planes, two x
 // passes, the stress sums, the k^2 multiply, the inverse passes and the pointwise
 // update), each reading and writing whole spectra or fields: 33 us a step at 64^3, and
-// 18.6 ms for a forward and backward pass of 128 steps.  Fused: 13 us a step, 9.5 ms a
-// pass (half of it the sweeps and their recomputation from checkpoints); a step is
-// bound by the latency of its two launches, 128 and 132 CTAs.  Replaying the passes as
-// graphs changed nothing: the launches are not the limit.
+// 18.6 ms for a forward and backward pass of 128 steps.  Fused: 13 us a step, 9.9 ms a
+// pass (half of it the sweeps and their recomputation from checkpoints), 7.8 with the
+// adjoints of both sweeps in the same launches; a step is bound by the latency of its
+// two launches.  Replaying the passes as graphs changed nothing: the launches are not
+// the limit.  Nor is one CTA of 240 registers per SM: with 128 (two) 7.6 to 7.9 ms.
 // Now it is two: the x pass keeps U and V in registers between their forward
 // transforms, the stress sums and U's way back, and the plane pass turns mu into the
 // next lambda and starts its transform (and that of wf q) in the same pass.
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__(AdjX<L>::TH)
   double2* s_tw = bv + L * TK;
   double* s_k2 = reinterpret_cast<double*>(s_tw + L);  // k_x^2
   double* s_sum = s_k2 + L;
-  const AdjXWork w = *work;
+  const AdjXWork w = work[blockIdx.y];
   const int tid = threadIdx.x;
   const int cc = tid % TK, j = tid / TK;
   const int hz = nz / 2, inner = ny * (hz + 1);
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(AdjX<L>::TH)
 }
 
 template <int L>
-static cudaError_t launch_adj_x_t(const AdjXWork* w, int ny, int nz, double dx, double dy, double dz, int stride,
+static cudaError_t launch_adj_x_t(const AdjXWork* w, int nw, int ny, int nz, double dx, double dy, double dz, int stride,
                                   const double2* tw, cudaStream_t st) {
   using P = AdjX<L>;
   auto kern = adj_x_kernel<L>;
@@ -167,7 +168,7 @@ static cudaError_t launch_adj_x_t(const AdjXWork* w, int ny, int nz, double dx, 
   cudaError_t e = ensure_smem_attr(kern, P::SMEM, &attr_mask);
   if (e != cudaSuccess) return e;
   const int inner = ny * (nz / 2 + 1);
-  return launch_sweep_kernel(kern, dim3((inner + P::TK - 1) / P::TK), dim3(P::TH), P::SMEM, st, w, ny, nz, dx, dy, dz,
+  return launch_sweep_kernel(kern, dim3((inner + P::TK - 1) / P::TK, nw), dim3(P::TH), P::SMEM, st, w, ny, nz, dx, dy, dz,
                              stride, tw);
 }
 
@@ -181,10 +182,10 @@ int adj_x_tiles(int nx, int inner) {
   return 0;
 }
 
-cudaError_t launch_adj_x(const AdjXWork* w, int nx, int ny, int nz, double dx, double dy, double dz, int stride,
+cudaError_t launch_adj_x(const AdjXWork* w, int nw, int nx, int ny, int nz, double dx, double dy, double dz, int stride,
                          const double2* tw, cudaStream_t st) {
 #define PSB_X(L) \
-  if (nx == L) return launch_adj_x_t<L>(w, ny, nz, dx, dy, dz, stride, tw, st);
+  if (nx == L) return launch_adj_x_t<L>(w, nw, ny, nz, dx, dy, dz, stride, tw, st);
   PSB_ADJ_X(PSB_X)
 #undef PSB_X
   return cudaErrorInvalidValue;

@@ -23,8 +23,18 @@
 // sweep 0 covers n in [jC, min((j+1)C, M)]; the matching part of sweep 1
 // (m = M - n) starts at a checkpoint placed at m = M - min((j+1)C, M), so both
 // halves of a segment are recomputed from one checkpoint each into two
-// (C+1)-slice buffers, and the recomputed slices equal the stored ones bit for
-// bit.  The quadrature and each adjoint sweep recompute the segments once.
+// C-slice buffers (the checkpoint is the first slice), and the recomputed slices
+// equal the stored ones bit for bit.
+//
+// Up to nx = 96 the two adjoint sweeps advance together, sweep 0's through segments
+// J - 1, J - 2, ... and sweep 1's through 0, 1, ...: both segments are recomputed by
+// the same launches into two sets of buffers, and so are the quadrature's, two at a
+// time.  A launch has a sweep's nx planes to work on, so at 64^3 one sweep leaves
+// half the chip idle: forward and backward of 128 steps, one sweep's adjoint at a
+// time and both, ms: 16^3 4.9 and 3.2, 32^3 6.9 and 4.3, 64^3 9.9 and 7.8, 96^3 26.1
+// and 23.5.  At 128^3 (49.8 and 49.3) the second set of buffers is not worth its
+// memory.  On grids with a one-launch sweep (sweep_cluster.cuh) the forward and every
+// recomputation is one launch: 16^3 3.2 -> 2.3, 32^3 4.3 -> 3.8.
 //
 // Branched (tree) chains keep every slice of every sweep (no checkpoints): the
 // forward is the engine's own sweeps with junction products, and the adjoint
@@ -93,12 +103,24 @@ __device__ __forceinline__ double adj_block_sum(double v, double* sh) {
 #define ADJ_LOOP(r, N) \
   for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < (N); r += (long long)gridDim.x * blockDim.x)
 
+// dst += coef x y over the entries.  A block's entries follow one another, so that its
+// sum stays in a register (read and written back for every entry it was 29 us for the
+// 13 slice pairs of a 64^3 segment).
 __global__ void adj_accum_kernel(const AccumEntry* __restrict__ e, int ne, long long N) {
   ADJ_LOOP(r, N) {
+    double* dst = e[0].dst;
+    double acc = dst[r];
+#pragma unroll 4
     for (int i = 0; i < ne; ++i) {
       const AccumEntry a = e[i];
-      a.dst[r] += a.coef * a.x[r] * a.y[r];
+      if (a.dst != dst) {  // the next block
+        dst[r] = acc;
+        dst = a.dst;
+        acc = dst[r];
+      }
+      acc += a.coef * __ldg(a.x + r) * __ldg(a.y + r);
     }
+    dst[r] = acc;
   }
 }
 
@@ -310,11 +332,12 @@ struct ps_adj {
   std::vector<std::vector<std::pair<int, double>>> quad;  // per n: (block, densfac ds c)
   double* ck[2] = {nullptr, nullptr};
   double* endq[2] = {nullptr, nullptr};
-  double* seg[2] = {nullptr, nullptr};
-  double* lam[2] = {nullptr, nullptr};
+  double* seg[2][2] = {};       // [set][sweep]: slices 1 .. C of a recomputed segment
+  double* lam[4] = {};          // two of each adjoint lane
   double* mu = nullptr;
-  double2* spec[2] = {nullptr, nullptr};   // U and V of the adjoint steps
-  double2* rspec[2] = {nullptr, nullptr};  // the recomputed sweeps' (U stays across segments)
+  double2* spec[4] = {};   // U and V of the adjoint steps of each lane
+  double2* rspec[4] = {};  // the recomputed sweeps' (U stays across segments)
+  bool pair = false;       // the adjoints of both sweeps run in the same launches (two lanes)
   double* P = nullptr;
   double* gwb = nullptr;
   double* gphi = nullptr;
@@ -327,6 +350,11 @@ struct ps_adj {
   int stride = 0;
   size_t rows = 0;
   std::vector<int> slot_block;
+  psb::SweepWork<double>* d_sw = nullptr;  // one-launch sweeps
+  double** d_dst = nullptr;                // their slices' places
+  std::vector<psb::SweepWork<double>> h_sw;
+  std::vector<double*> h_dst;
+  std::vector<size_t> sw_dst;              // by work: its part of h_dst
   psb::AdjXWork* d_ax = nullptr;
   std::vector<psb::AdjXWork> h_ax;
   psb::PlaneWork<double>* d_pw = nullptr;
@@ -375,10 +403,12 @@ struct Builder {
   bool fused;
   bool step;  // the sweeps run the step plane pass and the register x pass (compact layout)
   bool adj;   // ... and the adjoint steps their fused forms
+  bool one;   // a sweep is one launch (sweep_cluster.cuh)
   Builder(ps_adj* a_, ps_handle* h_) : a(a_), h(h_), nx(h_->n[0]), ny(h_->n[1]), nz(h_->n[2]), nzh(h_->nzh) {
     fused = plane_fused_supported(8, ny, nz);
     step = step_plane_supported(ny, nz);
     adj = adj_step_supported(ny, nz);
+    one = sweep_cluster_supported(nx, ny, nz);
   }
 
   const double* wf(int b) const {
@@ -470,18 +500,33 @@ struct Builder {
       return launch_step_plane<double>(A->d_pw + p0, n, nx_, ny_, nz_, H->bd.tw_y, H->bd.tw_z, st);
     });
   }
-  // Fused adjoint steps.  lam: the lambda work in an adjoint mode with its point;
-  // q: the start of FFT(wf q) for the next step beside it (block -1: none).
-  void lambda_pass(std::vector<Op>& ops, int mode, const AdjPoint& p, const double* win, const double* wout,
-                   const double* q, const double* wq) {
-    const size_t p0 = plane(pw(mode, nullptr, a->spec[0], win, wout, nullptr));
-    int n = 1;
-    if (q) {
-      plane(pw(MODE_FIRST, q, a->spec[1], nullptr, wq, nullptr));
-      n = 2;
+  // Fused adjoint steps: the plane pass of lambda works in adjoint modes (with their
+  // points) and, beside them, starts of FFT(wf q) for the next steps; the x pass of
+  // steps of the given blocks (stress sums of the slot, U <- IFFT(K U)).
+  struct LamWork {
+    int mode, lane;
+    AdjPoint p;
+    const double *win, *wout;
+  };
+  struct QWork {
+    int lane;
+    const double *q, *wq;
+  };
+  struct XWork {
+    int lane, block, slot;
+  };
+  void lambda_pass(std::vector<Op>& ops, const std::vector<LamWork>& lam, const std::vector<QWork>& qs) {
+    const size_t p0 = a->h_pw.size(), pi = a->h_pt.size();
+    const int n = (int)(lam.size() + qs.size());
+    for (const LamWork& l : lam) {
+      plane(pw(l.mode, nullptr, a->spec[2 * l.lane], l.win, l.wout, nullptr));
+      a->h_pt.push_back(l.p);
     }
-    a->h_pt.push_back(p);
-    const size_t pi = a->h_pt.size() - 1;
+    for (const QWork& q : qs) plane(pw(MODE_FIRST, q.q, a->spec[2 * q.lane + 1], nullptr, q.wq, nullptr));
+    if (lam.empty()) {
+      step_pass(ops, p0, n);
+      return;
+    }
     ps_adj* A = a;
     ps_handle* H = h;
     const int nx_ = nx, ny_ = ny;
@@ -490,117 +535,172 @@ struct Builder {
       return launch_step_plane_adj(A->d_pw + p0, n, nx_, ny_, H->bd.tw_y, H->bd.tw_z, args, st);
     });
   }
-  void q_pass(std::vector<Op>& ops, const double* q, const double* wq) {
-    step_pass(ops, plane(pw(MODE_FIRST, q, a->spec[1], nullptr, wq, nullptr)), 1);
-  }
-  // x pass of an adjoint step of block b: stress sums of slot, U <- IFFT(K U).
-  void stress_x(std::vector<Op>& ops, int b, int slot) {
-    AdjXWork x;
-    x.u = a->spec[0];
-    x.v = a->spec[1];
-    x.kx = h->bd.kx[ktab(b)];
-    x.kyzc = h->bd.kyzc[ktab(b)];
-    x.part = a->row((size_t)slot * 4);
-    a->h_ax.push_back(x);
-    const size_t xi = a->h_ax.size() - 1;
+  void stress_x(std::vector<Op>& ops, const std::vector<XWork>& xs) {
+    const size_t xi = a->h_ax.size();
+    for (const XWork& w : xs) {
+      AdjXWork x;
+      x.u = a->spec[2 * w.lane];
+      x.v = a->spec[2 * w.lane + 1];
+      x.kx = h->bd.kx[ktab(w.block)];
+      x.kyzc = h->bd.kyzc[ktab(w.block)];
+      x.part = a->row((size_t)w.slot * 4);
+      a->h_ax.push_back(x);
+    }
     ps_adj* A = a;
     ps_handle* H = h;
-    const int nx_ = nx, ny_ = ny, nz_ = nz;
+    const int nx_ = nx, ny_ = ny, nz_ = nz, n = (int)xs.size();
     ops.push_back([=](cudaStream_t st) {
-      return launch_adj_x(A->d_ax + xi, nx_, ny_, nz_, H->cfg.cell[0], H->cfg.cell[1], H->cfg.cell[2], A->stride,
+      return launch_adj_x(A->d_ax + xi, n, nx_, ny_, nz_, H->cfg.cell[0], H->cfg.cell[1], H->cfg.cell[2], A->stride,
                           H->bd.tw_x, st);
     });
   }
-  // Lockstep sweeps over `len` steps.  Sweep i runs steps s0[i] .. s0[i]+len-1
-  // of sweep sig[i] from slice src[i] (nullptr: ones); store(i, k) gives the
-  // destination of its slice k (nullptr: not stored).
-  void sweeps(std::vector<Op>& ops, int nsw, const int* sig, const int* s0, const double* const* src, int len,
-              const std::function<double*(int, int)>& store) {
-    for (int k = 0; k <= len; ++k) {
-      const int mode = (k == 0) ? MODE_FIRST : (k == len ? MODE_LAST : MODE_MID);
-      size_t p0 = 0, y0 = 0;
-      for (int i = 0; i < nsw; ++i) {
-        const std::vector<int>& bl = a->blk[sig[i]];
-        const double* win = (k > 0) ? wf(bl[s0[i] + k - 1]) : nullptr;
-        const double* wout = (k < len) ? wf(bl[s0[i] + k]) : nullptr;
-        const size_t p = plane(pw(mode, k == 0 ? src[i] : nullptr, a->rspec[i], win, wout, store(i, k)));
-        const size_t y = pencil(xw(a->rspec[i], -1));
-        if (i == 0) {
-          p0 = p;
-          y0 = y;
-        }
+  // Every run in one launch.
+  struct Run;
+  bool one_launch(std::vector<Op>& ops, const std::vector<Run>& runs);
+
+  // Lockstep sweeps.  Sweep i runs steps s0 .. s0 + len - 1 of sweep sig from slice
+  // src (nullptr: ones); store(k) gives the destination of its slice k (nullptr: not
+  // stored).
+  struct Run {
+    int sig, s0, len;
+    const double* src;
+    std::function<double*(int)> store;
+  };
+  void sweeps(std::vector<Op>& ops, const std::vector<Run>& runs) {
+    if (one && one_launch(ops, runs)) return;
+    int top = 0;
+    for (const Run& r : runs) top = std::max(top, r.len);
+    for (int k = 0; k <= top; ++k) {
+      const size_t p0 = a->h_pw.size(), y0 = a->h_xw.size();
+      int n = 0;
+      int mode = MODE_MID;  // of the separate passes, whose runs have one length
+      for (size_t i = 0; i < runs.size(); ++i) {
+        const Run& r = runs[i];
+        if (k > r.len) continue;
+        const std::vector<int>& bl = a->blk[r.sig];
+        mode = (k == 0) ? MODE_FIRST : (k == r.len ? MODE_LAST : MODE_MID);
+        const double* win = (k > 0) ? wf(bl[r.s0 + k - 1]) : nullptr;
+        const double* wout = (k < r.len) ? wf(bl[r.s0 + k]) : nullptr;
+        plane(pw(mode, k == 0 ? r.src : nullptr, a->rspec[i], win, wout, r.store(k)));
+        pencil(xw(a->rspec[i], -1));
+        ++n;
       }
-      if (step) step_pass(ops, p0, nsw);
-      else real_pass(ops, p0, nsw, y0, mode);
-      if (k < len) {
-        size_t x0 = 0;
-        for (int i = 0; i < nsw; ++i) {
-          const size_t x = pencil(xw(a->rspec[i], a->blk[sig[i]][s0[i] + k]));
-          if (i == 0) x0 = x;
+      if (step) step_pass(ops, p0, n);
+      else real_pass(ops, p0, n, y0, mode);
+      const size_t x0 = a->h_xw.size();
+      int nx_works = 0;
+      for (size_t i = 0; i < runs.size(); ++i)
+        if (k < runs[i].len) {
+          pencil(xw(a->rspec[i], a->blk[runs[i].sig][runs[i].s0 + k]));
+          ++nx_works;
         }
-        if (step) {
-          ps_adj* A = a;
-          ps_handle* H = h;
-          const int nx_ = nx, inner = ny * nzh;
-          ops.push_back([=](cudaStream_t st) {
-            return launch_step_pencil<double>(A->d_xw + x0, nsw, nx_, inner, true, H->bd.tw_x, st);
-          });
-        } else {
-          x_pass(ops, x0, nsw, PENCIL_KINV);
-        }
+      if (nx_works == 0) continue;
+      if (step) {
+        ps_adj* A = a;
+        ps_handle* H = h;
+        const int nx_ = nx, inner = ny * nzh;
+        ops.push_back([=](cudaStream_t st) {
+          return launch_step_pencil<double>(A->d_xw + x0, nx_works, nx_, inner, true, H->bd.tw_x, st);
+        });
+      } else {
+        x_pass(ops, x0, nx_works, PENCIL_KINV);
       }
     }
   }
 };
 
-// Slice idx of sweep sig while segment j is resident.
-static double* slice_ptr(ps_adj* a, int sig, int idx, int j) {
-  const long long N = a->N;
-  if (a->C == 1) {
-    if (sig == 0) return (idx == a->M) ? a->endq[0] : a->ck[0] + (size_t)idx * N;
-    return (idx == a->M) ? a->endq[1] : a->ck[1] + (size_t)(a->M - 1 - idx) * N;
+bool Builder::one_launch(std::vector<Op>& ops, const std::vector<Run>& runs) {
+  std::vector<SweepWork<double>> ws;
+  for (const Run& r : runs) {
+    SweepWork<double> w;
+    memset(&w, 0, sizeof(w));
+    w.src = r.src;
+    w.status = &h->d_sc->error_flags;
+    w.total = r.len;
+    const std::vector<int>& bl = a->blk[r.sig];
+    int g = 0;
+    for (int k = 0; k < r.len; ++k) {
+      const int b = bl[r.s0 + k];
+      if (k > 0 && b != bl[r.s0 + k - 1] && ++g == kSweepSegs) return false;
+      w.seg[g].wfac = wf(b);
+      w.seg[g].kx = h->bd.kx[ktab(b)];
+      w.seg[g].kyzc = h->bd.kyzc[ktab(b)];
+      w.seg[g].end = k + 1;
+    }
+    ws.push_back(w);
   }
-  if (sig == 0) return a->seg[0] + (size_t)(idx - a->seg_a[j]) * N;
-  return a->seg[1] + (size_t)(idx - (a->M - a->seg_b[j])) * N;
+  const size_t w0 = a->h_sw.size();
+  const int n = (int)ws.size();
+  for (int i = 0; i < n; ++i) {
+    a->sw_dst.push_back(a->h_dst.size());
+    a->h_sw.push_back(ws[i]);
+    for (int k = 0; k <= runs[i].len; ++k) a->h_dst.push_back(runs[i].store(k));
+  }
+  ps_adj* A = a;
+  ps_handle* H = h;
+  const int nx_ = nx, ny_ = ny, nz_ = nz;
+  ops.push_back([=](cudaStream_t st) {
+    return launch_sweep_cluster_to(A->d_sw + w0, n, nx_, ny_, nz_, H->bd.tw_x, H->bd.tw_y, H->bd.tw_z, st);
+  });
+  return true;
 }
 
-static void recompute(Builder& B, std::vector<Op>& ops, int j) {
+// Slice idx of sweep sig while segment j is resident in buffer set `set` (its first
+// slice is the checkpoint).
+static double* slice_ptr(ps_adj* a, int sig, int idx, int j, int set) {
+  const long long N = a->N;
+  if (a->C == 1) {
+    if (idx == a->M) return a->endq[sig];
+    return a->ck[sig] + (size_t)(sig == 0 ? idx : a->M - 1 - idx) * N;
+  }
+  const int at = idx - (sig == 0 ? a->seg_a[j] : a->M - a->seg_b[j]);
+  return at == 0 ? a->ck[sig] + (size_t)j * N : a->seg[set][sig] + (size_t)(at - 1) * N;
+}
+
+// Segment js[set] of both sweeps into buffer set `set`, for n sets.
+static void recompute(Builder& B, std::vector<Op>& ops, const int* js, int n) {
   ps_adj* a = B.a;
   if (a->C == 1) return;
-  const int sig[2] = {0, 1};
-  const int s0[2] = {a->seg_a[j], a->M - a->seg_b[j]};
-  const double* src[2] = {a->ck[0] + (size_t)j * a->N, a->ck[1] + (size_t)j * a->N};
-  const int len = a->seg_b[j] - a->seg_a[j];
-  B.sweeps(ops, 2, sig, s0, src, len, [a](int i, int k) { return a->seg[i] + (size_t)k * a->N; });
+  std::vector<Builder::Run> runs;
+  for (int set = 0; set < n; ++set)
+    for (int sig = 0; sig < 2; ++sig) {
+      const int j = js[set];
+      double* const to = a->seg[set][sig];
+      const long long N = a->N;
+      runs.push_back({sig, sig == 0 ? a->seg_a[j] : a->M - a->seg_b[j], a->seg_b[j] - a->seg_a[j],
+                      a->ck[sig] + (size_t)j * N,
+                      [to, N](int k) { return k == 0 ? nullptr : to + (size_t)(k - 1) * N; }});
+    }
+  B.sweeps(ops, runs);
 }
 
 // Sources of slice idx of sweep sig: every quadrature pair it belongs to, and Q.
-static void fill_sources(ps_adj* a, AdjPoint& p, int sig, int idx, int j) {
+static void fill_sources(ps_adj* a, AdjPoint& p, int sig, int idx, int j, int set) {
   const int n = (sig == 0) ? idx : a->M - idx;
   p.n_src = 0;
   for (auto& e : a->quad[n]) {
     const int f = a->h->blocks[a->ip][e.first].field;
     SrcEntry s;
     s.gphi = a->gphi + (size_t)f * a->N;
-    s.partner = slice_ptr(a, 1 - sig, a->M - idx, j);
+    s.partner = slice_ptr(a, 1 - sig, a->M - idx, j, set);
     s.coef = e.second;
     p.src[p.n_src++] = s;
   }
   const int qslice = (sig == 0) ? a->n0 : a->M - a->n0;
-  p.q_partner = (idx == qslice) ? slice_ptr(a, 1 - sig, a->M - idx, j) : nullptr;
+  p.q_partner = (idx == qslice) ? slice_ptr(a, 1 - sig, a->M - idx, j, set) : nullptr;
 }
 
 // One adjoint step through block b: mu = wf G(wf lam_next), the stress
 // partials of (U, V) = (FFT(wf lam_next), FFT(wf q_s)), dL/dw of the step and,
 // when lam_out is set, lam_s = mu + the explicit sources of slice s (in `src`).
 static AdjPoint step_point(Builder& B, int b, int slot, const double* q_s, const double* q_next,
-                           const double* lam_next, double* lam_out, const AdjPoint& src, int b2 = -1) {
+                           const double* lam_next, double* lam_out, const AdjPoint& src, int b2 = -1, int lane = 0) {
   ps_adj* a = B.a;
   ps_handle* h = B.h;
   const BlockMap& bm = h->blocks[a->ip][b];
   AdjPoint p = src;
   if (b2 >= 0) {
-    p.gwb2 = a->gwb + (size_t)b2 * a->N;
+    p.gwb2 = a->gwb + (size_t)(lane * a->nb + b2) * a->N;
     p.half_ds2 = 0.5 * h->blocks[a->ip][b2].ds;
   }
   p.mu = a->mu;
@@ -608,7 +708,7 @@ static AdjPoint step_point(Builder& B, int b, int slot, const double* q_s, const
   p.q_s = q_s;
   p.q_next = q_next;
   p.w = h->d_w + (size_t)bm.field * a->N;
-  p.gwb = a->gwb + (size_t)b * a->N;
+  p.gwb = a->gwb + (size_t)(lane * a->nb + b) * a->N;
   p.lam_out = lam_out;
   p.dsw_part = a->row((size_t)slot * 4 + 3);
   p.half_ds = 0.5 * bm.ds;
@@ -668,43 +768,69 @@ static void adjoint_step(Builder& B, std::vector<Op>& ops, int sig, int s, int j
   ps_adj* a = B.a;
   AdjPoint src;
   memset(&src, 0, sizeof(src));
-  if (s >= 1) fill_sources(a, src, sig, s, j);
-  adjoint_step_p(B, ops, a->blk[sig][s], slice_ptr(a, sig, s, j), slice_ptr(a, sig, s + 1, j), a->lam[cur],
+  if (s >= 1) fill_sources(a, src, sig, s, j, 0);
+  adjoint_step_p(B, ops, a->blk[sig][s], slice_ptr(a, sig, s, j, 0), slice_ptr(a, sig, s + 1, j, 0), a->lam[cur],
                  (s >= 1) ? a->lam[1 - cur] : nullptr, src);
 }
 
-// The adjoint steps seg_hi - 1 .. seg_lo of sweep sig while segment j is resident,
-// fused: one plane pass and one x pass a step.  At the sweep's end (first) lambda
-// starts there; at later segments only q's transform is missing.
-static void adjoint_segment(Builder& B, std::vector<Op>& ops, int sig, int j, int lo, int hi, bool first, int& cur) {
+// The adjoint steps hi - 1 .. lo of sweep sig while segment j is resident in `set`.
+struct SegRun {
+  int sig, j, set, lo, hi;
+  bool first;  // lambda starts here (the sweep's end); at later segments only q's transform is missing
+};
+
+// The runs' steps, fused: one plane pass and one x pass a step for all of them.  Run i
+// is lane i; cur[i] says which of the lane's two lambda buffers is current.
+static void adjoint_segments(Builder& B, std::vector<Op>& ops, const std::vector<SegRun>& runs, int* cur) {
   ps_adj* a = B.a;
-  const std::vector<int>& bl = a->blk[sig];
-  const double* wtop = B.wf(bl[hi - 1]);
-  if (first) {
-    AdjPoint p;
-    memset(&p, 0, sizeof(p));
-    p.lam_out = a->lam[cur];
-    p.q_s = slice_ptr(a, sig, hi, j);
-    p.gwb2 = a->gwb + (size_t)bl[hi - 1] * a->N;
-    p.half_ds2 = 0.5 * B.h->blocks[a->ip][bl[hi - 1]].ds;
-    fill_sources(a, p, sig, hi, j);
-    B.lambda_pass(ops, MODE_ADJ_INIT, p, nullptr, wtop, slice_ptr(a, sig, hi - 1, j), wtop);
-  } else {
-    B.q_pass(ops, slice_ptr(a, sig, hi - 1, j), wtop);
+  std::vector<Builder::LamWork> lam;
+  std::vector<Builder::QWork> qs;
+  std::vector<Builder::XWork> xs;
+  int top = 0;
+  for (size_t i = 0; i < runs.size(); ++i) {
+    const SegRun& r = runs[i];
+    const int lane = (int)i;
+    const int b = a->blk[r.sig][r.hi - 1];
+    top = std::max(top, r.hi - r.lo);
+    if (r.first) {
+      AdjPoint p;
+      memset(&p, 0, sizeof(p));
+      p.lam_out = a->lam[2 * lane + cur[i]];
+      p.q_s = slice_ptr(a, r.sig, r.hi, r.j, r.set);
+      p.gwb2 = a->gwb + (size_t)(lane * a->nb + b) * a->N;
+      p.half_ds2 = 0.5 * B.h->blocks[a->ip][b].ds;
+      fill_sources(a, p, r.sig, r.hi, r.j, r.set);
+      lam.push_back({MODE_ADJ_INIT, lane, p, nullptr, B.wf(b)});
+    }
+    qs.push_back({lane, slice_ptr(a, r.sig, r.hi - 1, r.j, r.set), B.wf(b)});
   }
-  for (int s = hi - 1; s >= lo; --s) {
-    const int slot = (int)a->slot_block.size();
-    a->slot_block.push_back(bl[s]);
-    B.stress_x(ops, bl[s], slot);
-    AdjPoint src;
-    memset(&src, 0, sizeof(src));
-    if (s >= 1) fill_sources(a, src, sig, s, j);
-    const AdjPoint p = step_point(B, bl[s], slot, slice_ptr(a, sig, s, j), slice_ptr(a, sig, s + 1, j), a->lam[cur],
-                                  (s >= 1) ? a->lam[1 - cur] : nullptr, src, s >= 1 ? bl[s - 1] : -1);
-    const double* wn = (s >= 1) ? B.wf(bl[s - 1]) : nullptr;
-    B.lambda_pass(ops, s >= 1 ? MODE_ADJ_MID : MODE_ADJ_LAST, p, B.wf(bl[s]), wn,
-                  s > lo ? slice_ptr(a, sig, s - 1, j) : nullptr, wn);
-    cur = 1 - cur;
+  B.lambda_pass(ops, lam, qs);
+  for (int k = 1; k <= top; ++k) {
+    lam.clear();
+    qs.clear();
+    xs.clear();
+    for (size_t i = 0; i < runs.size(); ++i) {
+      const SegRun& r = runs[i];
+      const int s = r.hi - k, lane = (int)i;
+      if (s < r.lo) continue;
+      const std::vector<int>& bl = a->blk[r.sig];
+      const int slot = r.sig * a->M + (a->M - 1 - s);
+      a->slot_block[slot] = bl[s];
+      xs.push_back({lane, bl[s], slot});
+      AdjPoint src;
+      memset(&src, 0, sizeof(src));
+      if (s >= 1) fill_sources(a, src, r.sig, s, r.j, r.set);
+      double* const* const l = a->lam + 2 * lane;
+      const AdjPoint p =
+          step_point(B, bl[s], slot, slice_ptr(a, r.sig, s, r.j, r.set), slice_ptr(a, r.sig, s + 1, r.j, r.set),
+                     l[cur[i]], (s >= 1) ? l[1 - cur[i]] : nullptr, src, s >= 1 ? bl[s - 1] : -1, lane);
+      const double* wn = (s >= 1) ? B.wf(bl[s - 1]) : nullptr;
+      lam.push_back({s >= 1 ? MODE_ADJ_MID : MODE_ADJ_LAST, lane, p, B.wf(bl[s]), wn});
+      if (s > r.lo) qs.push_back({lane, slice_ptr(a, r.sig, s - 1, r.j, r.set), wn});
+      cur[i] = 1 - cur[i];
+    }
+    B.stress_x(ops, xs);
+    B.lambda_pass(ops, lam, qs);
   }
 }
 
@@ -712,7 +838,7 @@ static void adjoint_init(ps_adj* a, std::vector<Op>& ops, int sig, int j, int cu
   AdjPoint p;
   memset(&p, 0, sizeof(p));
   p.lam_out = a->lam[cur];
-  fill_sources(a, p, sig, a->M, j);
+  fill_sources(a, p, sig, a->M, j, 0);
   a->h_pt.push_back(p);
   const size_t pi = a->h_pt.size() - 1;
   const long long N = a->N;
@@ -948,11 +1074,11 @@ static int tree_build(ps_adj* a, int ec) {
         p0.half_ds2 = 0.5 * h->blocks[ip][bl[T - 1]].ds;
         fill(p0, t, T);
         p0.extra = a->jacc[t];
-        B.lambda_pass(a->bwd, MODE_ADJ_INIT, p0, nullptr, B.wf(bl[T - 1]), S(sw, T - 1), B.wf(bl[T - 1]));
+        B.lambda_pass(a->bwd, {{MODE_ADJ_INIT, 0, p0, nullptr, B.wf(bl[T - 1])}}, {{0, S(sw, T - 1), B.wf(bl[T - 1])}});
         for (int st_ = T - 1; st_ >= 0; --st_) {
           const int slot = (int)a->slot_block.size();
           a->slot_block.push_back(bl[st_]);
-          B.stress_x(a->bwd, bl[st_], slot);
+          B.stress_x(a->bwd, {{0, bl[st_], slot}});
           AdjPoint src_;
           memset(&src_, 0, sizeof(src_));
           const bool out = (st_ >= 1) || junction;
@@ -960,8 +1086,9 @@ static int tree_build(ps_adj* a, int ec) {
           const AdjPoint p = step_point(B, bl[st_], slot, S(sw, st_), S(sw, st_ + 1), a->lam[cur],
                                         out ? a->lam[1 - cur] : nullptr, src_, st_ >= 1 ? bl[st_ - 1] : -1);
           const double* wn = (st_ >= 1) ? B.wf(bl[st_ - 1]) : nullptr;
-          B.lambda_pass(a->bwd, st_ >= 1 ? MODE_ADJ_MID : MODE_ADJ_LAST, p, B.wf(bl[st_]), wn,
-                        st_ >= 1 ? S(sw, st_ - 1) : nullptr, wn);
+          std::vector<Builder::QWork> q;
+          if (st_ >= 1) q.push_back({0, S(sw, st_ - 1), wn});
+          B.lambda_pass(a->bwd, {{st_ >= 1 ? MODE_ADJ_MID : MODE_ADJ_LAST, 0, p, B.wf(bl[st_]), wn}}, q);
           if (out) cur = 1 - cur;
         }
       } else {
@@ -1121,18 +1248,26 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
   const size_t NB = sizeof(double) * (size_t)a->N;
   const size_t nspec = (size_t)h->n[0] * h->n[1] * h->nzh;
   PA_CUDA(a, cudaSetDevice(h->dev));
+  Builder B(a, h);
+  a->pair = B.adj && h->n[0] <= 96;  // see the header
+  const int lanes = a->pair ? 2 : 1;
+  const int sets = C == 1 ? 0 : lanes;
   for (int sg = 0; sg < 2; ++sg) {
     PA_CUDA(a, cudaMalloc((void**)&a->ck[sg], NB * a->J));
-    PA_CUDA(a, cudaMalloc((void**)&a->endq[sg], NB));
-    if (C > 1) PA_CUDA(a, cudaMalloc((void**)&a->seg[sg], NB * (C + 1)));
-    PA_CUDA(a, cudaMalloc((void**)&a->lam[sg], NB));
-    PA_CUDA(a, cudaMalloc((void**)&a->spec[sg], sizeof(double2) * nspec));
-    PA_CUDA(a, cudaMalloc((void**)&a->rspec[sg], sizeof(double2) * nspec));
+    for (int set = 0; set < sets; ++set) PA_CUDA(a, cudaMalloc((void**)&a->seg[set][sg], NB * C));
+    // the last slices are needed for Q alone: in checkpointed runs they pass through a segment buffer
+    if (C == 1) PA_CUDA(a, cudaMalloc((void**)&a->endq[sg], NB));
+    else a->endq[sg] = a->seg[0][sg];
   }
-  a->storage_bytes = NB * (2 * (size_t)a->J + 2 + (C > 1 ? 2 * (size_t)(C + 1) : 0));
+  for (int i = 0; i < 2 * lanes; ++i) {
+    PA_CUDA(a, cudaMalloc((void**)&a->lam[i], NB));
+    PA_CUDA(a, cudaMalloc((void**)&a->spec[i], sizeof(double2) * nspec));
+    PA_CUDA(a, cudaMalloc((void**)&a->rspec[i], sizeof(double2) * nspec));
+  }
+  a->storage_bytes = NB * (2 * (size_t)a->J + (C > 1 ? 2 * (size_t)sets * C : 2));
   PA_CUDA(a, cudaMalloc((void**)&a->mu, NB));
   PA_CUDA(a, cudaMalloc((void**)&a->P, NB * a->nb));
-  PA_CUDA(a, cudaMalloc((void**)&a->gwb, NB * a->nb));
+  PA_CUDA(a, cudaMalloc((void**)&a->gwb, NB * a->nb * lanes));
   PA_CUDA(a, cudaMalloc((void**)&a->gphi, NB * a->nf));
   PA_CUDA(a, cudaMemset(a->gphi, 0, NB * a->nf));
   PA_CUDA(a, cudaMalloc((void**)&a->gq, sizeof(double)));
@@ -1141,23 +1276,23 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
     if (rp) return rp;
   }
 
-  Builder B(a, h);
   const BlockFieldMap fm = field_map(a);
   const long long N = a->N;
+  if (B.adj) a->slot_block.assign(2 * (size_t)M, 0);
 
   // ---- forward: both sweeps in lockstep, checkpoints and end slices stored
   {
-    const int sig[2] = {0, 1};
-    const int st0[2] = {0, 0};
-    const double* src[2] = {nullptr, nullptr};
-    B.sweeps(a->fwd, 2, sig, st0, src, M, [a, M](int i, int k) -> double* {
-      if (k == M) return a->endq[i];
-      for (int j = 0; j < a->J; ++j) {
-        const int pos = (i == 0) ? a->seg_a[j] : M - a->seg_b[j];
-        if (pos == k) return a->ck[i] + (size_t)j * a->N;
-      }
-      return nullptr;
-    });
+    std::vector<Builder::Run> runs;
+    for (int i = 0; i < 2; ++i)
+      runs.push_back({i, 0, M, nullptr, [a, M, i](int k) -> double* {
+                        if (k == M) return a->endq[i];
+                        for (int j = 0; j < a->J; ++j) {
+                          const int pos = (i == 0) ? a->seg_a[j] : M - a->seg_b[j];
+                          if (pos == k) return a->ck[i] + (size_t)j * a->N;
+                        }
+                        return nullptr;
+                      }});
+    B.sweeps(a->fwd, runs);
     // Q = <q_n0 q+_{M-n0}>
     const double* qx = (a->n0 == 0) ? a->ck[0] : a->endq[0];
     const double* qy = (a->n0 == 0) ? a->endq[1] : a->ck[1] + (size_t)(a->J - 1) * N;
@@ -1170,24 +1305,31 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
     });
     // quadrature, segment by segment
     a->fwd.push_back([=](cudaStream_t st) { return cudaMemsetAsync(a->P, 0, sizeof(double) * N * a->nb, st); });
-    for (int j = 0; j < a->J; ++j) {
-      recompute(B, a->fwd, j);
-      const size_t e0 = a->h_acc.size();
-      const int nend = (j == a->J - 1) ? a->seg_b[j] : a->seg_b[j] - 1;
-      for (int n = a->seg_a[j]; n <= nend; ++n)
-        for (auto& e : a->quad[n]) {
-          AccumEntry ae;
-          ae.dst = a->P + (size_t)e.first * N;
-          ae.x = slice_ptr(a, 0, n, j);
-          ae.y = slice_ptr(a, 1, M - n, j);
-          ae.coef = e.second;
-          a->h_acc.push_back(ae);
-        }
+    size_t e0 = 0;
+    const int group = C == 1 ? a->J : lanes;  // segments resident together
+    for (int j0 = 0; j0 < a->J; j0 += group) {
+      const int n = std::min(group, a->J - j0);
+      const int js[2] = {j0, j0 + 1};
+      recompute(B, a->fwd, js, n);
+      for (int j = j0; j < j0 + n; ++j) {
+        const int nend = (j == a->J - 1) ? a->seg_b[j] : a->seg_b[j] - 1;
+        for (int n_ = a->seg_a[j]; n_ <= nend; ++n_)
+          for (auto& e : a->quad[n_]) {
+            AccumEntry ae;
+            ae.dst = a->P + (size_t)e.first * N;
+            ae.x = slice_ptr(a, 0, n_, j, j - j0);
+            ae.y = slice_ptr(a, 1, M - n_, j, j - j0);
+            ae.coef = e.second;
+            a->h_acc.push_back(ae);
+          }
+      }
       const int ne = (int)(a->h_acc.size() - e0);
+      const size_t off = e0;
       a->fwd.push_back([=](cudaStream_t st) {
-        adj_accum_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->d_acc + e0, ne, N);
+        adj_accum_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->d_acc + off, ne, N);
         return cudaGetLastError();
       });
+      e0 = a->h_acc.size();
     }
     a->fwd.push_back([=](cudaStream_t st) {
       adj_normalize_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->P, h->d_phi, fm, N, h->d_sc);
@@ -1210,35 +1352,56 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
         return cudaGetLastError();
       });
     }
-    a->bwd.push_back([=](cudaStream_t st) { return cudaMemsetAsync(a->gwb, 0, sizeof(double) * N * a->nb, st); });
-    // sweep 0: lambda from n = M down, segments last to first
-    int cur = 0;
-    for (int j = a->J - 1; j >= 0; --j) {
-      recompute(B, a->bwd, j);
-      if (B.adj) {
-        adjoint_segment(B, a->bwd, 0, j, a->seg_a[j], a->seg_b[j], j == a->J - 1, cur);
-        continue;
+    a->bwd.push_back(
+        [=](cudaStream_t st) { return cudaMemsetAsync(a->gwb, 0, sizeof(double) * N * a->nb * lanes, st); });
+    // sweep 0: lambda from n = M down, segments last to first; sweep 1: lambda+ from
+    // m = M down, segments first to last
+    int cur[2] = {0, 0};
+    auto seg_run = [&](int sig, int j, int set, bool first) {
+      return SegRun{sig, j, set, sig == 0 ? a->seg_a[j] : M - a->seg_b[j], sig == 0 ? a->seg_b[j] : M - a->seg_a[j],
+                    first};
+    };
+    if (B.adj && C == 1) {  // every slice is resident
+      const SegRun all[2] = {{0, 0, 0, 0, M, true}, {1, 0, 0, 0, M, true}};
+      if (a->pair) {
+        adjoint_segments(B, a->bwd, {all[0], all[1]}, cur);
+      } else {
+        for (int sig = 0; sig < 2; ++sig) {
+          cur[0] = 0;
+          adjoint_segments(B, a->bwd, {all[sig]}, cur);
+        }
       }
-      if (j == a->J - 1) adjoint_init(a, a->bwd, 0, j, cur);
-      for (int s = a->seg_b[j] - 1; s >= a->seg_a[j]; --s) {
-        adjoint_step(B, a->bwd, 0, s, j, cur);
-        cur = 1 - cur;
+    } else if (a->pair) {
+      for (int t = 0; t < a->J; ++t) {
+        const int js[2] = {a->J - 1 - t, t};
+        const int n = js[0] == js[1] ? 1 : 2;
+        recompute(B, a->bwd, js, n);
+        adjoint_segments(B, a->bwd, {seg_run(0, js[0], 0, t == 0), seg_run(1, js[1], n - 1, t == 0)}, cur);
+      }
+    } else {
+      for (int sig = 0; sig < 2; ++sig) {
+        cur[0] = 0;
+        for (int t = 0; t < a->J; ++t) {
+          const int j = sig == 0 ? a->J - 1 - t : t;
+          recompute(B, a->bwd, &j, 1);
+          const SegRun run = seg_run(sig, j, 0, t == 0);
+          if (B.adj) {
+            adjoint_segments(B, a->bwd, {run}, cur);
+            continue;
+          }
+          if (t == 0) adjoint_init(a, a->bwd, sig, j, cur[0]);
+          for (int s = run.hi - 1; s >= run.lo; --s) {
+            adjoint_step(B, a->bwd, sig, s, j, cur[0]);
+            cur[0] = 1 - cur[0];
+          }
+        }
       }
     }
-    // sweep 1: lambda+ from m = M down, i.e. segments first to last
-    cur = 0;
-    for (int j = 0; j < a->J; ++j) {
-      recompute(B, a->bwd, j);
-      if (B.adj) {
-        adjoint_segment(B, a->bwd, 1, j, M - a->seg_b[j], M - a->seg_a[j], j == 0, cur);
-        continue;
-      }
-      if (j == 0) adjoint_init(a, a->bwd, 1, j, cur);
-      for (int m = M - a->seg_a[j] - 1; m >= M - a->seg_b[j]; --m) {
-        adjoint_step(B, a->bwd, 1, m, j, cur);
-        cur = 1 - cur;
-      }
-    }
+    if (a->pair)  // the lanes' sums
+      a->bwd.push_back([=](cudaStream_t st) {
+        adj_axpy_kernel<<<kAdjRB, kAdjRT, 0, st>>>(a->gwb, a->gwb + (size_t)a->nb * N, 1.0, N * a->nb);
+        return cudaGetLastError();
+      });
   }
   push_dotw(B, a->bwd);
   int r2 = adj_upload(a, &a->d_pw, a->h_pw);
@@ -1246,6 +1409,9 @@ static int adj_build(ps_adj* a, const ps_config* cfg, int polymer, int chain, bo
   if (!r2) r2 = adj_upload(a, &a->d_acc, a->h_acc);
   if (!r2) r2 = adj_upload(a, &a->d_pt, a->h_pt);
   if (!r2) r2 = adj_upload(a, &a->d_ax, a->h_ax);
+  if (!r2) r2 = adj_upload(a, &a->d_dst, a->h_dst);
+  for (size_t i = 0; i < a->h_sw.size(); ++i) a->h_sw[i].dst = a->d_dst + a->sw_dst[i];
+  if (!r2) r2 = adj_upload(a, &a->d_sw, a->h_sw);
   return r2;
 }
 
@@ -1257,11 +1423,13 @@ static void adj_free(ps_adj* a) {
   auto f = [](void* p) { if (p) cudaFree(p); };
   for (int sg = 0; sg < 2; ++sg) {
     f(a->ck[sg]);
-    f(a->endq[sg]);
-    f(a->seg[sg]);
-    f(a->lam[sg]);
-    f(a->spec[sg]);
-    f(a->rspec[sg]);
+    if (a->C == 1) f(a->endq[sg]);
+    for (int set = 0; set < 2; ++set) f(a->seg[set][sg]);
+  }
+  for (int i = 0; i < 4; ++i) {
+    f(a->lam[i]);
+    f(a->spec[i]);
+    f(a->rspec[i]);
   }
   f(a->mu);
   f(a->P);
@@ -1271,6 +1439,8 @@ static void adj_free(ps_adj* a) {
   f(a->part);
   f(a->d_sum);
   f(a->d_ax);
+  f(a->d_sw);
+  f(a->d_dst);
   if (a->h_sum) cudaFreeHost(a->h_sum);
   f(a->d_pw);
   f(a->d_xw);
@@ -1440,7 +1610,13 @@ int ps_adj_backward(ps_adj* a, const double* g_phi, double g_log_q, double* g_w,
   adj_rows_kernel<<<(unsigned)a->rows, kAdjRT, 0, h->st>>>(a->part, a->stride, a->d_sum);
   PA_CUDA(a, cudaGetLastError());
   PA_CUDA(a, cudaMemcpyAsync(a->h_sum, a->d_sum, sizeof(double) * a->rows, cudaMemcpyDeviceToHost, h->st));
+  PA_CUDA(a, cudaMemcpyAsync(&h->h_sc->error_flags, &h->d_sc->error_flags, sizeof(int), cudaMemcpyDeviceToHost,
+                             h->st));
   PA_CUDA(a, cudaStreamSynchronize(h->st));
+  if (h->h_sc->error_flags & 4) {
+    a->err = "an exchange of a recomputed sweep did not complete within the wait limit";
+    return PS_GPU_ERR;
+  }
   // host sums in a fixed order
   double gbox[3] = {0.0, 0.0, 0.0};
   std::vector<double> gds(a->nb, 0.0);

@@ -71,7 +71,7 @@ struct AdjXWork {
   double* part;
 };
 int adj_x_tiles(int nx, int inner);  // CTAs of the pass
-cudaError_t launch_adj_x(const AdjXWork* d_work, int nx, int ny, int nz, double dx, double dy, double dz, int stride,
+cudaError_t launch_adj_x(const AdjXWork* d_works, int nworks, int nx, int ny, int nz, double dx, double dy, double dz, int stride,
                          const double2* tw, cudaStream_t st);
 
 }  // namespace psb

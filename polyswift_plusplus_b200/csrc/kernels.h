@@ -75,6 +75,7 @@ constexpr int kSweepSegs = 16;
 template <typename T> struct SweepWork {
   const T* src;  // initial q (nullptr = ones)
   T* slices;
+  T* const* dst;    // where slice k goes (nullptr in it: nowhere); launch_sweep_cluster_to alone
   int* status;      // error word: bit 2 set when a cluster exchange did not arrive in time
   int total;
   int dc;           // mean-mode carry (see PlaneWork)
@@ -93,6 +94,9 @@ bool sweep_cluster_supported(int nx, int ny, int nz);
 template <typename T>
 cudaError_t launch_sweep_cluster(const SweepWork<T>* d_works, int nworks, int nx, int ny, int nz, const c2_t<T>* tw_x,
                                  const c2_t<T>* tw_y, const c2_t<T>* tw_z, cudaStream_t st);
+// ... with every slice's place in dst.
+cudaError_t launch_sweep_cluster_to(const SweepWork<double>* d_works, int nworks, int nx, int ny, int nz,
+                                    const double2* tw_x, const double2* tw_y, const double2* tw_z, cudaStream_t st);
 // Poll limit of its waits (ps_gpu_set_bulk_wait_limit).
 cudaError_t sweep_cluster_set_polls(uint32_t polls);
 

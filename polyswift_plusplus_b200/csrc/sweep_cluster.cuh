@@ -113,7 +113,8 @@ template <typename T, int NX, int NY, int NZ, int CL_> struct SweepCl {
 // Poll limit of the waits below (see ps_gpu_set_bulk_wait_limit).
 static __constant__ uint32_t c_sweep_wait_polls = kMaxPolls;
 
-template <typename T, int NX, int NY, int NZ, int CL_>
+// DST: the slices' places come from w.dst (1% of a step at 16^3 as a run-time choice).
+template <typename T, int NX, int NY, int NZ, int CL_, bool DST>
 __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
     sweep_cluster_kernel(const SweepWork<T>* __restrict__ works, const c2_t<T>* __restrict__ tw_x,
                          const c2_t<T>* __restrict__ tw_y, const c2_t<T>* __restrict__ tw_z) {
@@ -225,6 +226,8 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
   load_ktab(0);
 
   for (int k = 0; k <= total; ++k) {
+    T* slice = nullptr;
+    if constexpr (DST) slice = w.dst[k];
     // ---- y inverse -------------------------------------------------------
     if (k > 0) wait(bar_a, (uint32_t)(k - 1), bytes_a, k < total);
     if (!FILM && k > 0) {
@@ -346,8 +349,8 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
           for (int u = 0; u < UZ; ++u) q[u][r] = C{x.v[u], x2.v[u]};
         }
       }
-      if (on) {
-        T* const st = slices + (size_t)k * ((size_t)NX * NY * NZ) + ra;
+      if (on && (!DST || slice)) {
+        T* const st = (DST ? slice : slices + (size_t)k * ((size_t)NX * NY * NZ)) + ra;
 #pragma unroll
         for (int r = 0; r < GZ; ++r) {
           RealRun<T, UZ> x, x2;
@@ -556,11 +559,11 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
   cl_sync();  // no CTA leaves while another may still write to it
 }
 
-template <typename T, int NX, int NY, int NZ, int CL>
+template <typename T, int NX, int NY, int NZ, int CL, bool DST>
 cudaError_t launch_sweep_cluster_t(const SweepWork<T>* d_works, int nworks, const c2_t<T>* tx, const c2_t<T>* ty,
                                    const c2_t<T>* tz, cudaStream_t st) {
   using P = SweepCl<T, NX, NY, NZ, CL>;
-  auto kern = sweep_cluster_kernel<T, NX, NY, NZ, CL>;
+  auto kern = sweep_cluster_kernel<T, NX, NY, NZ, CL, DST>;
   static unsigned attr_mask = 0;
   cudaError_t e = ensure_smem_attr(kern, P::SMEM, &attr_mask);
   if (e != cudaSuccess) return e;

@@ -79,3 +79,54 @@ def test_fused_adjoint_steps(gpu, m):
         for got, ref in ((phi, tphi.detach()), (gw, wt.grad), (torch.tensor(gbox), box.grad), (torch.tensor(gds), ds.grad)):
             assert (got - ref).abs().max().item() <= 1e-10 * ref.abs().max().item(), (m, checkpoint)
         adj.close()
+
+
+@pytest.mark.parametrize("n", [(16, 16, 16), (48, 48, 48), (24, 32, 32), (128, 16, 16)])
+def test_adjoint_schedules(gpu, n):
+    """One-launch and stepwise sweeps, both adjoints together (nx <= 96) and one at a time: the
+    results do not depend on the checkpoint interval (whole, uneven and single segments), bit for
+    bit, and match torch."""
+    cfg = W.diblock_config(16, 2.0, 0.35, 20.0, 20, W.Updater(kind="steepestDescent"), "fp64")
+    cfg = dataclasses.replace(cfg, n=n, cell=(0.08, 0.07, 0.06))
+    rng = np.random.default_rng(sum(n))
+    w = torch.tensor(rng.uniform(-1, 1, (2, cfg.n_total)), device="cuda")
+    gphi = torch.tensor(rng.standard_normal((2, cfg.n_total)), device="cuda")
+    wt = w.clone().requires_grad_(True)
+    box = torch.tensor([cfg.n[d] * cfg.cell[d] for d in range(3)], dtype=torch.float64, requires_grad=True)
+    ds = torch.full((2,), 1.0 / 20, dtype=torch.float64, requires_grad=True)
+    tphi, tlnq = _torch_forward(cfg, wt, box, ds)
+    ((tphi * gphi).sum() + 0.7 * tlnq).backward()
+    first = None
+    for checkpoint in (1, 0, 7, 20):
+        adj = ChainAdjoint(cfg, checkpoint=checkpoint)
+        for again in range(2):
+            phi, lnq = adj.forward(w)
+            gw, gbox, gds = adj.backward(gphi, 0.7)
+            got = [phi, torch.tensor([lnq], dtype=torch.float64), gw, torch.tensor(gbox), torch.tensor(gds)]
+            if first is None:
+                first = got
+            assert all(torch.equal(a, b) for a, b in zip(got, first)), (n, checkpoint, again)
+        adj.close()
+    for got, ref in zip(first, (tphi.detach(), tlnq.detach().cpu().reshape(1), wt.grad, box.grad, ds.grad)):
+        assert (got - ref).abs().max().item() <= 1e-10 * max(ref.abs().max().item(), 1e-2), n
+
+
+def test_adjoint_wait_timeout_is_reported(gpu):
+    """With a poll limit of 0 the one-launch sweeps' waits give up: forward and backward report it."""
+    from polyswift_plusplus_b200 import _abi as A
+    cfg = W.diblock_config(16, 2.0, 0.35, 20.0, 20, W.Updater(kind="steepestDescent"), "fp64")
+    w = torch.zeros((2, cfg.n_total), dtype=torch.float64, device="cuda")
+    adj = ChainAdjoint(cfg)
+    for step in ("forward", "backward"):
+        if step == "backward":
+            ref, _ = adj.forward(w)
+        assert gpu.ps_gpu_set_bulk_wait_limit(0) == A.PS_OK
+        try:
+            with pytest.raises(A.PsError) as ei:
+                adj.forward(w) if step == "forward" else adj.backward(torch.ones_like(w), 1.0)
+        finally:
+            assert gpu.ps_gpu_set_bulk_wait_limit(0xFFFFFFFF) == A.PS_OK
+        assert ei.value.code == A.PS_GPU_ERR and "wait limit" in str(ei.value)
+    phi, _ = adj.forward(w)
+    assert torch.equal(phi, ref)
+    adj.close()
