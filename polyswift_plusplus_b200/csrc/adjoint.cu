@@ -599,8 +599,11 @@ struct Builder {
         ps_adj* A = a;
         ps_handle* H = h;
         const int nx_ = nx, inner = ny * nzh;
+        // the plane pass behind it starts early (early_path in sweeps.cuh): 64^3 7.65 -> 7.4 ms,
+        // 96^3 23.4 -> 23.0
+        const bool early = nx <= 96 && a->N <= 96LL * 96 * 96;
         ops.push_back([=](cudaStream_t st) {
-          return launch_step_pencil<double>(A->d_xw + x0, nx_works, nx_, inner, true, H->bd.tw_x, st);
+          return launch_step_pencil<double>(A->d_xw + x0, nx_works, nx_, inner, true, early, H->bd.tw_x, st);
         });
       } else {
         x_pass(ops, x0, nx_works, PENCIL_KINV);

@@ -65,12 +65,12 @@ __device__ __forceinline__ C mul_mi(C a) {
 // of it on the stream has finished: it does its independent prologue (twiddle
 // tables, work descriptors), then pdl_wait() blocks until that kernel has
 // completed and its writes are visible; without the attribute pdl_wait() is a
-// no-op.  No kernel triggers its dependents early: blocks of the next sweep
-// kernel parked on pdl_wait() hold shared memory and registers that the
-// concurrent sweep's kernels need.  At 128^3 a trigger after the loads was 4%
-// slower, and a late one (plane pass after its real-space step, pencil pass
-// after its k^2 pass) 2-3% slower, although it cut the time from the last
-// block's exit to the next kernel's release from about 2.5 to 1.6 us.
+// no-op.  Kernels do not trigger their dependents early as a rule: blocks of the next
+// sweep kernel parked on pdl_wait() hold shared memory and registers that the
+// concurrent sweep's kernels need, and land where this kernel's blocks have left room
+// instead of evenly.  At 128^3 a trigger in the plane pass, early or late, was 2-4%
+// slower.  The x pass can (VARIANT_EARLY).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 }  // namespace psb

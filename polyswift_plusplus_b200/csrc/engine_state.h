@@ -159,6 +159,7 @@ struct ps_handle {
   int eager_iters = 0;
   long long launches_per_iter = 0;
   int variant = -1;  // kernel variant (VARIANT_* bits); -1: autotune before the graph is built
+  int early = 0;     // VARIANT_EARLY where the autotuner found it faster
   float tune_ms[psb::VARIANT_COUNT] = {};
   bool xy_ok = false;  // the row + x-y plane design exists for this grid
   bool cluster_ok = false;  // the two-CTA cluster plane pass exists for this grid and precision

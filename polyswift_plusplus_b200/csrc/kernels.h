@@ -125,7 +125,8 @@ enum {
   VARIANT_XY = 4,
   VARIANT_SPLIT = 8,
   VARIANT_CLUSTER = 16,
-  VARIANT_COUNT = 32
+  VARIANT_COUNT = 32,
+  VARIANT_EARLY = 32  // beside a variant, chosen by the autotuner alone: see early_path in sweeps.cuh
 };
 bool cluster_plane_supported(int prec_bytes, int ny, int nz);
 // The cluster plane pass (ny = nz = 256): grid 8 nx x nworks, eight CTAs per
@@ -165,7 +166,7 @@ template <typename T>
 cudaError_t launch_step_plane(const PlaneWork<T>* d_works, int nworks, int nx, int ny, int nz,
                               const c2_t<T>* tw_y, const c2_t<T>* tw_z, cudaStream_t st);
 template <typename T>
-cudaError_t launch_step_pencil(const PencilWork<T>* d_works, int nworks, int L, int inner, bool compact,
+cudaError_t launch_step_pencil(const PencilWork<T>* d_works, int nworks, int L, int inner, bool compact, bool early,
                                const c2_t<T>* tw, cudaStream_t st);
 
 // The step with the y transform split over the two passes (step_split.cuh), and the

@@ -25,7 +25,9 @@ template <typename T, int L> struct PencilG {
   static_assert(R * G == L && TH >= 32, "pencil groups");
 };
 
-template <typename T, int L>
+// EARLY: see early_path in sweeps.cuh (a template argument: as a run-time one it cost up to
+// 4% of an FP32 step at 48^3).
+template <typename T, int L, bool EARLY>
 __global__ void __launch_bounds__((PencilG<T, L>::TH))
     step_pencil_kernel(const PencilWork<T>* __restrict__ works, int inner, int compact,
                        const c2_t<T>* __restrict__ tw) {
@@ -48,6 +50,7 @@ __global__ void __launch_bounds__((PencilG<T, L>::TH))
   }
   const T fyz = in ? __ldg((compact ? w.kyzc : w.kyz) + c) : T(0);
   pdl_wait();  // before any read or write of the spectrum
+  if constexpr (EARLY) pdl_trigger();
   C v[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) v[r] = in ? __ldcg(base + (size_t)(j + G * r) * inner) : C{T(0), T(0)};
@@ -93,35 +96,36 @@ __global__ void __launch_bounds__((PencilG<T, L>::TH))
 }
 
 template <typename T, int L>
-static cudaError_t launch_step_pencil_t(const PencilWork<T>* d_works, int nworks, int inner, bool compact,
+static cudaError_t launch_step_pencil_t(const PencilWork<T>* d_works, int nworks, int inner, bool compact, bool early,
                                         const c2_t<T>* tw, cudaStream_t st) {
   using P = PencilG<T, L>;
-  return launch_sweep_kernel(step_pencil_kernel<T, L>, dim3((inner + P::TK - 1) / P::TK, nworks), dim3(P::TH), 0, st,
-                             d_works, inner, compact ? 1 : 0, tw);
+  return launch_sweep_kernel(early ? step_pencil_kernel<T, L, true> : step_pencil_kernel<T, L, false>,
+                             dim3((inner + P::TK - 1) / P::TK, nworks), dim3(P::TH), 0, st, d_works, inner,
+                             compact ? 1 : 0, tw);
 }
 
 template <typename T>
-cudaError_t launch_step_pencil(const PencilWork<T>* w, int nw, int L, int inner, bool compact, const c2_t<T>* tw,
-                               cudaStream_t st) {
+cudaError_t launch_step_pencil(const PencilWork<T>* w, int nw, int L, int inner, bool compact, bool early,
+                               const c2_t<T>* tw, cudaStream_t st) {
   switch (L) {
-    case 1: return launch_step_pencil_t<T, 1>(w, nw, inner, compact, tw, st);
-    case 4: return launch_step_pencil_t<T, 4>(w, nw, inner, compact, tw, st);
-    case 8: return launch_step_pencil_t<T, 8>(w, nw, inner, compact, tw, st);
-    case 12: return launch_step_pencil_t<T, 12>(w, nw, inner, compact, tw, st);
-    case 16: return launch_step_pencil_t<T, 16>(w, nw, inner, compact, tw, st);
-    case 24: return launch_step_pencil_t<T, 24>(w, nw, inner, compact, tw, st);
-    case 32: return launch_step_pencil_t<T, 32>(w, nw, inner, compact, tw, st);
-    case 48: return launch_step_pencil_t<T, 48>(w, nw, inner, compact, tw, st);
-    case 64: return launch_step_pencil_t<T, 64>(w, nw, inner, compact, tw, st);
-    case 96: return launch_step_pencil_t<T, 96>(w, nw, inner, compact, tw, st);
-    case 128: return launch_step_pencil_t<T, 128>(w, nw, inner, compact, tw, st);
-    case 256: return launch_step_pencil_t<T, 256>(w, nw, inner, compact, tw, st);
+    case 1: return launch_step_pencil_t<T, 1>(w, nw, inner, compact, early, tw, st);
+    case 4: return launch_step_pencil_t<T, 4>(w, nw, inner, compact, early, tw, st);
+    case 8: return launch_step_pencil_t<T, 8>(w, nw, inner, compact, early, tw, st);
+    case 12: return launch_step_pencil_t<T, 12>(w, nw, inner, compact, early, tw, st);
+    case 16: return launch_step_pencil_t<T, 16>(w, nw, inner, compact, early, tw, st);
+    case 24: return launch_step_pencil_t<T, 24>(w, nw, inner, compact, early, tw, st);
+    case 32: return launch_step_pencil_t<T, 32>(w, nw, inner, compact, early, tw, st);
+    case 48: return launch_step_pencil_t<T, 48>(w, nw, inner, compact, early, tw, st);
+    case 64: return launch_step_pencil_t<T, 64>(w, nw, inner, compact, early, tw, st);
+    case 96: return launch_step_pencil_t<T, 96>(w, nw, inner, compact, early, tw, st);
+    case 128: return launch_step_pencil_t<T, 128>(w, nw, inner, compact, early, tw, st);
+    case 256: return launch_step_pencil_t<T, 256>(w, nw, inner, compact, early, tw, st);
   }
   return cudaErrorInvalidValue;
 }
-template cudaError_t launch_step_pencil<float>(const PencilWork<float>*, int, int, int, bool, const float2*,
+template cudaError_t launch_step_pencil<float>(const PencilWork<float>*, int, int, int, bool, bool, const float2*,
                                                cudaStream_t);
-template cudaError_t launch_step_pencil<double>(const PencilWork<double>*, int, int, int, bool, const double2*,
+template cudaError_t launch_step_pencil<double>(const PencilWork<double>*, int, int, int, bool, bool, const double2*,
                                                 cudaStream_t);
 
 }  // namespace psb

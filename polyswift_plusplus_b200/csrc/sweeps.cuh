@@ -86,11 +86,24 @@ inline bool split_path(const SweepSet<T>& s, int variant) {
   constexpr int both = VARIANT_FUSE_Z | VARIANT_FUSE_K;
   return (variant & both) == both && !(variant & VARIANT_CLUSTER) && step_split_supported(s.n[1], s.n[2]);
 }
+// The x pass may let the plane pass behind it start early (VARIANT_EARLY) on step-pass
+// grids whose plane CTAs leave room on an SM beside the x pass's.  Whether that pays
+// depends on where the CTAs land, so the engine times it.  An iteration of a diblock
+// of 100 steps, us, before and with the choice: 48^3 FP64 1011 -> 918, 64^3 FP64 1223 ->
+// 1165, 96^3 FP64 2558 -> 2493, 96 x 32 x 32 FP32 857 -> 779, 64 x 96 x 48 FP32 1175 ->
+// 1138.  Above the limit it mostly loses (forced: 128 x 96 x 96 FP64 3335 -> 3654, 128^3 FP64
+// 10210 -> 10820).
+template <typename T>
+inline bool early_path(const SweepSet<T>& s, int variant) {
+  return compact_path(s, variant) && (variant & VARIANT_FUSE_K) && !(variant & (VARIANT_XY | VARIANT_CLUSTER)) &&
+         !resident_path(s, variant) && sizeof(T) * s.n[0] * s.n[1] * s.n[2] <= sizeof(double) * 96 * 96 * 96;
+}
 template <typename T>
 inline cudaError_t launch_x_pass(const SweepSet<T>& s, const PencilWork<T>* w, int nw, bool compact, int variant,
                                  cudaStream_t st) {
   if (variant & VARIANT_FUSE_K)
-    return launch_step_pencil<T>(w, nw, s.n[0], s.n[1] * s.nzh, compact, s.tw_x, st);
+    return launch_step_pencil<T>(w, nw, s.n[0], s.n[1] * s.nzh, compact, compact && (variant & VARIANT_EARLY), s.tw_x,
+                                 st);
   return launch_pencil<T>(w, nw, compact ? PENCIL_KINVC : PENCIL_KINV, s.n[0], 1, s.n[1] * s.nzh, s.tw_x, s.n[0],
                           s.n[1], s.n[2], st);
 }

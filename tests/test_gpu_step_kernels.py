@@ -174,3 +174,24 @@ def test_one_launch_sweep_wait_timeout_is_reported(gpu, oracle_lib):
     assert ei.value.code == A.PS_GPU_ERR and "wait limit" in str(ei.value)
     s.close()
     test_one_launch_sweeps(gpu, (16, 16, 16), "fp64")
+
+
+@pytest.mark.parametrize("n,precision", [((64, 24, 24), "fp64"), ((48, 48, 48), "fp64"), ((96, 32, 64), "mixed")])
+def test_tuned_run_matches_forced_variant(gpu, n, precision):
+    """The tuned choice (variants timed as graphs, the plane pass perhaps started early) gives what
+    the same variant gives when forced, bit for bit: starting early changes no arithmetic."""
+    cfg, w = _case(n, precision)
+    tuned = ScftSolver(cfg)
+    tuned.restore(w)
+    tuned.update(4)
+    v, _ = tuned.variant()
+    forced = ScftSolver(cfg)
+    forced.restore(w)
+    forced.update(1)  # the iteration before tuning
+    forced.set_variant(v)
+    forced.update(3)
+    for i in range(len(cfg.fields)):
+        assert np.array_equal(tuned.w(i), forced.w(i)) and np.array_equal(tuned.phi(i), forced.phi(i))
+    assert tuned.scalars()["free_energy"] == forced.scalars()["free_energy"]
+    tuned.close()
+    forced.close()
