@@ -20,7 +20,7 @@ template <int N>
 static cudaError_t launch_adj_plane(const PlaneWork<double>* w, int nw, int nx, const double2* ty, const double2* tz,
                                     const AdjArgs& adj, cudaStream_t st) {
   using P = StepPlane<double, N, N>;
-  auto kern = step_plane_kernel<double, N, N, true>;
+  auto kern = step_plane_kernel<double, N, N, true, false>;
   static unsigned attr_mask = 0;
   cudaError_t e = ensure_smem_attr(kern, P::SMEM, &attr_mask);
   if (e != cudaSuccess) return e;

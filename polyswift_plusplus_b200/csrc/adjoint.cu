@@ -497,7 +497,7 @@ struct Builder {
     ps_handle* H = h;
     const int nx_ = nx, ny_ = ny, nz_ = nz;
     ops.push_back([=](cudaStream_t st) {
-      return launch_step_plane<double>(A->d_pw + p0, n, nx_, ny_, nz_, H->bd.tw_y, H->bd.tw_z, st);
+      return launch_step_plane<double>(A->d_pw + p0, n, nx_, ny_, nz_, false, H->bd.tw_y, H->bd.tw_z, st);
     });
   }
   // Fused adjoint steps: the plane pass of lambda works in adjoint modes (with their

@@ -680,7 +680,8 @@ static int launch_post(ps_handle* h, long long* nlaunch) {
   return PS_OK;
 }
 
-// One variant's sweeps as a graph: the faster of two replays after a first one.
+// One variant's sweeps as a graph: the median of three replays after a first one (CTAs
+// placed early do not always land alike).
 template <typename T>
 static int time_as_graph(ps_handle* h, int v, cudaEvent_t a, cudaEvent_t b, float* ms) {
   long long nl = 0;
@@ -690,16 +691,16 @@ static int time_as_graph(ps_handle* h, int v, cudaEvent_t a, cudaEvent_t b, floa
   int rc = launch_sweeps<T>(h, &nl, v);
   cudaError_t e = cudaStreamEndCapture(h->st, &g);
   if (rc == PS_OK && e == cudaSuccess) e = cudaGraphInstantiate(&x, g, 0);
-  *ms = 1e30f;
-  for (int i = 0; i < 3 && rc == PS_OK && e == cudaSuccess; ++i) {
+  float t[4] = {1e30f, 1e30f, 1e30f, 1e30f};
+  for (int i = 0; i < 4 && rc == PS_OK && e == cudaSuccess; ++i) {
     e = cudaEventRecord(a, h->st);
     if (e == cudaSuccess) e = cudaGraphLaunch(x, h->st);
     if (e == cudaSuccess) e = cudaEventRecord(b, h->st);
     if (e == cudaSuccess) e = cudaEventSynchronize(b);
-    float t = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&t, a, b);
-    if (i > 0) *ms = std::min(*ms, t);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&t[i], a, b);
   }
+  std::sort(t + 1, t + 4);
+  *ms = t[2];
   if (x) cudaGraphExecDestroy(x);
   if (g) cudaGraphDestroy(g);
   if (rc) return rc;
@@ -749,16 +750,19 @@ static int autotune_t(ps_handle* h) {
       if (early_path(set, v) && h->tune_ms[v] >= 0.f && (t < 0 || h->tune_ms[v] < h->tune_ms[t])) t = v;
     }
     float least = 1e30f;
-    for (int i = 0; i < 4 && rc == PS_OK && e == cudaSuccess; ++i) {
-      if (top[i / 2] < 0) continue;
+    const int early[3] = {0, VARIANT_EARLY, VARIANT_EARLY | VARIANT_EARLY_PLANE};
+    const int ne = early_plane_path(set, best_v) ? 3 : 2;
+    for (int i = 0; i < 2 * ne && rc == PS_OK && e == cudaSuccess; ++i) {
+      const int v = top[i / ne], how = early[i % ne];
+      if (v < 0) continue;
       float ms = 0.f;
-      rc = time_as_graph<T>(h, top[i / 2] | (i % 2 ? VARIANT_EARLY : 0), a, b, &ms);
+      rc = time_as_graph<T>(h, v | how, a, b, &ms);
       if (rc) break;
-      if (i % 2 == 0 || ms < h->tune_ms[top[i / 2]]) h->tune_ms[top[i / 2]] = ms;
+      if (how == 0 || ms < h->tune_ms[v]) h->tune_ms[v] = ms;
       if (ms < least) {
         least = ms;
-        best_v = top[i / 2];
-        h->early = (i % 2) ? VARIANT_EARLY : 0;
+        best_v = v;
+        h->early = how;
       }
     }
   }

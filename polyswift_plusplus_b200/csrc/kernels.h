@@ -126,7 +126,9 @@ enum {
   VARIANT_SPLIT = 8,
   VARIANT_CLUSTER = 16,
   VARIANT_COUNT = 32,
-  VARIANT_EARLY = 32  // beside a variant, chosen by the autotuner alone: see early_path in sweeps.cuh
+  // beside a variant, chosen by the autotuner alone: see early_path in sweeps.cuh
+  VARIANT_EARLY = 32,
+  VARIANT_EARLY_PLANE = 64
 };
 bool cluster_plane_supported(int prec_bytes, int ny, int nz);
 // The cluster plane pass (ny = nz = 256): grid 8 nx x nworks, eight CTAs per
@@ -163,7 +165,7 @@ cudaError_t launch_rows(const PlaneWork<T>* d_works, int nworks, int nrows, int 
 // (step_plane.cuh), and the x pass in registers (step_pencil.cu).
 bool step_plane_supported(int ny, int nz);
 template <typename T>
-cudaError_t launch_step_plane(const PlaneWork<T>* d_works, int nworks, int nx, int ny, int nz,
+cudaError_t launch_step_plane(const PlaneWork<T>* d_works, int nworks, int nx, int ny, int nz, bool early,
                               const c2_t<T>* tw_y, const c2_t<T>* tw_z, cudaStream_t st);
 template <typename T>
 cudaError_t launch_step_pencil(const PencilWork<T>* d_works, int nworks, int L, int inner, bool compact, bool early,

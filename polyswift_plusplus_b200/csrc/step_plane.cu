@@ -23,22 +23,22 @@ bool step_plane_supported(int ny, int nz) {
 }
 
 template <typename T>
-cudaError_t launch_step_plane(const PlaneWork<T>* w, int nw, int nx, int ny, int nz, const c2_t<T>* ty,
-                              const c2_t<T>* tz, cudaStream_t st) {
+cudaError_t launch_step_plane(const PlaneWork<T>* w, int nw, int nx, int ny, int nz, bool early,
+                              const c2_t<T>* ty, const c2_t<T>* tz, cudaStream_t st) {
   switch (ny) {
-    case 16: return launch_step_plane_ny<T, 16>(w, nw, nx, nz, ty, tz, st);
-    case 24: return launch_step_plane_ny<T, 24>(w, nw, nx, nz, ty, tz, st);
-    case 32: return launch_step_plane_ny<T, 32>(w, nw, nx, nz, ty, tz, st);
-    case 48: return launch_step_plane_ny<T, 48>(w, nw, nx, nz, ty, tz, st);
-    case 64: return launch_step_plane_ny<T, 64>(w, nw, nx, nz, ty, tz, st);
-    case 96: return launch_step_plane_ny<T, 96>(w, nw, nx, nz, ty, tz, st);
-    case 128: return launch_step_plane_ny<T, 128>(w, nw, nx, nz, ty, tz, st);
+    case 16: return launch_step_plane_ny<T, 16>(w, nw, nx, nz, early, ty, tz, st);
+    case 24: return launch_step_plane_ny<T, 24>(w, nw, nx, nz, early, ty, tz, st);
+    case 32: return launch_step_plane_ny<T, 32>(w, nw, nx, nz, early, ty, tz, st);
+    case 48: return launch_step_plane_ny<T, 48>(w, nw, nx, nz, early, ty, tz, st);
+    case 64: return launch_step_plane_ny<T, 64>(w, nw, nx, nz, early, ty, tz, st);
+    case 96: return launch_step_plane_ny<T, 96>(w, nw, nx, nz, early, ty, tz, st);
+    case 128: return launch_step_plane_ny<T, 128>(w, nw, nx, nz, early, ty, tz, st);
   }
   return cudaErrorInvalidValue;
 }
-template cudaError_t launch_step_plane<float>(const PlaneWork<float>*, int, int, int, int, const float2*,
+template cudaError_t launch_step_plane<float>(const PlaneWork<float>*, int, int, int, int, bool, const float2*,
                                               const float2*, cudaStream_t);
-template cudaError_t launch_step_plane<double>(const PlaneWork<double>*, int, int, int, int, const double2*,
+template cudaError_t launch_step_plane<double>(const PlaneWork<double>*, int, int, int, int, bool, const double2*,
                                                const double2*, cudaStream_t);
 
 }  // namespace psb

@@ -80,6 +80,7 @@ template <typename T, int NY, int NZ> struct StepPlane {
   static constexpr int BY_SMEM = (int)((size_t)224 * 1024 / (SMEM + 1024));
   static constexpr int MINB0 = BY_REG < BY_SMEM ? BY_REG : BY_SMEM;
   static constexpr int MINB = MINB0 < 1 ? 1 : (MINB0 > 16 ? 16 : MINB0);
+  static constexpr bool CAN_EARLY = sizeof(T) == 4 && NY >= 96 && NZ >= 96;
   static_assert(TH % 32 == 0 && TH <= 1024 && TASKS % 32 == 0 && UZ <= 2, "step plane layout");
   static_assert(NG == 1 || ((CG * GY) % 32 == 0 && NG <= 15), "step plane groups");
   static_assert(S >= NZ && RY * GY == NY && RZ * GZ == NZ && GY % 2 == 0, "step plane layout");
@@ -212,7 +213,9 @@ template <int U, int M> struct AdjRuns {
 };
 
 // ADJ (FP64): works in the adjoint modes of adjoint.cuh beside FIRST ones.
-template <typename T, int NY, int NZ, bool ADJ>
+// EARLY: the x pass behind it may be placed before this pass has ended (early_path in
+// sweeps.cuh).
+template <typename T, int NY, int NZ, bool ADJ, bool EARLY>
 __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (ADJ ? 1 : StepPlane<T, NY, NZ>::MINB))
     step_plane_kernel(const PlaneWork<T>* __restrict__ works, const c2_t<T>* __restrict__ tw_y,
                       const c2_t<T>* __restrict__ tw_z, AdjArgs adj) {
@@ -296,6 +299,7 @@ __global__ void __launch_bounds__((StepPlane<T, NY, NZ>::TH), (ADJ ? 1 : StepPla
     __syncthreads();  // every row complete
   }
 
+  if constexpr (EARLY) pdl_trigger();
   // z rows: inverse, real-space step, forward
   T acc = T(0);
   const AdjPoint* const point = ADJ ? adj.points + blockIdx.y : nullptr;
@@ -533,10 +537,19 @@ RealRun<T, UZ> xs[2 * CH];  // the rows' values at the chunk's positions
 }
 
 template <typename T, int NY, int NZ>
-cudaError_t launch_step_plane_t(const PlaneWork<T>* d_works, int nworks, int nx, const c2_t<T>* tw_y,
+cudaError_t launch_step_plane_t(const PlaneWork<T>* d_works, int nworks, int nx, bool early, const c2_t<T>* tw_y,
                                 const c2_t<T>* tw_z, cudaStream_t st) {
   using P = StepPlane<T, NY, NZ>;
-  auto kern = step_plane_kernel<T, NY, NZ, false>;
+  if constexpr (P::CAN_EARLY) {
+    if (early) {
+      auto kern = step_plane_kernel<T, NY, NZ, false, true>;
+      static unsigned attr_mask = 0;
+      cudaError_t e = ensure_smem_attr(kern, P::SMEM, &attr_mask);
+      if (e != cudaSuccess) return e;
+      return launch_sweep_kernel(kern, dim3(nx, nworks), dim3(P::TH), P::SMEM, st, d_works, tw_y, tw_z, AdjArgs{});
+    }
+  }
+  auto kern = step_plane_kernel<T, NY, NZ, false, false>;
   static unsigned attr_mask = 0;
   cudaError_t e = ensure_smem_attr(kern, P::SMEM, &attr_mask);
   if (e != cudaSuccess) return e;
@@ -545,23 +558,23 @@ cudaError_t launch_step_plane_t(const PlaneWork<T>* d_works, int nworks, int nx,
 
 // Planes of NY rows, for every nz of kStepExtents (one translation unit per NY).
 template <typename T, int NY>
-cudaError_t launch_step_plane_ny(const PlaneWork<T>* w, int nw, int nx, int nz, const c2_t<T>* ty, const c2_t<T>* tz,
-                                 cudaStream_t st) {
+cudaError_t launch_step_plane_ny(const PlaneWork<T>* w, int nw, int nx, int nz, bool early, const c2_t<T>* ty,
+                                 const c2_t<T>* tz, cudaStream_t st) {
   switch (nz) {
-    case 16: return launch_step_plane_t<T, NY, 16>(w, nw, nx, ty, tz, st);
-    case 24: return launch_step_plane_t<T, NY, 24>(w, nw, nx, ty, tz, st);
-    case 32: return launch_step_plane_t<T, NY, 32>(w, nw, nx, ty, tz, st);
-    case 48: return launch_step_plane_t<T, NY, 48>(w, nw, nx, ty, tz, st);
-    case 64: return launch_step_plane_t<T, NY, 64>(w, nw, nx, ty, tz, st);
-    case 96: return launch_step_plane_t<T, NY, 96>(w, nw, nx, ty, tz, st);
-    case 128: return launch_step_plane_t<T, NY, 128>(w, nw, nx, ty, tz, st);
+    case 16: return launch_step_plane_t<T, NY, 16>(w, nw, nx, early, ty, tz, st);
+    case 24: return launch_step_plane_t<T, NY, 24>(w, nw, nx, early, ty, tz, st);
+    case 32: return launch_step_plane_t<T, NY, 32>(w, nw, nx, early, ty, tz, st);
+    case 48: return launch_step_plane_t<T, NY, 48>(w, nw, nx, early, ty, tz, st);
+    case 64: return launch_step_plane_t<T, NY, 64>(w, nw, nx, early, ty, tz, st);
+    case 96: return launch_step_plane_t<T, NY, 96>(w, nw, nx, early, ty, tz, st);
+    case 128: return launch_step_plane_t<T, NY, 128>(w, nw, nx, early, ty, tz, st);
   }
   return cudaErrorInvalidValue;
 }
 #define PSB_STEP_PLANE_NY(PREFIX, NY)                                                                             \
-  PREFIX template cudaError_t launch_step_plane_ny<float, NY>(const PlaneWork<float>*, int, int, int,             \
+  PREFIX template cudaError_t launch_step_plane_ny<float, NY>(const PlaneWork<float>*, int, int, int, bool,       \
                                                               const float2*, const float2*, cudaStream_t);        \
-  PREFIX template cudaError_t launch_step_plane_ny<double, NY>(const PlaneWork<double>*, int, int, int,           \
+  PREFIX template cudaError_t launch_step_plane_ny<double, NY>(const PlaneWork<double>*, int, int, int, bool,     \
                                                                const double2*, const double2*, cudaStream_t);
 
 }  // namespace psb

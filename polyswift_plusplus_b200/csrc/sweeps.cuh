@@ -86,17 +86,24 @@ inline bool split_path(const SweepSet<T>& s, int variant) {
   constexpr int both = VARIANT_FUSE_Z | VARIANT_FUSE_K;
   return (variant & both) == both && !(variant & VARIANT_CLUSTER) && step_split_supported(s.n[1], s.n[2]);
 }
-// The x pass may let the plane pass behind it start early (VARIANT_EARLY) on step-pass
-// grids whose plane CTAs leave room on an SM beside the x pass's.  Whether that pays
-// depends on where the CTAs land, so the engine times it.  An iteration of a diblock
-// of 100 steps, us, before and with the choice: 48^3 FP64 1011 -> 918, 64^3 FP64 1223 ->
-// 1165, 96^3 FP64 2558 -> 2493, 96 x 32 x 32 FP32 857 -> 779, 64 x 96 x 48 FP32 1175 ->
-// 1138.  Above the limit it mostly loses (forced: 128 x 96 x 96 FP64 3335 -> 3654, 128^3 FP64
-// 10210 -> 10820).
+// The x pass may let the plane pass behind it be placed early (VARIANT_EARLY), where the
+// plane's CTAs leave room on an SM beside the x pass's, and the plane pass the x pass
+// behind it (VARIANT_EARLY_PLANE).  Whether that pays depends on where the CTAs land, so
+// the engine times it.  An iteration of a diblock of 100 steps, us, before and with the
+// choice: 48^3 FP64 1011 -> 918, 64^3 FP64 1223 -> 1165, 96^3 FP64 2558 -> 2493,
+// 96 x 32 x 32 FP32 857 -> 779, 64 x 96 x 48 FP32 1175 -> 1138, 128^3 FP32 2990 -> 2803.
+// Above the limit it mostly loses (forced: 128 x 96 x 96 FP64 3335 -> 3654, 128^3 FP64
+// 10210 -> 10820 for 200 steps).
 template <typename T>
 inline bool early_path(const SweepSet<T>& s, int variant) {
   return compact_path(s, variant) && (variant & VARIANT_FUSE_K) && !(variant & (VARIANT_XY | VARIANT_CLUSTER)) &&
-         !resident_path(s, variant) && sizeof(T) * s.n[0] * s.n[1] * s.n[2] <= sizeof(double) * 96 * 96 * 96;
+         !resident_path(s, variant) &&
+         (sizeof(T) * s.n[0] * s.n[1] * s.n[2] <= sizeof(double) * 96 * 96 * 96 ||
+          (sizeof(T) == 4 && s.n[1] * s.n[2] >= 128 * 128));
+}
+template <typename T>
+inline bool early_plane_path(const SweepSet<T>& s, int variant) {
+  return early_path(s, variant) && sizeof(T) == 4 && s.n[1] >= 96 && s.n[2] >= 96;  // StepPlane::CAN_EARLY
 }
 template <typename T>
 inline cudaError_t launch_x_pass(const SweepSet<T>& s, const PencilWork<T>* w, int nw, bool compact, int variant,
@@ -144,7 +151,7 @@ cudaError_t launch_sweep_set(const SweepSet<T>& s, int variant, cudaStream_t st,
       PSB_L(launch_split_plane<T>(pw, np, nx, s.tw_y, s.tw_z, st));
       if (nxw > 0) PSB_L(launch_split_pencil<T>(xw, nxw, nx, nz, s.tw_x, st));
     } else if (compact_path(s, variant)) {
-      PSB_L(launch_step_plane<T>(pw, np, nx, ny, nz, s.tw_y, s.tw_z, st));
+      PSB_L(launch_step_plane<T>(pw, np, nx, ny, nz, (variant & VARIANT_EARLY_PLANE) != 0, s.tw_y, s.tw_z, st));
       if (nxw > 0) PSB_L(launch_x_pass<T>(s, xw, nxw, true, variant, st));
     } else if (s.fused_plane) {
       PSB_L(launch_plane<T>(pw, np, nx, ny, nz, s.tw_y, s.tw_zh, s.tw_z, st));

@@ -195,3 +195,9 @@ def test_tuned_run_matches_forced_variant(gpu, n, precision):
     assert tuned.scalars()["free_energy"] == forced.scalars()["free_energy"]
     tuned.close()
     forced.close()
+
+
+@pytest.mark.parametrize("n", [(16, 128, 128), (24, 96, 96), (12, 96, 128)])
+def test_tuned_run_with_early_plane_pass(gpu, n):
+    """The same for the planes whose pass has an early form."""
+    test_tuned_run_matches_forced_variant(gpu, n, "mixed")
