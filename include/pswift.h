@@ -457,11 +457,12 @@ void* ps_adj_stream(const ps_adj* a);
 const char* ps_adj_last_error(const ps_adj* a);
 
 /* --- Fault injection for the bounded waits --------------------------------
- * No counterpart in the reference.  Every wait of a kernel on a bulk copy is
- * bounded; when a plane pass's wait runs out, the pass sets error bit 2 of the
- * handle's status word, drains the copy still in flight (full bound) and
- * returns, and the handle reports PS_GPU_ERR with the context still usable.
- * This sets the poll limit of that first wait on the current device (default
+ * No counterpart in the reference.  Every wait of a kernel on a bulk copy or
+ * on another CTA of its cluster is bounded; when a wait runs out, the kernel
+ * sets error bit 2 of the handle's status word, gives what is still in flight
+ * time to land (full bound) and returns, and the handle reports PS_GPU_ERR with
+ * the context still usable.  This sets the poll limit of a plane pass's first
+ * wait and of the one-launch sweeps' exchanges on the current device (default
  * 2^22 polls; 0 gives up at once, 0xFFFFFFFF restores the default), so a test
  * can drive the timeout path without a fault.  Not for production runs. */
 int ps_gpu_set_bulk_wait_limit(unsigned int polls);

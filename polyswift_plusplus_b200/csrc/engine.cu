@@ -718,19 +718,24 @@ static int autotune_t(ps_handle* h) {
   float best = 1e30f;
   int best_v = 0;
   int rc = PS_OK;
-  for (int v = 0; v < VARIANT_COUNT && e == cudaSuccess && rc == PS_OK; ++v) {
+  // the usual winners first: a variant whose first pass (with the loading of its kernels)
+  // is far behind is not run again
+  for (int i = 0; i < VARIANT_COUNT && e == cudaSuccess && rc == PS_OK; ++i) {
+    const int v = i ^ (VARIANT_FUSE_Z | VARIANT_FUSE_K);
     h->tune_ms[v] = -1.f;
     if ((v & VARIANT_XY) && (!h->xy_ok || (v & VARIANT_FUSE_Z))) continue;  // absent / same
     if ((v & VARIANT_CLUSTER) && (!h->cluster_ok || (v & VARIANT_XY))) continue;
     if ((v & VARIANT_SPLIT) && h->sw_st.empty()) continue;                 // one sweep only
-    long long nl = 0;
-    rc = launch_sweeps<T>(h, &nl, v);  // warm-up
-    if (rc == PS_OK) e = cudaEventRecord(a, h->st);
-    if (rc == PS_OK && e == cudaSuccess) rc = launch_sweeps<T>(h, &nl, v);
-    if (rc == PS_OK && e == cudaSuccess) e = cudaEventRecord(b, h->st);
-    if (rc == PS_OK && e == cudaSuccess) e = cudaEventSynchronize(b);
     float ms = 0.f;
-    if (rc == PS_OK && e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
+    for (int pass = 0; pass < 2 && rc == PS_OK && e == cudaSuccess; ++pass) {
+      if (pass == 1 && ms > 1.25f * best + 0.5f) break;
+      long long nl = 0;
+      e = cudaEventRecord(a, h->st);
+      if (e == cudaSuccess) rc = launch_sweeps<T>(h, &nl, v);
+      if (rc == PS_OK && e == cudaSuccess) e = cudaEventRecord(b, h->st);
+      if (rc == PS_OK && e == cudaSuccess) e = cudaEventSynchronize(b);
+      if (rc == PS_OK && e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
+    }
     if (rc != PS_OK || e != cudaSuccess) break;
     h->tune_ms[v] = ms;
     if (ms < best) {
@@ -752,9 +757,10 @@ static int autotune_t(ps_handle* h) {
     float least = 1e30f;
     const int early[3] = {0, VARIANT_EARLY, VARIANT_EARLY | VARIANT_EARLY_PLANE};
     const int ne = early_plane_path(set, best_v) ? 3 : 2;
+    // first neither early, then the early starts of a variant that is not far behind
     for (int i = 0; i < 2 * ne && rc == PS_OK && e == cudaSuccess; ++i) {
-      const int v = top[i / ne], how = early[i % ne];
-      if (v < 0) continue;
+      const int v = top[i % 2], how = early[i / 2];
+      if (v < 0 || (how && h->tune_ms[v] > 1.08f * least)) continue;
       float ms = 0.f;
       rc = time_as_graph<T>(h, v | how, a, b, &ms);
       if (rc) break;

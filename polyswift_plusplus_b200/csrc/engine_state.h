@@ -162,7 +162,7 @@ struct ps_handle {
   int early = 0;     // VARIANT_EARLY where the autotuner found it faster
   float tune_ms[psb::VARIANT_COUNT] = {};
   bool xy_ok = false;  // the row + x-y plane design exists for this grid
-  bool cluster_ok = false;  // the two-CTA cluster plane pass exists for this grid and precision
+  bool cluster_ok = false;  // the cluster plane pass (bit 4) exists for this grid and precision
   bool in_batch = false;  // owned by a ps_batch, whose merged work tables point into it
   bool branched = false;  // a branched polymer: its sweeps run as dependent launch chains only
   int n_jbuf = 0;

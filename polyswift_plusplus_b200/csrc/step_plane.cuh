@@ -26,9 +26,10 @@
 //
 // Both sweeps of a diblock, one propagator step each, with the x pass of
 // step_pencil.cu (B200, us; the fastest earlier variant first): 128^3 FP32 30.6 ->
-// 25.1, FP64 59.0 -> 46.2; 96^3 27.0 -> 15.5, 34.6 -> 22.8; 64^3 12.0 -> 8.3, 14.1 ->
-// 10.1; 48^3 11.7 -> 7.3, 11.9 -> 8.3; 32^3 6.5 -> 5.0, 6.7 -> 5.5.  64 x 96 x 48 (a
-// blend, three sweeps; it had a row pass and two y pencil passes): 28 -> 13.
+// 23.8, FP64 59.0 -> 44.4; 96^3 27.0 -> 14.2, 34.6 -> 20.9; 64^3 12.0 -> 7.2, 14.1 ->
+// 9.2; 48^3 11.7 -> 5.5, 11.9 -> 7.2; 32^3 6.5 -> 4.5, 6.7 -> 4.6; less with early starts
+// (early_path in sweeps.cuh).  64 x 96 x 48 (a blend, three sweeps; it had a row pass
+// and two y pencil passes): 28 -> 10.
 // What bounds it now: at 128^2 the shared-memory and L1 data path (66% busy, 13.4 k
 // wavefronts a plane) with one wave of CTAs that load, compute and store at the
 // same time; at 64^2 and below the latency of one plane's chain.
