@@ -662,7 +662,7 @@ def run_ours(args, world, rank, local):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": (achieved / peak) if achieved else None,
                 "traffic": profile_traffic(grid, args.precision),
-                "kernel": "propagator step (plane_kernel + pencil_kernel per step of every sweep)",
+                "kernel": "propagator step (step_plane_kernel + step_pencil_kernel per step of every sweep)",
                 "peak_source": f"{peak_kind} hbm_gbs (burst copy)",
                 "algorithmic_bytes_per_step": 3 * N * (4 if args.precision == "mixed" else 8),
                 "step_us": per_step_ms * 1000.0, "samples": len(sweep_ms)}
