@@ -3,22 +3,6 @@
 
 namespace psb {
 
-// (nx, ny, nz, CTAs of the cluster), a film nx x ny x 1 as (nx, 1, ny).  One plane
-// or a few rows per CTA, as many CTAs as a cluster may have: us per step of both
-// sweeps, FP64 (FP32), against the step passes' two launches:
-//   8^3 1.3 (1.4), 12^3 1.7 (1.6)      passes 5.6 and 6.3 (7.0)
-//   16^3 1.8, eight CTAs 1.9           passes 4.6
-//   24^3 3.7 (2.8), eight CTAs 4.6 (3.3), passes 5.7
-//   32^3 4.6 (3.2), passes 5.5 (5.0)
-//   films, eight rows a CTA: 24^2 1.6 (1.5), passes 10 (12); 48^2 2.1 (1.9), 11 (13);
-//   64^2 2.3, 4.9; 96^2 3.5 (2.6), 16 (19); 128^2 3.9, eight CTAs 4.5, passes 6.4
-// 48^3 has too much work for 16 SMs per sweep: FP32 9.0 against 7.3.
-#define PSB_SWEEP_GRIDS(X)                                        \
-  X(8, 8, 8, 8) X(12, 12, 12, 12) X(16, 16, 16, 16)               \
-  X(24, 24, 24, 12) X(32, 32, 32, 16) X(16, 1, 16, 2)             \
-  X(24, 1, 24, 3) X(32, 1, 32, 4) X(48, 1, 48, 6)                 \
-  X(64, 1, 64, 8) X(96, 1, 96, 12) X(128, 1, 128, 16)
-
 bool sweep_cluster_supported(int nx, int ny, int nz) {
   const int f = (nz == 1);
 #define PSB_X(NX, NY, NZ, CL) \

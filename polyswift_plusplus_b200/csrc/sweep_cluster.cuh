@@ -91,7 +91,15 @@ template <typename T, int NX, int NY, int NZ, int CL_> struct SweepCl {
   static constexpr int S0 = GZ * PA;
   static constexpr int S = (sizeof(T) == 4) ? S0 + ((24 - S0 % 16) % 16) : S0;
   static constexpr int NCOL = NY * (H + 1);
-  static constexpr int COLS = (NCOL + CL - 1) / CL;     // columns of a CTA (the last may have fewer)
+  // CTA m owns the columns from col0(m) to col0(m + 1), the last one also what is left
+  // over (a film's Nyquist column), and none owns nothing: what a CTA sends from its
+  // columns is what keeps the others from running into the next step while it is still
+  // in this one (see bar_a and bar_b below).
+  static constexpr int EACH = NCOL / CL, COLS = NCOL - EACH * (CL - 1);  // COLS: at most
+  static constexpr __host__ __device__ int col0(int m) { return m < CL ? m * EACH : NCOL; }
+  static constexpr __host__ __device__ int owner(int col) {
+    return (COLS == EACH || col < EACH * CL) ? col / EACH : CL - 1;
+  }
   // threads of a plane's z rows and of a plane: whole warps.  At nz < 16 the last
   // warp has lanes without a row (they take PRB - PR spare rows of the buffer along)
   // or without a column.
@@ -108,7 +116,25 @@ template <typename T, int NX, int NY, int NZ, int CL_> struct SweepCl {
   static_assert(PX * CL == NX && TH <= 1024 && PRB * GZ == ROWT && (!FILM || PRB == PR), "cluster sweep layout");
   static_assert(S >= NZ && RZ * GZ == NZ && RX * GX == NX && (FILM || RY * GY == NY) && UZ <= 2, "cluster sweep layout");
   static_assert(NP <= 15 && (!FILM || PX % 2 == 0) && CL * 2 <= TH, "cluster sweep layout");
+  static_assert(EACH >= 1 && COLS <= EACH + 1, "every CTA owns columns, as many as the others or one more");
 };
+
+// The grids that have one, as
+// (nx, ny, nz, CTAs of the cluster), a film nx x ny x 1 as (nx, 1, ny).  One plane
+// or a few rows per CTA, as many CTAs as a cluster may have: us per step of both
+// sweeps, FP64 (FP32), against the step passes' two launches:
+//   8^3 1.3 (1.4), 12^3 1.7 (1.6)      passes 5.6 and 6.3 (7.0)
+//   16^3 1.8, eight CTAs 1.9           passes 4.6
+//   24^3 3.7 (2.8), eight CTAs 4.6 (3.3), passes 5.7
+//   32^3 4.6 (3.2), passes 5.5 (5.0)
+//   films, eight rows a CTA: 24^2 1.6 (1.5), passes 10 (12); 48^2 2.1 (1.9), 11 (13);
+//   64^2 2.3, 4.9; 96^2 3.5 (2.6), 16 (19); 128^2 3.9, eight CTAs 4.5, passes 6.4
+// 48^3 has too much work for 16 SMs per sweep: FP32 9.0 against 7.3.
+#define PSB_SWEEP_GRIDS(X)                                        \
+  X(8, 8, 8, 8) X(12, 12, 12, 12) X(16, 16, 16, 16)               \
+  X(24, 24, 24, 12) X(32, 32, 32, 16) X(16, 1, 16, 2)             \
+  X(24, 1, 24, 3) X(32, 1, 32, 4) X(48, 1, 48, 6)                 \
+  X(64, 1, 64, 8) X(96, 1, 96, 12) X(128, 1, 128, 16)
 
 // Poll limit of the waits below (see ps_gpu_set_bulk_wait_limit).
 static __constant__ uint32_t c_sweep_wait_polls = kMaxPolls;
@@ -168,9 +194,10 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
   constexpr size_t RB = (size_t)PR * NZ;
   // x part: column cc of this CTA, butterfly jx
   const int cc = tid % COLS, jx = tid / COLS;
-  const int gcols0 = (int)me * COLS;
+  const int gcols0 = P::col0((int)me);
+  const int my_cols = P::col0((int)me + 1) - gcols0;
   const int gc = gcols0 + cc;
-  const bool in_col = jx < GX && gc < NCOL;
+  const bool in_col = jx < GX && cc < my_cols;
 
   int seg = 0, seg_end = w.seg[0].end;
   T* const slices = w.slices;
@@ -193,10 +220,11 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
     }
   };
   double dc_err = 0.0;
-  // A phase of bar_a or bar_b completes when this thread has armed it and every
-  // byte has arrived.  Phases cannot overlap: a CTA's part of the next one is sent
-  // only after the data that completes this one.
-  const uint32_t my_cols = (uint32_t)(gcols0 >= NCOL ? 0 : (NCOL - gcols0 < COLS ? NCOL - gcols0 : COLS));
+  // A phase of bar_a or bar_b completes when thread 0 has armed it and every byte has
+  // arrived.  Phases cannot overlap: a CTA sends its part of bar_b's next phase after its
+  // bar_a has the columns of every CTA, which each sends after its own bar_b phase (and
+  // after its warps have read s_part); and its part of bar_a's next phase after its bar_b
+  // has rows of every CTA, which each sends after its own bar_a phase.
   const uint32_t bytes_a = (uint32_t)(P::AIN * sizeof(C));
   const uint32_t bytes_b = (uint32_t)(NX * my_cols * sizeof(C)) + (dc ? (uint32_t)(CL * W * sizeof(double)) : 0u);
   if (tid == 0) {
@@ -207,12 +235,11 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
     mbar_arrive_expect_tx(bar_b, bytes_b);
   }
   // A wait that runs out sets the error flag; this thread then waits no more, and
-  // every CTA still comes to the end.  (A CTA without columns and without a carry
-  // has nothing to wait for on bar_b: its empty phases would run ahead.)
+  // every CTA still comes to the end.
   const uint32_t polls = c_sweep_wait_polls;
   bool failed = false;
   auto wait = [&](uint64_t* bar, uint32_t phase, uint32_t bytes, bool rearm) {
-    if (failed || bytes == 0) return;
+    if (failed) return;
     if (!cl_wait(bar, phase & 1u, polls)) {
       failed = true;
       if (w.status) atomicOr(w.status, 4);
@@ -466,15 +493,14 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
               const int ky = j + GY * r;
               const C d = ny[(NY - ky) % NY], a = v[r];
               v[r] = C{a.x + d.x, a.y - d.y};
-              const int col = NY * H + ky;
-              cl_store(cl_addr(b_in + x * COLS + col % COLS, col / COLS), cl_addr(bar_b, col / COLS),
-                       C{a.y + d.y, d.x - a.x});
+              const int col = NY * H + ky, to = P::owner(col);
+              cl_store(cl_addr(b_in + x * COLS + col - P::col0(to), to), cl_addr(bar_b, to), C{a.y + d.y, d.x - a.x});
             }
           }
 #pragma unroll
           for (int r = 0; r < RY; ++r) {
-            const int col = (j + GY * r) * H + c;
-            cl_store(cl_addr(b_in + x * COLS + col % COLS, col / COLS), cl_addr(bar_b, col / COLS), v[r]);
+            const int col = (j + GY * r) * H + c, to = P::owner(col);
+            cl_store(cl_addr(b_in + x * COLS + col - P::col0(to), to), cl_addr(bar_b, to), v[r]);
           }
         }
       }
@@ -483,8 +509,8 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
       for (int e = tid; e < PR * (H + 1); e += TH) {
         const int rb = e / (H + 1), kz = e - rb * (H + 1);
         const C z = buf[rb * S + kz], m = buf[rb * S + (kz == 0 || kz == H ? kz : NZ - kz)];
-        const uint32_t to = kz / COLS;
-        C* const at = b_in + (x0 + rb) * COLS + kz % COLS;
+        const int to = P::owner(kz);
+        C* const at = b_in + (x0 + rb) * COLS + kz - P::col0(to);
         const uint32_t bb = cl_addr(bar_b, to);
         cl_store(cl_addr(at, to), bb, C{z.x + m.x, z.y - m.y});
         cl_store(cl_addr(at + PR * COLS, to), bb, C{z.y + m.y, m.x - z.x});
