@@ -460,8 +460,9 @@ const char* ps_adj_last_error(const ps_adj* a);
  * No counterpart in the reference.  Every wait of a kernel on a bulk copy or
  * on another CTA of its cluster is bounded; when a wait runs out, the kernel
  * sets error bit 2 of the handle's status word, gives what is still in flight
- * time to land (full bound) and returns, and the handle reports PS_GPU_ERR with
- * the context still usable.  This sets the poll limit of a plane pass's first
+ * time to land (a bulk copy the full bound; the cluster exchange, whose CTAs
+ * stop sending, 200,000 cycles) and returns, and the handle reports PS_GPU_ERR
+ * with the context still usable.  This sets the poll limit of a plane pass's first
  * wait and of the one-launch sweeps' exchanges on the current device (default
  * 2^22 polls; 0 gives up at once, 0xFFFFFFFF restores the default), so a test
  * can drive the timeout path without a fault.  Not for production runs. */

@@ -53,6 +53,10 @@ __device__ __forceinline__ void cl_store(uint32_t addr, uint32_t bar, double v) 
                "r"(bar)
                : "memory");
 }
+// A plain store of 1; a cluster barrier makes it visible.
+__device__ __forceinline__ void cl_store_flag(uint32_t addr) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(1) : "memory");
+}
 // Bounded wait for a phase whose data other CTAs of the cluster wrote.
 __device__ __forceinline__ bool cl_wait(uint64_t* bar, uint32_t parity, uint32_t polls) {
   for (uint32_t i = 0; i < polls; ++i) {
@@ -112,10 +116,13 @@ template <typename T, int NX, int NY, int NZ, int CL_> struct SweepCl {
   static constexpr int BUF = NP * PRB * S, AIN = PX * NCOL, BIN = NX * COLS;
   static constexpr size_t SMEM =
       sizeof(c2_t<T>) * ((size_t)BUF + AIN + 2 * BIN + NP * NY + NX + NX / 2 + NY + NZ) +
-      sizeof(double) * (CL * (TH / 32) + 1) + 2 * sizeof(uint64_t);
+      sizeof(double) * (CL * (TH / 32) + 1) + 2 * sizeof(uint64_t) + sizeof(int);
   static_assert(PX * CL == NX && TH <= 1024 && PRB * GZ == ROWT && (!FILM || PRB == PR), "cluster sweep layout");
   static_assert(S >= NZ && RZ * GZ == NZ && RX * GX == NX && (FILM || RY * GY == NY) && UZ <= 2, "cluster sweep layout");
   static_assert(NP <= 15 && (!FILM || PX % 2 == 0) && CL * 2 <= TH, "cluster sweep layout");
+  // the bytes of two phases are within an mbarrier's transaction count
+  static_assert(2 * (sizeof(c2_t<T>) * (AIN > BIN ? AIN : BIN) + sizeof(double) * CL * (TH / 32)) < (1u << 20),
+                "cluster sweep phases");
   static_assert(EACH >= 1 && COLS <= EACH + 1, "every CTA owns columns, as many as the others or one more");
 };
 
@@ -166,6 +173,7 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
   double* s_mean = s_part + CL * W;                         // the mean-mode value of the inverse
   uint64_t* bar_a = reinterpret_cast<uint64_t*>(s_mean + 1);  // a_in written
   uint64_t* bar_b = bar_a + 1;                                // b_in (and s_part) written
+  int* s_stop = reinterpret_cast<int*>(bar_b + 1);            // a wait ran out in this cluster
 
   const SweepWork<T>& w = works[blockIdx.y];
   const int tid = threadIdx.x;
@@ -228,20 +236,25 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
   const uint32_t bytes_a = (uint32_t)(P::AIN * sizeof(C));
   const uint32_t bytes_b = (uint32_t)(NX * my_cols * sizeof(C)) + (dc ? (uint32_t)(CL * W * sizeof(double)) : 0u);
   if (tid == 0) {
+    *s_stop = 0;
     mbar_init(bar_a, 1);
     mbar_init(bar_b, 1);
     fence_mbar_init();
     mbar_arrive_expect_tx(bar_a, bytes_a);
     mbar_arrive_expect_tx(bar_b, bytes_b);
   }
-  // A wait that runs out sets the error flag; this thread then waits no more, and
-  // every CTA still comes to the end.
+  // A wait that runs out sets the error flag and stops its CTA before it sends anything
+  // from its columns.  The bar_a phases that lack them stay incomplete, so that the other
+  // CTAs' waits run out too: within a step nobody sends, and no barrier counts more than the
+  // bytes of two phases (were a CTA to go on for the rest of the sweep, 60 steps at 32^3
+  // would pass what an mbarrier can count).
   const uint32_t polls = c_sweep_wait_polls;
   bool failed = false;
   auto wait = [&](uint64_t* bar, uint32_t phase, uint32_t bytes, bool rearm) {
     if (failed) return;
     if (!cl_wait(bar, phase & 1u, polls)) {
       failed = true;
+      *reinterpret_cast<volatile int*>(s_stop) = 1;  // waits come before a step's first CTA barrier in the x part
       if (w.status) atomicOr(w.status, 4);
     } else if (rearm && tid == 0) {
       mbar_arrive_expect_tx(bar, bytes);
@@ -540,6 +553,7 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
       for (int r = 0; r < RX; ++r) ex[(jx * RX + r) * COLS] = v[r];
     }
     __syncthreads();
+    const int stop = *reinterpret_cast<volatile int*>(s_stop);  // between two barriers: the same for every thread
     if (in_col) {
       C* const ex = b_ex + cc;
 #pragma unroll
@@ -565,6 +579,7 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
       }
     }
     __syncthreads();
+    if (stop) break;
     if (in_col) {
       const C* const ex = b_ex + cc;
       C v[RX];
@@ -580,9 +595,16 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
       }
     }
   }
-  if (failed)  // stores of this CTA that nothing waits for are given time to land
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
-  cl_sync();  // no CTA leaves while another may still write to it
+  // No CTA leaves while another may still write to it.  After a wait that ran out, stores
+  // may be on their way that nothing waits for: every CTA stays 200,000 cycles (about 100
+  // us; a store between two SMs takes about one) after the last one has sent its last.
+  __syncthreads();
+  if (*s_stop && tid < CL) cl_store_flag(cl_addr(s_stop, tid));
+  cl_sync();
+  if (*s_stop) {
+    for (const long long t0 = clock64(); clock64() - t0 < 200000;) __nanosleep(1000);
+    cl_sync();
+  }
 }
 
 template <typename T, int NX, int NY, int NZ, int CL, bool DST>

@@ -24,3 +24,34 @@ def test_mixed_films_repeat_bit_for_bit(gpu, n):
         first = first or got
         assert all(np.array_equal(a, b) for a, b in zip(got, first))
     s.close()
+
+
+@pytest.mark.parametrize("n,precision", [((32, 32, 32), "fp64"), ((24, 24, 24), "fp64"), ((128, 128, 1), "fp64"),
+                                         ((128, 128, 1), "mixed"), ((8, 8, 8), "mixed")])
+def test_wait_timeout_of_a_long_sweep(gpu, n, precision):
+    """With a poll limit of 0 every CTA's first wait gives up, and the CTAs stop sending: a sweep
+    whose later steps would have sent the barriers more than 2^20 bytes ends, is reported, and a
+    new handle's run is the undisturbed one's."""
+    from polyswift_plusplus_b200 import _abi as A
+    cfg, w = _case(n, precision, 200)
+    s = ScftSolver(cfg)
+    s.set_variant(3)
+    s.restore(w)
+    s.update(2)
+    want = [s.w(0), s.phi(1)]
+    for _ in range(3):
+        s.restore(w)
+        assert gpu.ps_gpu_set_bulk_wait_limit(0) == A.PS_OK
+        try:
+            with pytest.raises(A.PsError) as ei:
+                s.update(1)
+        finally:
+            assert gpu.ps_gpu_set_bulk_wait_limit(0xFFFFFFFF) == A.PS_OK
+        assert ei.value.code == A.PS_GPU_ERR and "wait limit" in str(ei.value)
+    s.close()
+    s = ScftSolver(cfg)
+    s.set_variant(3)
+    s.restore(w)
+    s.update(2)
+    assert all(np.array_equal(a, b) for a, b in zip(want, [s.w(0), s.phi(1)]))
+    s.close()
