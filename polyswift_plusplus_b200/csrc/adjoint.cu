@@ -1568,6 +1568,7 @@ int ps_adj_forward(ps_adj* a, const double* w, double* phi, double* log_q) {
   if (!a || !w) return PS_ATTRIB_ERR;
   ps_handle* h = a->h;
   const size_t nfN = (size_t)a->nf * a->N;
+  a->have_forward = a->have_backward = false;  // until this one is complete
   PA_CUDA(a, cudaSetDevice(h->dev));
   PA_CUDA(a, cudaMemcpyAsync(h->d_w, w, sizeof(double) * nfN, cudaMemcpyDeviceToDevice, h->st));
   PA_CUDA(a, cudaMemsetAsync(&h->d_sc->error_flags, 0, sizeof(int), h->st));
@@ -1587,7 +1588,6 @@ int ps_adj_forward(ps_adj* a, const double* w, double* phi, double* log_q) {
   }
   if (log_q) *log_q = h->h_sc->log_q[0];
   a->have_forward = true;
-  a->have_backward = false;
   return PS_OK;
 }
 
@@ -1600,7 +1600,10 @@ int ps_adj_backward(ps_adj* a, const double* g_phi, double g_log_q, double* g_w,
   }
   ps_handle* h = a->h;
   const long long N = a->N;
+  a->have_backward = false;
   PA_CUDA(a, cudaSetDevice(h->dev));
+  // a wait that ran out in an earlier backward pass says nothing about this one
+  PA_CUDA(a, cudaMemsetAsync(&h->d_sc->error_flags, 0, sizeof(int), h->st));
   PA_CUDA(a, cudaMemcpyAsync(a->gphi, g_phi, sizeof(double) * (size_t)a->nf * N, cudaMemcpyDeviceToDevice,
                              h->st));
   PA_CUDA(a, a->bwd[0](h->st));

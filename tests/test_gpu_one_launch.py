@@ -55,3 +55,38 @@ def test_wait_timeout_of_a_long_sweep(gpu, n, precision):
     s.update(2)
     assert all(np.array_equal(a, b) for a, b in zip(want, [s.w(0), s.phi(1)]))
     s.close()
+
+
+def test_adjoint_after_a_wait_timeout(gpu):
+    """A backward pass that timed out leaves the forward pass valid: the next backward pass gives
+    the undisturbed gradients.  A forward pass that timed out leaves none."""
+    import torch
+    from polyswift_plusplus_b200 import _abi as A
+    from polyswift_plusplus_b200 import workloads as W
+    from polyswift_plusplus_b200.adjoint import ChainAdjoint
+    cfg = W.diblock_config(16, 2.0, 0.35, 20.0, 20, W.Updater(kind="steepestDescent"), "fp64")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w = torch.rand((2, cfg.n_total), generator=g, dtype=torch.float64, device="cuda")
+
+    def timed_out(call):
+        assert gpu.ps_gpu_set_bulk_wait_limit(0) == A.PS_OK
+        try:
+            with pytest.raises(A.PsError) as ei:
+                call()
+        finally:
+            assert gpu.ps_gpu_set_bulk_wait_limit(0xFFFFFFFF) == A.PS_OK
+        assert ei.value.code == A.PS_GPU_ERR and "wait limit" in str(ei.value)
+
+    with_gphi = torch.ones_like(w)
+    adj = ChainAdjoint(cfg)
+    adj.forward(w)
+    want = adj.backward(with_gphi, 0.5)[0].clone()
+    timed_out(lambda: adj.backward(with_gphi, 0.5))
+    assert torch.equal(adj.backward(with_gphi, 0.5)[0], want)
+    timed_out(lambda: adj.forward(w))
+    with pytest.raises(A.PsError) as ei:
+        adj.backward(with_gphi, 0.5)
+    assert ei.value.code == A.PS_ATTRIB_ERR
+    adj.forward(w)
+    assert torch.equal(adj.backward(with_gphi, 0.5)[0], want)
+    adj.close()
