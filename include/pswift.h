@@ -311,6 +311,12 @@ void* ps_gpu_stream(const ps_handle* h);
 int ps_gpu_set_variant(ps_handle* h, int variant);
 int ps_gpu_get_variant(const ps_handle* h, int* variant, float* tune_ms, int n_tune);
 
+/* 1 when the current device can run each sweep of an n[0] x n[1] x n[2] grid in
+ * one launch on a thread-block cluster (variants with bits 0 and 1), 0 when it
+ * has no such kernel or no room for its cluster: the sweeps then run step by
+ * step.  precision: PS_PREC_*. */
+int ps_gpu_one_launch(const int n[3], int precision);
+
 /* Switch the arithmetic of the propagator sweeps between iterations (no
  * reference counterpart).  w, p, phi and the FP64 Anderson history carry over
  * unchanged, so a run can iterate in PS_PREC_MIXED until the FP32 noise floor

@@ -145,6 +145,7 @@ SIGNATURES = {
     "ps_gpu_enable_sweep_timing": (C.c_int, [_vp, C.c_int]),
     "ps_gpu_stream": (_vp, [_vp]),
     "ps_gpu_set_variant": (C.c_int, [_vp, C.c_int]),
+    "ps_gpu_one_launch": (C.c_int, [C.POINTER(C.c_int), C.c_int]),
     "ps_gpu_get_variant": (C.c_int, [_vp, C.POINTER(C.c_int), C.POINTER(C.c_float), C.c_int]),
     "ps_gpu_set_precision": (C.c_int, [_vp, C.c_int]),
     "ps_gpu_set_spectral_filter": (C.c_int, [_vp, C.POINTER(ps_filter_config)]),

@@ -408,7 +408,7 @@ struct Builder {
     fused = plane_fused_supported(8, ny, nz);
     step = step_plane_supported(ny, nz);
     adj = adj_step_supported(ny, nz);
-    one = sweep_cluster_supported(nx, ny, nz);
+    one = sweep_cluster_to_fits(nx, ny, nz);
   }
 
   const double* wf(int b) const {

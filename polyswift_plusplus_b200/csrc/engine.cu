@@ -415,18 +415,24 @@ static int build_device_tables(ps_handle* h) {
   if (!rc) rc = alloc_copy(h, &B.d_pencil, xw);
   B.h_plane = pw;
   B.h_pencil = xw;
-  // one-launch sweeps in start order (blocks beyond kSweepSegs: none)
+  // one-launch sweeps in start order (none with blocks beyond kSweepSegs, and none where
+  // the device has no room for the cluster: such a handle takes the step passes)
   std::vector<int> order(ne);
   for (size_t e = 0; e < ne; ++e) order[e] = (int)e;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h->sw_start[a] < h->sw_start[b]; });
   h->levels.clear();
   h->sw_level.assign(ne, SweepLevel{0, 0, 1});
   B.h_sweep.clear();
-  bool fits = !h->no_slices;
+  bool fits = !h->no_slices && sweep_cluster_fits<T>(h->n[0], h->n[1], h->n[2]);
   for (int e : order) fits = fits && (int)h->sweeps[h->exec[e]].segs.size() <= kSweepSegs;
-  for (size_t i = 0; i < ne && fits; ++i) {
+  for (size_t i = 0; i < ne; ++i) {
     const int e = order[i];
     const Sweep& sw = h->sweeps[h->exec[e]];
+    if (h->levels.empty() || h->levels.back().k != h->sw_start[e])
+      h->levels.push_back(SweepLevel{h->sw_start[e], (int)i, 0});
+    h->levels.back().cnt++;
+    h->sw_level[e] = SweepLevel{h->sw_start[e], (int)i, 1};
+    if (!fits) continue;  // the levels serve both precisions
     SweepWork<T> w;
     memset(&w, 0, sizeof(w));
     w.src = sw.jbuf >= 0 ? B.jbuf[sw.jbuf] : nullptr;
@@ -441,10 +447,6 @@ static int build_device_tables(ps_handle* h) {
       w.seg[g].kyzc = B.kyzc[sw.segs[g].ktab_id];
       w.seg[g].end = sw.segs[g].off + sw.segs[g].steps;
     }
-    if (h->levels.empty() || h->levels.back().k != h->sw_start[e])
-      h->levels.push_back(SweepLevel{h->sw_start[e], (int)i, 0});
-    h->levels.back().cnt++;
-    h->sw_level[e] = SweepLevel{h->sw_start[e], (int)i, 1};
     B.h_sweep.push_back(w);
   }
   if (!rc && fits) rc = alloc_copy(h, &B.d_sweep, B.h_sweep);

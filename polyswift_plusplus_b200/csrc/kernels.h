@@ -89,8 +89,10 @@ template <typename T> struct SweepWork {
   } seg[kSweepSegs];
 };
 
-// The grid has a one-launch sweep (a film nx x ny x 1 runs as nx rows of ny).
-bool sweep_cluster_supported(int nx, int ny, int nz);
+// The grid has a one-launch sweep (a film nx x ny x 1 runs as nx rows of ny), and the
+// current device can place its cluster; the same for launch_sweep_cluster_to.
+template <typename T> bool sweep_cluster_fits(int nx, int ny, int nz);
+bool sweep_cluster_to_fits(int nx, int ny, int nz);
 template <typename T>
 cudaError_t launch_sweep_cluster(const SweepWork<T>* d_works, int nworks, int nx, int ny, int nz, const c2_t<T>* tw_x,
                                  const c2_t<T>* tw_y, const c2_t<T>* tw_z, cudaStream_t st);

@@ -1,16 +1,21 @@
 // Grids with a one-launch sweep (sweep_cluster.cuh) and its dispatch.
+#include "../../include/pswift.h"
 #include "sweep_cluster.cuh"
 
 namespace psb {
 
-bool sweep_cluster_supported(int nx, int ny, int nz) {
+template <typename T, bool DST> static bool fits_any(int nx, int ny, int nz) {
   const int f = (nz == 1);
 #define PSB_X(NX, NY, NZ, CL) \
-  if (nx == NX && (f ? (NY == 1 && ny == NZ) : (ny == NY && nz == NZ))) return true;
+  if (nx == NX && (f ? (NY == 1 && ny == NZ) : (ny == NY && nz == NZ))) return sweep_cluster_fits_t<T, NX, NY, NZ, CL, DST>();
   PSB_SWEEP_GRIDS(PSB_X)
 #undef PSB_X
   return false;
 }
+template <typename T> bool sweep_cluster_fits(int nx, int ny, int nz) { return fits_any<T, false>(nx, ny, nz); }
+bool sweep_cluster_to_fits(int nx, int ny, int nz) { return fits_any<double, true>(nx, ny, nz); }
+template bool sweep_cluster_fits<float>(int, int, int);
+template bool sweep_cluster_fits<double>(int, int, int);
 
 template <typename T, bool DST>
 static cudaError_t launch_any(const SweepWork<T>* w, int nw, int nx, int ny, int nz, const c2_t<T>* tx,
@@ -42,3 +47,9 @@ cudaError_t sweep_cluster_set_polls(uint32_t polls) {
 }
 
 }  // namespace psb
+
+extern "C" int ps_gpu_one_launch(const int n[3], int precision) {
+  if (!n) return 0;
+  return precision == PS_PREC_MIXED ? psb::sweep_cluster_fits<float>(n[0], n[1], n[2])
+                                    : psb::sweep_cluster_fits<double>(n[0], n[1], n[2]);
+}

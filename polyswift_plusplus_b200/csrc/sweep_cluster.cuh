@@ -607,33 +607,53 @@ __global__ void __launch_bounds__((SweepCl<T, NX, NY, NZ, CL_>::TH), 1)
   }
 }
 
+template <typename T, int NX, int NY, int NZ, int CL, bool DST> struct SweepClLaunch {
+  using P = SweepCl<T, NX, NY, NZ, CL>;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  static auto kernel() { return sweep_cluster_kernel<T, NX, NY, NZ, CL, DST>; }
+  cudaError_t set(int nworks, cudaStream_t st) {
+    static unsigned attr_mask = 0;
+    cudaError_t e = ensure_smem_attr(kernel(), P::SMEM, &attr_mask);
+    if (e != cudaSuccess) return e;
+    if (CL > 8) {
+      e = cudaFuncSetAttribute(kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return e;
+    }
+    cfg.gridDim = dim3(CL, nworks);
+    cfg.blockDim = dim3(P::TH);
+    cfg.dynamicSmemBytes = P::SMEM;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CL;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaSuccess;
+  }
+};
+
 template <typename T, int NX, int NY, int NZ, int CL, bool DST>
 cudaError_t launch_sweep_cluster_t(const SweepWork<T>* d_works, int nworks, const c2_t<T>* tx, const c2_t<T>* ty,
                                    const c2_t<T>* tz, cudaStream_t st) {
-  using P = SweepCl<T, NX, NY, NZ, CL>;
-  auto kern = sweep_cluster_kernel<T, NX, NY, NZ, CL, DST>;
-  static unsigned attr_mask = 0;
-  cudaError_t e = ensure_smem_attr(kern, P::SMEM, &attr_mask);
+  SweepClLaunch<T, NX, NY, NZ, CL, DST> l;
+  cudaError_t e = l.set(nworks, st);
   if (e != cudaSuccess) return e;
-  if (CL > 8) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CL, nworks);
-  cfg.blockDim = dim3(P::TH);
-  cfg.dynamicSmemBytes = P::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CL;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, d_works, tx, ty, tz);
+  return cudaLaunchKernelEx(&l.cfg, l.kernel(), d_works, tx, ty, tz);
+}
+
+// The device can place a cluster of this kernel: a part of it (a partition, a share given
+// to the process) may have no 16 SMs that can form one.
+template <typename T, int NX, int NY, int NZ, int CL, bool DST> bool sweep_cluster_fits_t() {
+  SweepClLaunch<T, NX, NY, NZ, CL, DST> l;
+  int clusters = 0;
+  cudaError_t e = l.set(1, nullptr);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, l.kernel(), &l.cfg);
+  if (e != cudaSuccess) cudaGetLastError();  // not this caller's error: the sweeps take the step passes
+  return e == cudaSuccess && clusters > 0;
 }
 
 }  // namespace psb

@@ -46,7 +46,8 @@ template <typename T> struct SweepSet {
   const int* plane_cnt = nullptr;
   const int* pencil_off = nullptr;
   const int* pencil_cnt = nullptr;
-  // one-launch sweeps, by the global step at which they start
+  // one-launch sweeps, by the global step at which they start (nullptr: this grid or
+  // device has none)
   const SweepWork<T>* d_sweep = nullptr;
   const SweepLevel* levels = nullptr;
   int nlevels = 0;
@@ -72,8 +73,7 @@ inline cudaError_t launch_plane_cluster_t(const PlaneWork<T>* w, int nw, int nx,
 template <typename T>
 inline bool resident_path(const SweepSet<T>& s, int variant) {
   constexpr int both = VARIANT_FUSE_Z | VARIANT_FUSE_K;
-  return (variant & both) == both && !(variant & (VARIANT_XY | VARIANT_CLUSTER)) && s.d_sweep &&
-         sweep_cluster_supported(s.n[0], s.n[1], s.n[2]);
+  return (variant & both) == both && !(variant & (VARIANT_XY | VARIANT_CLUSTER)) && s.d_sweep;
 }
 // The sweeps' spectra are in the compact layout of step_plane.cuh.
 template <typename T>

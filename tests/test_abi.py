@@ -627,3 +627,14 @@ setupPS(8, 8, 8, 0.25, 0.25, 0.25, "'off'")
     blocks = pc.polymers[0].blocks
     assert [(b.n_head, b.n_tail) for b in list(blocks)[:3]] == [(0, 2), (0, 2), (0, 2)]
     assert list(blocks[0].tail_joined[:2]) == [1, 2] and list(blocks[2].tail_joined[:2]) == [0, 1]
+
+
+def test_no_one_launch_sweep_without_room_for_its_cluster(native_lib):
+    """Without a device (as on one that cannot place the cluster) the query says no, so that
+    a handle takes the step passes."""
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("a device is here")
+    for n in ((16, 16, 16), (128, 128, 1), (20, 20, 20)):
+        for precision in (A.PS_PREC_FP64, A.PS_PREC_MIXED):
+            assert native_lib.ps_gpu_one_launch((C.c_int * 3)(*n), precision) == 0

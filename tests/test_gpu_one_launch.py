@@ -90,3 +90,15 @@ def test_adjoint_after_a_wait_timeout(gpu):
     adj.forward(w)
     assert torch.equal(adj.backward(with_gphi, 0.5)[0], want)
     adj.close()
+
+
+def test_one_launch_grids_of_this_device(gpu):
+    """The whole device has room for every cluster; other grids have no such kernel."""
+    import ctypes as C
+    from polyswift_plusplus_b200 import _abi as A
+    from test_gpu_step_kernels import ONE_LAUNCH
+    for precision in (A.PS_PREC_FP64, A.PS_PREC_MIXED):
+        for n in ONE_LAUNCH:
+            assert gpu.ps_gpu_one_launch((C.c_int * 3)(*n), precision) == 1, n
+        for n in ((48, 48, 48), (16, 16, 24), (128, 64, 1), (20, 20, 20)):
+            assert gpu.ps_gpu_one_launch((C.c_int * 3)(*n), precision) == 0, n
