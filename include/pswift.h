@@ -307,7 +307,11 @@ void* ps_gpu_stream(const ps_handle* h);
  * sweep leaving a junction starts one step after the last arriving sweep
  * ends, its junction product launched in between (so branched polymers also
  * run in batches).
- * ps_gpu_get_variant also returns the measured sweep time of each variant (ms). */
+ * ps_gpu_get_variant also returns the measured sweep time of each variant (ms):
+ * one pass of its launches one by one, its kernels loaded; -1: not timed.  Where
+ * the gaps between launches count, the fastest variant with and the fastest
+ * without bit 3 are then timed as graphs, with and without early starts, and
+ * the fastest graph is kept: its variant need not have the least time here. */
 int ps_gpu_set_variant(ps_handle* h, int variant);
 int ps_gpu_get_variant(const ps_handle* h, int* variant, float* tune_ms, int n_tune);
 

@@ -9,6 +9,7 @@
 // Semantics follow PsDomain::update (pstrol/PsDomain.cpp:332-372): densities
 // reset, PsBlockCopolymer::update for each polymer, then the updater with F
 // evaluated on the updated w (pseffhamil/PsSteepDUpdater.cpp:200-201).
+#include <limits.h>
 #include <math.h>
 #include <stdlib.h>
 #include <stdio.h>
@@ -473,18 +474,22 @@ static int build_device_tables(ps_handle* h) {
   return rc;
 }
 
-// Launch the propagator sweeps of one iteration.
+// Launch the propagator sweeps of one iteration (their steps up to `last` alone, where they
+// are launched step by step).
 template <typename T>
-static int launch_sweeps(ps_handle* h, long long* nlaunch, int variant) {
+static int launch_sweeps(ps_handle* h, long long* nlaunch, int variant, int last = INT_MAX) {
   if (!(variant & VARIANT_SPLIT) || h->sw_st.empty()) {
     // lockstep: every sweep's step in shared launches, junction starts between steps
-    PS_CUDA(h, launch_sweep_set<T>(handle_sweep_set<T>(h), variant, h->st, nlaunch));
+    SweepSet<T> s = handle_sweep_set<T>(h);
+    s.kmax = std::min(s.kmax, last);
+    PS_CUDA(h, launch_sweep_set<T>(s, variant, h->st, nlaunch));
     return PS_OK;
   }
   // one launch chain per executed sweep, forked from and joined back into h->st
   PS_CUDA(h, cudaEventRecord(h->ev_split, h->st));
   for (size_t e = 0; e < h->sw_st.size(); ++e) {
     SweepSet<T> s = handle_sweep_set<T>(h);
+    s.kmax = std::min(s.kmax, last);
     s.plane_off = h->sw_plane_off[e].data();
     s.plane_cnt = h->sw_plane_cnt[e].data();
     s.pencil_off = h->sw_pencil_off[e].data();
@@ -710,8 +715,10 @@ static int time_as_graph(ps_handle* h, int v, cudaEvent_t a, cudaEvent_t b, floa
   return PS_OK;
 }
 
-// Time every kernel variant on this instance's own sweeps (same inputs, one
-// warm-up and one timed sweep each) and keep the fastest.
+// Time every kernel variant on this instance's own sweeps (same inputs) and keep the
+// fastest: one pass each, after its first two steps have loaded its kernels.  A variant
+// whose first pass was far behind was once not timed again, and that pass held the loading
+// of its kernels: what was kept then hung on what the process had run before.
 template <typename T>
 static int autotune_t(ps_handle* h) {
   cudaEvent_t a = nullptr, b = nullptr;
@@ -720,24 +727,19 @@ static int autotune_t(ps_handle* h) {
   float best = 1e30f;
   int best_v = 0;
   int rc = PS_OK;
-  // the usual winners first: a variant whose first pass (with the loading of its kernels)
-  // is far behind is not run again
-  for (int i = 0; i < VARIANT_COUNT && e == cudaSuccess && rc == PS_OK; ++i) {
-    const int v = i ^ (VARIANT_FUSE_Z | VARIANT_FUSE_K);
+  for (int v = 0; v < VARIANT_COUNT && e == cudaSuccess && rc == PS_OK; ++v) {
     h->tune_ms[v] = -1.f;
     if ((v & VARIANT_XY) && (!h->xy_ok || (v & VARIANT_FUSE_Z))) continue;  // absent / same
     if ((v & VARIANT_CLUSTER) && (!h->cluster_ok || (v & VARIANT_XY))) continue;
     if ((v & VARIANT_SPLIT) && h->sw_st.empty()) continue;                 // one sweep only
     float ms = 0.f;
-    for (int pass = 0; pass < 2 && rc == PS_OK && e == cudaSuccess; ++pass) {
-      if (pass == 1 && ms > 1.25f * best + 0.5f) break;
-      long long nl = 0;
-      e = cudaEventRecord(a, h->st);
-      if (e == cudaSuccess) rc = launch_sweeps<T>(h, &nl, v);
-      if (rc == PS_OK && e == cudaSuccess) e = cudaEventRecord(b, h->st);
-      if (rc == PS_OK && e == cudaSuccess) e = cudaEventSynchronize(b);
-      if (rc == PS_OK && e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
-    }
+    long long nl = 0;
+    rc = launch_sweeps<T>(h, &nl, v, 1);
+    if (rc == PS_OK) e = cudaEventRecord(a, h->st);
+    if (rc == PS_OK && e == cudaSuccess) rc = launch_sweeps<T>(h, &nl, v);
+    if (rc == PS_OK && e == cudaSuccess) e = cudaEventRecord(b, h->st);
+    if (rc == PS_OK && e == cudaSuccess) e = cudaEventSynchronize(b);
+    if (rc == PS_OK && e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
     if (rc != PS_OK || e != cudaSuccess) break;
     h->tune_ms[v] = ms;
     if (ms < best) {
@@ -756,17 +758,17 @@ static int autotune_t(ps_handle* h) {
       int& t = top[(v & VARIANT_SPLIT) ? 1 : 0];
       if (early_path(set, v) && h->tune_ms[v] >= 0.f && (t < 0 || h->tune_ms[v] < h->tune_ms[t])) t = v;
     }
-    float least = 1e30f;
+    float least = 1e30f, plain[2] = {};  // as graphs: the least of all, and without early starts
     const int early[3] = {0, VARIANT_EARLY, VARIANT_EARLY | VARIANT_EARLY_PLANE};
     const int ne = early_plane_path(set, best_v) ? 3 : 2;
     // first neither early, then the early starts of a variant that is not far behind
     for (int i = 0; i < 2 * ne && rc == PS_OK && e == cudaSuccess; ++i) {
       const int v = top[i % 2], how = early[i / 2];
-      if (v < 0 || (how && h->tune_ms[v] > 1.08f * least)) continue;
+      if (v < 0 || (how && plain[i % 2] > 1.08f * least)) continue;
       float ms = 0.f;
       rc = time_as_graph<T>(h, v | how, a, b, &ms);
       if (rc) break;
-      if (how == 0 || ms < h->tune_ms[v]) h->tune_ms[v] = ms;
+      if (how == 0) plain[i % 2] = ms;
       if (ms < least) {
         least = ms;
         best_v = v;

@@ -102,3 +102,33 @@ def test_one_launch_grids_of_this_device(gpu):
             assert gpu.ps_gpu_one_launch((C.c_int * 3)(*n), precision) == 1, n
         for n in ((48, 48, 48), (16, 16, 24), (128, 64, 1), (20, 20, 20)):
             assert gpu.ps_gpu_one_launch((C.c_int * 3)(*n), precision) == 0, n
+
+
+TUNE = """
+import sys
+sys.path[:0] = {paths}
+from test_gpu_step_kernels import _case
+from polyswift_plusplus_b200.scft import ScftSolver
+cfg, w = _case((24, 48, 48), "fp64", 100)
+for _ in range(3):
+    s = ScftSolver(cfg)
+    s.restore(w)
+    s.update(2)
+    print(*s.variant()[1])
+    s.close()
+"""
+
+
+def test_tuner_times_no_kernel_loading(gpu):
+    """The times of a fresh process's first handle are those of the next ones: a pass takes about
+    1 ms here, loading the kernels of a variant about 20."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    here = Path(__file__).resolve().parent
+    out = subprocess.run([sys.executable, "-c", TUNE.format(paths=[str(here.parent), str(here)])], check=True,
+                         capture_output=True, text=True).stdout
+    first, *later = [[float(x) for x in line.split()] for line in out.splitlines()]
+    for v, ms in enumerate(first):
+        assert ms <= 2 * min(t[v] for t in later) + 2.0 or ms < 0, (v, ms)
+    assert sum(ms > 0 for ms in first) == 8
