@@ -132,3 +132,18 @@ def test_tuner_times_no_kernel_loading(gpu):
     for v, ms in enumerate(first):
         assert ms <= 2 * min(t[v] for t in later) + 2.0 or ms < 0, (v, ms)
     assert sum(ms > 0 for ms in first) == 8
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [16, 24, 32, 48, 64, 96, 128])
+def test_one_row_planes(gpu, n, precision):
+    """n x 1 x n grids take the films' one-launch sweeps with the tables of another axis."""
+    from test_gpu_step_kernels import _compare
+    _compare((n, 1, n), precision, [3, 11], 0)
+
+
+@pytest.mark.parametrize("n", [(24, 24, 1), (64, 64, 1), (128, 128, 1), (32, 1, 32), (12, 12, 12)])
+def test_adjoint_on_one_launch_grids(gpu, n):
+    """Forward and recomputation in one launch each, the adjoint steps in separate passes."""
+    from test_gpu_adjoint_steps import test_adjoint_schedules
+    test_adjoint_schedules(gpu, n)
