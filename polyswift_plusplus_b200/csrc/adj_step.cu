@@ -3,15 +3,16 @@
 //
 // What was slow: an adjoint step was seven launches (two forward planes, two x
 // passes, the stress sums, the k^2 multiply, the inverse passes and the pointwise
-// update), each reading and writing whole spectra or fields: 33 us a step at 64^3, and
-// 18.6 ms for a forward and backward pass of 128 steps.  Fused: 13 us a step, 9.9 ms a
-// pass (half of it the sweeps and their recomputation from checkpoints), 7.8 with the
-// adjoints of both sweeps in the same launches; a step is bound by the latency of its
-// two launches.  Replaying the passes as graphs changed nothing: the launches are not
-// the limit.  Nor is one CTA of 240 registers per SM: with 128 (two) 7.6 to 7.9 ms.
-// Now it is two: the x pass keeps U and V in registers between their forward
-// transforms, the stress sums and U's way back, and the plane pass turns mu into the
-// next lambda and starts its transform (and that of wf q) in the same pass.
+// update), each reading and writing whole spectra or fields.  Now it is two: the x pass
+// keeps U and V in registers between their forward transforms, the stress sums and U's
+// way back, and the plane pass turns mu into the next lambda and starts its transform
+// (and that of wf q) in the same pass.
+//
+// At 64^3: 33 -> 13 us a step; forward and backward of 128 steps 18.6 -> 9.9 ms (half of
+// it the sweeps and their recomputation from checkpoints), 7.6 with the adjoints of both
+// sweeps in the same launches.  A step is bound by the latency of its two launches.
+// Replaying the passes as graphs changed nothing: submitting them is not the limit.
+// Neither is one plane CTA of 240 registers per SM: with 128 (two) 7.6 to 7.9 ms.
 #include "step_plane.cuh"
 
 namespace psb {

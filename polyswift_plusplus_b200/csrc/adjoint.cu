@@ -599,8 +599,11 @@ struct Builder {
         ps_adj* A = a;
         ps_handle* H = h;
         const int nx_ = nx, inner = ny * nzh;
-        // the plane pass behind it starts early (early_path in sweeps.cuh): 64^3 7.65 -> 7.4 ms,
-        // 96^3 23.4 -> 23.0
+        // The plane pass behind it starts early (early_path in sweeps.cuh).  Forward and
+        // backward of 100 steps, ms, without and with: 16 x 24^2 2.78 -> 2.64, 48^3 4.10 -> 3.99,
+        // 64 x 48^2 4.64 -> 4.47, 64^3 5.74 -> 5.59, 64 x 96 x 48 15.27 -> 15.05, 96^3 18.08 ->
+        // 17.87; of 14 grids and two checkpoint intervals in this range one lost 2%
+        // (32 x 48^2 3.48 -> 3.56, at full storage 2.34 -> 2.28), the others 0 to 6% less.
         const bool early = nx <= 96 && a->N <= 96LL * 96 * 96;
         ops.push_back([=](cudaStream_t st) {
           return launch_step_pencil<double>(A->d_xw + x0, nx_works, nx_, inner, true, early, H->bd.tw_x, st);

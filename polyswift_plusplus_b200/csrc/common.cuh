@@ -65,11 +65,13 @@ __device__ __forceinline__ C mul_mi(C a) {
 // of it on the stream has finished: it does its independent prologue (twiddle
 // tables, work descriptors), then pdl_wait() blocks until that kernel has
 // completed and its writes are visible; without the attribute pdl_wait() is a
-// no-op.  Kernels do not trigger their dependents early as a rule: blocks of the next
-// sweep kernel parked on pdl_wait() hold shared memory and registers that the
+// no-op.  A kernel triggers its dependents early only in the two forms that the engine
+// times and takes where they are faster (VARIANT_EARLY: the x pass, VARIANT_EARLY_PLANE:
+// FP32 planes of 96 x 96 and more; early_path in sweeps.cuh), and in the adjoint's sweeps:
+// blocks of the next kernel parked on pdl_wait() hold shared memory and registers that a
 // concurrent sweep's kernels need, and land where this kernel's blocks have left room
-// instead of evenly.  At 128^3 a trigger in the plane pass, early or late, was 2-4%
-// slower.  The x pass can (VARIANT_EARLY).
+// instead of evenly.  Every kernel that triggers has waited first, so that a kernel which
+// starts early never overtakes the one before last.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -126,16 +126,15 @@ template <typename T, int NX, int NY, int NZ, int CL_> struct SweepCl {
   static_assert(EACH >= 1 && COLS <= EACH + 1, "every CTA owns columns, as many as the others or one more");
 };
 
-// The grids that have one, as
-// (nx, ny, nz, CTAs of the cluster), a film nx x ny x 1 as (nx, 1, ny).  One plane
-// or a few rows per CTA, as many CTAs as a cluster may have: us per step of both
-// sweeps, FP64 (FP32), against the step passes' two launches:
+// The grids that have one: (nx, ny, nz, CTAs of the cluster), a film nx x ny x 1 as
+// (nx, 1, ny).  One plane or a few rows per CTA, as many CTAs as a cluster may have: us
+// per step of both sweeps, FP64 (FP32), against the step passes' two launches:
 //   8^3 1.3 (1.4), 12^3 1.7 (1.6)      passes 5.6 and 6.3 (7.0)
-//   16^3 1.8, eight CTAs 1.9           passes 4.6
-//   24^3 3.7 (2.8), eight CTAs 4.6 (3.3), passes 5.7
-//   32^3 4.6 (3.2), passes 5.5 (5.0)
-//   films, eight rows a CTA: 24^2 1.6 (1.5), passes 10 (12); 48^2 2.1 (1.9), 11 (13);
-//   64^2 2.3, 4.9; 96^2 3.5 (2.6), 16 (19); 128^2 3.9, eight CTAs 4.5, passes 6.4
+//   16^3 1.8 (1.8), eight CTAs 1.9     passes 4.6
+//   24^3 3.6 (2.7), eight CTAs 4.6 (3.3), passes 5.7
+//   32^3 4.5 (3.2), passes 5.5 (5.0)
+//   films, eight rows a CTA: 24^2 1.6 (1.6), passes 10 (12); 48^2 2.1 (1.9), 11 (13);
+//   64^2 2.2 (1.9), 4.9; 96^2 3.6 (2.7), 16 (19); 128^2 3.8 (3.1), eight CTAs 4.5, passes 6.4
 // 48^3 has too much work for 16 SMs per sweep: FP32 9.0 against 7.3.
 #define PSB_SWEEP_GRIDS(X)                                        \
   X(8, 8, 8, 8) X(12, 12, 12, 12) X(16, 16, 16, 16)               \
